@@ -378,7 +378,9 @@ int walk(next_handle* h, bool potential) {
                                  h->prm.walk_warps, h->prm.walk_stack, h->queue, h->stats, h->err, h->sm_count, h->st),
                "group walk");
     } else {
-        NB_TRY(launch_walk_plain(bd, h->sysid, h->n, h->t, h->P, h->nsys > 1, h->stats, h->err, h->st), "plain walk");
+        NB_TRY(launch_walk_plain(bd, h->sysid, h->d_offsets, h->nsys, h->n, h->t, h->P, potential, h->stats, h->err,
+                                 h->st),
+               "plain walk");
     }
     return NEXT_OK;
 }

@@ -44,8 +44,9 @@ cudaError_t build_tree(const uint64_t* keys, int64_t n, const Bodies& bd, const 
                        cudaStream_t st);
 
 // walk_plain.cu
-cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, int64_t n, const Tree& t, const Params& P,
-                              bool multi_system, unsigned long long* stats, int* err, cudaStream_t st);
+cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int64_t* offsets, int nsys, int64_t n,
+                              const Tree& t, const Params& P, bool potential, unsigned long long* stats, int* err,
+                              cudaStream_t st);
 int direct_slices(int64_t n, int64_t k);
 // in: k sizes, k masses, k distances; out: k softening lengths (reference law)
 cudaError_t launch_softening_eval(const double* in, int64_t k, double* out, cudaStream_t st);

@@ -1,17 +1,20 @@
-// Plain FP64 force walk: one thread per target body, depth-first over the
-// tree in octant order 0..7 -- the order bhAccel recurses
-// (src/gravity/octree.h:176-178) -- with a per-level (next sibling, end)
-// stack instead of recursion.  Reference physics repeats bhAccel's
-// arithmetic (octree.h:134-173, softening.h:21-35) operation for operation;
-// accurate physics uses Plummer softening, the full-width opening test and
-// the corrected quadrupole.
+// Plain FP64 force walks: every body opens the tree by its own distance.
+//
+// Reference physics: one thread per target body, depth-first over the tree in
+// octant order 0..7 -- the order bhAccel recurses (src/gravity/octree.h:176-178)
+// -- with a per-level (next sibling, end) stack instead of recursion, and
+// bhAccel's arithmetic (octree.h:134-173, softening.h:21-35) operation for
+// operation.  Accurate physics (Plummer softening, full-width opening test,
+// corrected quadrupole): one warp per few bodies, one node per lane.
 //
 // Also: the FP64 direct-summation kernel used to state force errors.
 //
 // Built with -fmad=false so each + and * rounds on its own, matching the
-// reference's x86-64 build (no FMA contraction).  cbrt and pow come from
-// CUDA's math library; they may differ from the host libm in the last bit.
+// reference's x86-64 build (no FMA contraction); the accurate walk's sums use
+// fma() explicitly.  cbrt and pow come from CUDA's math library; they may
+// differ from the host libm in the last bit.
 #include "common.cuh"
+#include "fp64_math.cuh"
 #include "kernels.cuh"
 
 namespace nb {
@@ -66,9 +69,8 @@ __device__ __forceinline__ void add_stats(unsigned long long* stats, unsigned lo
     }
 }
 
-template <bool ACCURATE>
 __global__ void __launch_bounds__(128)
-walk_plain_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree t, Params P,
+walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree t, Params P,
                   unsigned long long* stats, int* err) {
     if (*err & kErrAbort) return;
     const int64_t nodes = t.counts[1];
@@ -79,8 +81,8 @@ walk_plain_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree 
         const int root = sysid ? sysid[i] : 0;
         const double xi = bd.x[i], yi = bd.y[i], zi = bd.z[i], mi = bd.m[i];
         const int ti = bd.type[i];
-        const double eps2 = P.eps * P.eps, G = P.G, theta = P.theta;
-        double ax = 0.0, ay = 0.0, az = 0.0, pot = 0.0;
+        const double theta = P.theta;
+        double ax = 0.0, ay = 0.0, az = 0.0;
         int2 stack[kMaxLevel + 2];
         int sp = 0;
         int cur = root, end = root + 1;
@@ -108,82 +110,248 @@ walk_plain_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree 
                 raise_error(err, leaf ? kErrIndex : kErrStack);
                 break;
             }
-            if (!ACCURATE) {
-                const int cnt = -lk.y;
-                if (leaf && cnt == 1 && lk.x == i) continue;          // own leaf (octree.h:135)
-                const double size = q64[6];
-                if (leaf && cnt > 1) {
-                    // deepest-level bucket: its bodies act as one-body leaves of this size
-                    const double Z[6] = {0, 0, 0, 0, 0, 0};
-                    for (int j = lk.x; j < lk.x + cnt; ++j) {
-                        if (j == i || bd.m[j] == 0.0) continue;
-                        ref_interact(bd.m[j], bd.x[j], bd.y[j], bd.z[j], size, Z, xi, yi, zi, mi, ti, ax, ay, az);
-                        ++npp;
-                    }
-                    continue;
+            const int cnt = -lk.y;
+            if (leaf && cnt == 1 && lk.x == i) continue;          // own leaf (octree.h:135)
+            const double size = q64[6];
+            if (leaf && cnt > 1) {
+                // deepest-level bucket: its bodies act as one-body leaves of this size
+                const double Z[6] = {0, 0, 0, 0, 0, 0};
+                for (int j = lk.x; j < lk.x + cnt; ++j) {
+                    if (j == i || bd.m[j] == 0.0) continue;
+                    ref_interact(bd.m[j], bd.x[j], bd.y[j], bd.z[j], size, Z, xi, yi, zi, mi, ti, ax, ay, az);
+                    ++npp;
                 }
-                const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                const double dist = sqrt(r2 + 1e-20);
-                if (leaf || (size / dist) < theta) {
-                    const double Q[6] = {q64[0], q64[1], q64[2], q64[3], q64[4], q64[5]};
-                    ref_interact(c.w, c.x, c.y, c.z, size, Q, xi, yi, zi, mi, ti, ax, ay, az);
-                    if (leaf) ++npp; else ++npc;
-                    continue;
-                }
-                stack[sp++] = make_int2(cur, end);
-                cur = lk.x;
-                end = lk.x + lk.y;
-            } else {
-                const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                const double rc = q64[7];
-                if (r2 < rc * rc) {
-                    if (!leaf) {
-                        stack[sp++] = make_int2(cur, end);
-                        cur = lk.x;
-                        end = lk.x + lk.y;
-                        continue;
-                    }
-                    for (int j = lk.x; j < lk.x - lk.y; ++j) {
-                        if (j == i) continue;
-                        const double ex = bd.x[j] - xi, ey = bd.y[j] - yi, ez = bd.z[j] - zi;
-                        const double e2 = ex * ex + ey * ey + ez * ez + eps2;
-                        const double rinv = 1.0 / sqrt(e2);
-                        const double mr3 = G * bd.m[j] * rinv * rinv * rinv;
-                        ax += mr3 * ex; ay += mr3 * ey; az += mr3 * ez;
-                        pot -= G * bd.m[j] * rinv;
-                        ++npp;
-                    }
-                    continue;
-                }
-                const double r2s = r2 + eps2;
-                const double rinv = 1.0 / sqrt(r2s);
-                const double rinv2 = rinv * rinv;
-                const double mr3 = G * c.w * rinv * rinv2;
-                ax += mr3 * dx; ay += mr3 * dy; az += mr3 * dz;
-                pot -= G * c.w * rinv;
-                if (P.quad) {
-                    const double qxx = q64[0], qyy = q64[1], qzz = q64[2];
-                    const double qxy = q64[3], qxz = q64[4], qyz = q64[5];
-                    const double qdx = qxx * dx + qxy * dy + qxz * dz;
-                    const double qdy = qxy * dx + qyy * dy + qyz * dz;
-                    const double qdz = qxz * dx + qyz * dy + qzz * dz;
-                    const double q = dx * qdx + dy * qdy + dz * qdz;
-                    const double rinv5 = rinv2 * rinv2 * rinv;
-                    const double rinv7 = rinv5 * rinv2;
-                    const double c7 = 2.5 * G * q * rinv7;
-                    const double c5 = G * rinv5;
-                    ax += c7 * dx - c5 * qdx;
-                    ay += c7 * dy - c5 * qdy;
-                    az += c7 * dz - c5 * qdz;
-                    pot -= 0.5 * G * q * rinv5;
-                }
-                ++npc;
+                continue;
             }
+            const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            const double dist = sqrt(r2 + 1e-20);
+            if (leaf || (size / dist) < theta) {
+                const double Q[6] = {q64[0], q64[1], q64[2], q64[3], q64[4], q64[5]};
+                ref_interact(c.w, c.x, c.y, c.z, size, Q, xi, yi, zi, mi, ti, ax, ay, az);
+                if (leaf) ++npp; else ++npc;
+                continue;
+            }
+            stack[sp++] = make_int2(cur, end);
+            cur = lk.x;
+            end = lk.x + lk.y;
         }
         bd.ax[i] = ax; bd.ay[i] = ay; bd.az[i] = az;
-        if (bd.pot) bd.pot[i] = pot;
+        if (bd.pot) bd.pot[i] = 0.0;
+    }
+    add_stats(stats, npp, npc);
+}
+
+// Accurate physics.  One warp walks the tree for W consecutive bodies (in key
+// order, so they lie close together).  A stack entry is a node and the mask of
+// the bodies that opened its parent; each round pops up to 32 nodes, one per
+// lane, and every lane tests and evaluates its node against the masked bodies
+// in turn, with the node's record in registers.  Each lane sums its own share
+// of every body's force; the shares are folded once, at the end.
+//
+// A thread per body read every node's record through 32 scattered lanes (L1
+// data wavefronts at 87-93% of their peak, 17 of 32 lanes active); here a record
+// is read once for W bodies, mostly with its siblings beside it, and small
+// systems have 1 / W of a warp per body instead of 1 / 32.  1,048,576 bodies
+// (theta 0.5, one body per leaf): 21.7 -> 9.25 ms per walk, 16,384 bodies 1.95 ->
+// 0.23 ms.  Bound now by the issue of the FP64 chains and the selects around
+// them (62% of issue slots, FP64 pipe 41%).  W = 4: the bodies of a warp open
+// different cells, so a larger W spends more lanes on nodes one body wants (W =
+// 6: 9.5 ms, 8: 10.1 ms) and a smaller one reads and tests more nodes per body
+// (3: 9.9 ms, 2: 12.5 ms, 1: 19 ms); 120 registers, 4 blocks per SM (5 spill: 15 ms).
+constexpr int kPlainW = 4;
+constexpr int kPlainWarps = 4;
+// Popping k nodes adds at most 7 k entries, and one node at a time never more
+// than 7 per level: rounds are cut short so that 7 * kMaxLevel + 8 entries stay
+// free for a walk that goes on one node at a time.
+constexpr int kPlainStack = 640;
+constexpr int kPlainReserve = 7 * kMaxLevel + 8;
+constexpr int kPlainChunk = 16;                          // bodies of an opened leaf appended per lane and turn
+constexpr int kPlainList = 32 + 32 * kPlainChunk;
+struct PlainShared {
+    int2 stack[kPlainStack];                             // node, mask of the bodies that opened its parent
+    int2 list[kPlainList];                               // body, mask of the bodies that opened its leaf
+};
+
+template <bool POT>
+__global__ void __launch_bounds__(32 * kPlainWarps, 4)
+walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, int64_t n, Tree t, Params P,
+                     unsigned long long* stats, int* err) {
+    if (*err & kErrAbort) return;
+    __shared__ PlainShared shared[kPlainWarps];
+    PlainShared& S = shared[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const uint32_t lt = (1u << lane) - 1u;
+    const int64_t w = blockIdx.x * (int64_t)kPlainWarps + (threadIdx.x >> 5);
+    unsigned npp = 0, npc = 0;
+    // Bodies first .. first + W of one system, counted from the system's first body, so that a body's
+    // sums do not depend on the systems around it: system s owns the warps from offsets[s] / W + s on.
+    int sys = 0;
+    int64_t first = w * kPlainW, last = n;
+    if (offsets) {
+        int top = nsys;
+        while (top - sys > 1) {
+            const int mid = (sys + top) >> 1;
+            if (offsets[mid] / kPlainW + mid <= w) sys = mid;
+            else top = mid;
+        }
+        first = offsets[sys] + (w - (offsets[sys] / kPlainW + sys)) * kPlainW;
+        last = offsets[sys + 1];
+    }
+    // a warp with any body of this device's share computes all of its bodies (again so that a body's
+    // sums do not depend on the share) and stores the share's
+    unsigned bodies = 0, own = 0;
+#pragma unroll
+    for (int b = 0; b < kPlainW; ++b) {
+        if (first + b >= last) continue;
+        bodies |= 1u << b;
+        if (first + b >= P.own_lo && first + b < P.own_hi) own |= 1u << b;
+    }
+    if (own) {                                           // warp-uniform
+        const unsigned nodes = static_cast<unsigned>(t.counts[1]), nbodies = static_cast<unsigned>(n);
+        const double eps2 = P.eps * P.eps, G = P.G;
+        double x[kPlainW], y[kPlainW], z[kPlainW], ax[kPlainW], ay[kPlainW], az[kPlainW], pot[kPlainW];
+        int sp = 1, pn = 0;
+#pragma unroll
+        for (int b = 0; b < kPlainW; ++b) {
+            const int64_t i = first + b < last ? first + b : first;
+            x[b] = bd.x[i]; y[b] = bd.y[i]; z[b] = bd.z[i];
+            ax[b] = ay[b] = az[b] = pot[b] = 0.0;
+        }
+        if (lane == 0) S.stack[0] = make_int2(sys, static_cast<int>(bodies));
+        __syncwarp();
+        while (sp > 0 || pn > 0) {
+            const int room = (kPlainStack - kPlainReserve - sp) / 7;
+            const int nb = min(min(sp, 32), max(room, 1));
+            sp -= nb;
+            const int2 entry = lane < nb ? S.stack[sp + lane] : make_int2(-1, 0);
+            const int node = entry.x;
+            unsigned mask = static_cast<unsigned>(entry.y);
+            __syncwarp();
+            int2 lk = make_int2(0, 0);
+            double4 c = make_double4(0.0, 0.0, 0.0, 0.0);
+            double2 qa = make_double2(0.0, 0.0), qb = qa, qc = qa, qd = qa;
+            if (mask) {
+                bool ok = static_cast<unsigned>(node) < nodes;
+                if (ok) {
+                    // the node's whole record in one round trip
+                    lk = __ldg(t.link + node);
+                    const double2* c2 = reinterpret_cast<const double2*>(t.com + node);
+                    const double2 ca = __ldg(c2), cb = __ldg(c2 + 1);
+                    const double2* q2 = reinterpret_cast<const double2*>(t.quad64 + 8 * static_cast<int64_t>(node));
+                    qd = __ldg(q2 + 3);
+                    if (P.quad) { qa = __ldg(q2); qb = __ldg(q2 + 1); qc = __ldg(q2 + 2); }
+                    c = make_double4(ca.x, ca.y, cb.x, cb.y);
+                    const unsigned e = static_cast<unsigned>(lk.x) + static_cast<unsigned>(lk.y > 0 ? lk.y : -lk.y);
+                    ok = lk.x >= 0 && lk.y <= 8 && e <= (lk.y > 0 ? nodes : nbodies);
+                }
+                if (!ok) raise_error(err, kErrIndex);
+                if (!ok || c.w == 0.0) mask = 0;
+            }
+            const double rc2 = qd.y * qd.y;
+            unsigned opened = 0;
+            // no branch in this loop: the bodies' chains of dependent FP64 operations interleave
+#pragma unroll
+            for (int b = 0; b < kPlainW; ++b) {
+                const bool mine = mask >> b & 1u;
+                const double dx = c.x - x[b], dy = c.y - y[b], dz = c.z - z[b];
+                const double r2 = dx * dx + dy * dy + dz * dz;
+                const bool open = mine && r2 < rc2, use = mine && !open;
+                opened |= static_cast<unsigned>(open) << b;
+                const double r2s = away_from_ends(r2 + eps2);
+                const double rinv = rsqrt_fast(r2s);
+                const double rinv2 = rinv * rinv;
+                // a = G rinv5 ((m r2 + 2.5 d.Q.d rinv2) d - Q d); Q = 0 in monopole walks
+                const double qx = fma(qc.x, dz, fma(qb.y, dy, qa.x * dx));
+                const double qy = fma(qc.y, dz, fma(qa.y, dy, qb.y * dx));
+                const double qz = fma(qb.x, dz, fma(qc.y, dy, qc.x * dx));
+                const double q = fma(dz, qz, fma(dy, qy, dx * qx));
+                const double g5 = G * rinv * (rinv2 * rinv2);
+                const double k = fma(2.5 * q, rinv2, c.w * r2s);
+                const double fx = fma(g5, fma(k, dx, -qx), ax[b]), fy = fma(g5, fma(k, dy, -qy), ay[b]),
+                             fz = fma(g5, fma(k, dz, -qz), az[b]);
+                ax[b] = use ? fx : ax[b];
+                ay[b] = use ? fy : ay[b];
+                az[b] = use ? fz : az[b];
+                if (POT) pot[b] = use ? pot[b] - fma(0.5 * q, g5, G * c.w * rinv) : pot[b];
+            }
+            npc += __popc(mask & ~opened & own);
+            // children of opened cells -> stack
+            const int push = opened && lk.y > 0 ? lk.y : 0;
+            int off = 0, total = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t m = __ballot_sync(0xffffffffu, (push >> k) & 1);
+                off += __popc(m & lt) << k;
+                total += __popc(m) << k;
+            }
+            if (sp + total > kPlainStack) {              // only a broken tree gets here
+                if (lane == 0) raise_error(err, kErrIndex);
+                break;
+            }
+            if (total > 0) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (k < push) S.stack[sp + off + k] = make_int2(lk.x + k, static_cast<int>(opened));
+            }
+            sp += total;
+            // bodies of opened leaves -> list, evaluated 32 at a time, the rest when the walk ends
+            int remaining = opened && lk.y < 0 ? -lk.y : 0;
+            int src = lk.x;
+            for (bool more = __any_sync(0xffffffffu, remaining > 0) || (sp == 0 && pn > 0); more;) {
+                const int take = min(remaining, kPlainChunk);
+                int o2 = 0, tot = 0;
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    const uint32_t m = __ballot_sync(0xffffffffu, (take >> k) & 1);
+                    o2 += __popc(m & lt) << k;
+                    tot += __popc(m) << k;
+                }
+                for (int k = 0; k < take; ++k) S.list[pn + o2 + k] = make_int2(src + k, static_cast<int>(opened));
+                pn += tot;
+                src += take;
+                remaining -= take;
+                more = __any_sync(0xffffffffu, remaining > 0);
+                __syncwarp();
+                while (pn >= 32 || (pn > 0 && sp == 0 && !more)) {
+                    const int k = pn - 32 > 0 ? pn - 32 : 0;     // from the end: nothing moves
+                    const int2 pe = k + lane < pn ? S.list[k + lane] : make_int2(-1, 0);
+                    const int j = pe.x;
+                    const unsigned jm = static_cast<unsigned>(pe.y);
+                    pn = k;
+                    double xj = 0.0, yj = 0.0, zj = 0.0, gm = 0.0;
+                    if (jm) { xj = bd.x[j]; yj = bd.y[j]; zj = bd.z[j]; gm = G * bd.m[j]; }
+#pragma unroll
+                    for (int b = 0; b < kPlainW; ++b) {
+                        if (!(jm >> b & 1u) || j == first + b) continue;
+                        const double dx = xj - x[b], dy = yj - y[b], dz = zj - z[b];
+                        const double rinv = rsqrt(dx * dx + dy * dy + dz * dz + eps2);
+                        const double mr = gm * rinv, mr3 = mr * rinv * rinv;
+                        ax[b] = fma(mr3, dx, ax[b]);
+                        ay[b] = fma(mr3, dy, ay[b]);
+                        az[b] = fma(mr3, dz, az[b]);
+                        if (POT) pot[b] -= mr;
+                        npp += own >> b & 1u;
+                    }
+                    __syncwarp();
+                }
+            }
+            __syncwarp();
+        }
+#pragma unroll
+        for (int b = 0; b < kPlainW; ++b) {
+            for (int o = 16; o > 0; o >>= 1) {
+                ax[b] += __shfl_xor_sync(0xffffffffu, ax[b], o);
+                ay[b] += __shfl_xor_sync(0xffffffffu, ay[b], o);
+                az[b] += __shfl_xor_sync(0xffffffffu, az[b], o);
+                if (POT) pot[b] += __shfl_xor_sync(0xffffffffu, pot[b], o);
+            }
+            const int64_t i = first + b;
+            if (lane == 0 && (own >> b & 1u)) {
+                bd.ax[i] = ax[b]; bd.ay[i] = ay[b]; bd.az[i] = az[b];
+                if (POT) bd.pot[i] = pot[b];
+            }
+        }
     }
     add_stats(stats, npp, npc);
 }
@@ -251,16 +419,20 @@ cudaError_t launch_softening_eval(const double* in, int64_t k, double* out, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, int64_t n, const Tree& t,
-                              const Params& P, bool multi_system, unsigned long long* stats, int* err,
+cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int64_t* offsets, int nsys, int64_t n,
+                              const Tree& t, const Params& P, bool potential, unsigned long long* stats, int* err,
                               cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const unsigned blocks = static_cast<unsigned>((n + 127) / 128);
-    const int32_t* sid = multi_system ? sysid : nullptr;
-    if (P.physics == NEXT_PHYSICS_ACCURATE)
-        walk_plain_kernel<true><<<blocks, 128, 0, st>>>(bd, sid, n, t, P, stats, err);
-    else
-        walk_plain_kernel<false><<<blocks, 128, 0, st>>>(bd, sid, n, t, P, stats, err);
+    const int32_t* sid = nsys > 1 ? sysid : nullptr;
+    if (P.physics == NEXT_PHYSICS_ACCURATE) {
+        const int64_t warps = (n + kPlainW - 1) / kPlainW + (nsys > 1 ? nsys : 0);
+        const unsigned blocks = static_cast<unsigned>((warps + kPlainWarps - 1) / kPlainWarps);
+        auto kern = potential ? walk_accurate_kernel<true> : walk_accurate_kernel<false>;
+        kern<<<blocks, 32 * kPlainWarps, 0, st>>>(bd, nsys > 1 ? offsets : nullptr, nsys, n, t, P, stats, err);
+    } else {
+        const unsigned blocks = static_cast<unsigned>((n + 127) / 128);
+        walk_reference_kernel<<<blocks, 128, 0, st>>>(bd, sid, n, t, P, stats, err);
+    }
     count_launches(1);
     return cudaGetLastError();
 }

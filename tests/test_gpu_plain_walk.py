@@ -1,0 +1,98 @@
+"""The plain FP64 walks at the edges of their warps, lists and stacks.
+
+The accurate walk takes four bodies of one system per warp and sums a body's
+terms in another order than the oracle: at most a few thousand terms, each
+rounded a few times, so forces and potentials agree to 1e-12 of the largest one
+(2^-53 times the term count leaves a factor of two); the opening decisions are
+the same FP64 comparisons, so the interaction counts are equal.
+"""
+import numpy as np
+import pytest
+
+from next_b200 import ic
+from next_b200.native import Simulation
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-12
+
+
+def close(a, b, names):
+    scale = max(np.max(np.abs(b[c])) for c in names)
+    for c in names:
+        np.testing.assert_allclose(a[c], b[c], rtol=0, atol=TOL * scale)
+
+
+@pytest.mark.parametrize("n,leaf_cap,theta,eps,quad", [
+    (1, 1, 0.5, 0.01, 1), (2, 1, 0.5, 0.0, 1), (3, 1, 0.5, 0.01, 1), (4, 2, 0.5, 0.01, 1), (5, 1, 0.5, 0.01, 1),
+    (31, 1, 0.5, 0.01, 1), (33, 3, 0.3, 0.01, 0), (129, 64, 0.5, 0.01, 1), (1003, 1, 0.2, 0.0, 1),
+    (1001, 17, 1.0, 0.01, 1), (4097, 1, 0.7, 0.005, 0), (4099, 64, 0.5, 0.01, 1),
+])
+def test_accurate_walk_sizes(oracle, n, leaf_cap, theta, eps, quad):
+    b = ic.plummer(n, seed=n)
+    sim = Simulation("accurate", "fp64", theta=theta, eps=eps, leaf_cap=leaf_cap, quadrupole=quad)
+    sim.upload(b)
+    sim.reset_timers()
+    a = sim.accel(potential=True)
+    r = oracle.accel(b, mode="accurate", theta=theta, eps=eps, leaf_cap=leaf_cap, quad=bool(quad), potential=True)
+    st = sim.stats()
+    assert (st["pp_interactions"], st["pc_interactions"], st["device_error"]) == (r["pp"], r["pc"], 0)
+    if n > 1:
+        close(a, r, ("ax", "ay", "az"))
+        close(a, r, ("pot",))
+    f = Simulation("accurate", "fp64", theta=theta, eps=eps, leaf_cap=leaf_cap, quadrupole=quad)
+    f.upload(b)
+    g = f.accel()                                   # the walk without the potential: the same forces
+    for c in ("ax", "ay", "az"):
+        np.testing.assert_array_equal(g[c], a[c])
+    sim.close()
+    f.close()
+
+
+def test_accurate_walk_buckets_and_massless(oracle):
+    """Coincident bodies (leaves of more bodies than the leaf size) and zero masses."""
+    b = ic.plummer(700, seed=5)
+    for k in ("x", "y", "z"):
+        b[k][100:200] = b[k][100]
+        b[k][300:303] = b[k][300]
+    b["m"][::7] = 0.0
+    sim = Simulation("accurate", "fp64", theta=0.5, eps=0.02, leaf_cap=1)
+    sim.upload(b)
+    a = sim.accel(potential=True)
+    r = oracle.accel(b, mode="accurate", theta=0.5, eps=0.02, leaf_cap=1, potential=True)
+    close(a, r, ("ax", "ay", "az"))
+    close(a, r, ("pot",))
+    sim.close()
+
+
+def test_accurate_walk_full_stack(oracle):
+    """An opening angle so small that nearly every cell opens: the stack fills and the rounds are cut short."""
+    b = ic.plummer(3000, seed=9)
+    sim = Simulation("accurate", "fp64", theta=0.02, eps=0.01, leaf_cap=1)
+    sim.upload(b)
+    a = sim.accel()
+    r = oracle.accel(b, mode="accurate", theta=0.02, eps=0.01, leaf_cap=1)
+    close(a, r, ("ax", "ay", "az"))
+    assert sim.stats()["device_error"] == 0
+    sim.close()
+
+
+def test_accurate_walk_ensemble_of_odd_sizes():
+    """Systems whose sizes are no multiples of a warp's bodies, some empty: bit-equal to each system alone."""
+    sizes = [5, 0, 1, 130, 3, 0, 2, 517, 64, 7]
+    parts = [ic.plummer(k, seed=i) for i, k in enumerate(sizes) if k]
+    b = {c: np.concatenate([p[c] for p in parts]) for c in parts[0]}
+    offsets = np.concatenate([[0], np.cumsum(sizes)])
+    sim = Simulation("accurate", "fp64")
+    sim.upload(b, offsets)
+    a = sim.accel()
+    for i, k in enumerate(sizes):
+        if k == 0:
+            continue
+        one = Simulation("accurate", "fp64")
+        one.upload(ic.plummer(k, seed=i))
+        r = one.accel()
+        for c in ("ax", "ay", "az"):
+            np.testing.assert_array_equal(a[c][offsets[i]:offsets[i + 1]], r[c])
+        one.close()
+    sim.close()
