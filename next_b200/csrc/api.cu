@@ -219,7 +219,7 @@ void free_tree(next_handle* h) {
     Tree& t = h->t;
     dfree(t.dlev); dfree(t.nint); dfree(t.int_start); dfree(t.int_level); dfree(t.int_bounds);
     dfree(t.int_packed); dfree(t.int_node); dfree(t.counter); dfree(t.climb); dfree(t.ready); dfree(t.link); dfree(t.parent); dfree(t.level);
-    dfree(t.com); dfree(t.quad64); dfree(t.box); dfree(t.quad32); dfree(t.groups);
+    dfree(t.com); dfree(t.quad64); dfree(t.box); dfree(t.quad32); dfree(t.soft); dfree(t.groups);
     dfree(h->scan_tmp);
     t.cap_int = t.cap_node = t.cap_group = 0;
 }
@@ -250,6 +250,7 @@ int alloc_tree(next_handle* h, int64_t cap_int) {
     A(&t.link, t.cap_node); A(&t.parent, t.cap_node); A(&t.level, t.cap_node);
     A(&t.com, t.cap_node); A(&t.quad64, 8 * t.cap_node);
     if (h->P.physics == NEXT_PHYSICS_ACCURATE) { A(&t.box, t.cap_node); A(&t.quad32, 2 * t.cap_node); }
+    else { A(&t.soft, 2 * t.cap_node); }
     A(&t.groups, t.cap_group);
     h->scan_tmp_elems = scan_tile_sums_needed(std::max<int64_t>(n + 1, cap_int + 1));
     int64_t* st64 = nullptr;
@@ -732,6 +733,7 @@ int next_create(const next_params* p, next_handle** out) {
     h->P.leaf_cap = p->physics == NEXT_PHYSICS_REFERENCE ? 1 : p->leaf_cap;
     h->P.group_cap = p->group_cap;
     h->P.quad = p->quadrupole ? 1 : 0;
+    h->P.theta_squarable = p->theta > 1e-100 && p->theta < 1e100;
     h->device = p->device;
     auto bail = [&](cudaError_t e, const char* w) {
         int rc = cuda_fail(h, e, w);
@@ -749,12 +751,13 @@ int next_create(const next_params* p, next_handle** out) {
     auto A = [&](auto** q, size_t c) { if (e == cudaSuccess) e = dalloc(q, c); };
     A(&h->err, 1); A(&h->stats, 4); A(&h->queue, 1); A(&h->tickets, 4); A(&h->partial, kReduceMax * 8);
     A(&h->dts, 2); A(&h->dt_out, 2); A(&h->diag, 8); A(&h->changed, 4); A(&h->fma_out, 1);
-    A(&h->t.counts, 6); A(&h->done, 1);
+    A(&h->t.counts, 6); A(&h->t.dark_mass, 1); A(&h->done, 1);
     if (e != cudaSuccess) return bail(e, "scalars");
     e = cudaMemset(h->err, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(h->tickets, 0, sizeof(unsigned int) * 4);
     if (e == cudaSuccess) e = cudaMemset(h->stats, 0, sizeof(unsigned long long) * 4);
     if (e == cudaSuccess) e = cudaMemset(h->t.counts, 0, sizeof(int64_t) * 6);
+    if (e == cudaSuccess) e = cudaMemset(h->t.dark_mass, 0xff, sizeof(double));   // NaN
     if (e == cudaSuccess) e = cudaMemset(h->done, 0, sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_dts), sizeof(double) * 2, cudaHostAllocDefault);
     if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_err), sizeof(int) * 2, cudaHostAllocDefault);
@@ -782,7 +785,7 @@ void next_destroy(next_handle* h) {
     h->comm = nullptr;
     free_bodies(h);
     dfree(h->err); dfree(h->stats); dfree(h->queue); dfree(h->tickets); dfree(h->partial);
-    dfree(h->dts); dfree(h->dt_out); dfree(h->diag); dfree(h->changed); dfree(h->fma_out); dfree(h->t.counts);
+    dfree(h->dts); dfree(h->dt_out); dfree(h->diag); dfree(h->changed); dfree(h->fma_out); dfree(h->t.counts); dfree(h->t.dark_mass);
     dfree(h->done);
     dfree(h->d_targets); dfree(h->d_targetpos); dfree(h->d_direct_partial); dfree(h->d_direct_out);
     if (h->flush) cudaFree(h->flush);
@@ -869,7 +872,7 @@ static int upload_staged(next_handle* h, int64_t n_systems, const int64_t* offse
         NB_TRY(launch_load_velocities(stage, b, h->inv, n, h->st), "velocities");
         return NEXT_OK;   // same positions: tree order and cached forces stay valid
     }
-    NB_TRY(launch_load_all(stage, stype, b, h->inv, n, h->st), "load");
+    NB_TRY(launch_load_all(stage, stype, b, h->inv, n, h->t.dark_mass, h->st), "load");
     h->forces_valid = false;
     h->have_bodies = true;
     set_key_levels(h, kMaxLevel);     // new positions: measure the depth again
@@ -1152,9 +1155,9 @@ int next_step_host(next_handle* h, double dt, int64_t n, double* x, double* y, d
                                    cudaMemcpyDeviceToDevice, h->st), "restore");
         NB_TRY(cudaMemcpyAsync(h->stage + 6 * n, h->io_in[p] + 6 * n, sizeof(double) * n, cudaMemcpyDeviceToDevice,
                                h->st), "restore");
-        NB_TRY(launch_load_all(h->stage, h->io_type[p], b, h->inv, n, h->st), "restore");
+        NB_TRY(launch_load_all(h->stage, h->io_type[p], b, h->inv, n, h->t.dark_mass, h->st), "restore");
     } else {
-        NB_TRY(launch_load_all(in, h->io_type[k], b, h->inv, n, h->st), "load");
+        NB_TRY(launch_load_all(in, h->io_type[k], b, h->inv, n, h->t.dark_mass, h->st), "load");
     }
     h->forces_valid = false;
     h->cube_fresh = false;

@@ -66,6 +66,9 @@ struct Tree {
     double* quad64;        // 8 per node: Qxx Qyy Qzz Qxy Qxz Qyz half-width rcrit
     float4* box;           // FP32 COM and rcrit^2 (mixed walk traversal)
     float4* quad32;        // 2 per node: -G (Qxx Qyy Qzz Qxy) (Qxz Qyz), G m, 0
+    double2* soft;         // reference physics, 2 per node: half-width, link (as bits); softening base, softening of
+                           // a dark body of mass *dark_mass
+    double* dark_mass;     // mass of some type-1 body (NaN: none was uploaded)
     // walk groups
     int4* groups;          // (first body, count, root node, 0)
     int32_t* ready;        // upward pass: internal ids whose children are all leaves
@@ -78,6 +81,7 @@ struct Params {
     int physics;           // NEXT_PHYSICS_*
     double theta, eps, G;
     int leaf_cap, group_cap, quad;
+    bool theta_squarable = true;   // theta^2 is neither tiny nor huge: opening tests may compare squares
     // bodies (working positions) whose forces this device computes; the
     // whole range on one device, one share of it per rank when sharded
     int64_t own_lo = 0, own_hi = INT64_MAX;

@@ -270,9 +270,10 @@ __global__ void load_velocities_kernel(const double* __restrict__ stage, Bodies 
 }
 
 __global__ void load_all_kernel(const double* __restrict__ stage, const int* __restrict__ stype, Bodies b,
-                                uint32_t* __restrict__ inv, int64_t n) {
+                                uint32_t* __restrict__ inv, int64_t n, double* dark_mass) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (stype[i] == 1) *dark_mass = stage[6 * n + i];   // any of them serves
     b.x[i] = stage[i]; b.y[i] = stage[n + i]; b.z[i] = stage[2 * n + i];
     b.vx[i] = stage[3 * n + i]; b.vy[i] = stage[4 * n + i]; b.vz[i] = stage[5 * n + i];
     b.m[i] = stage[6 * n + i];
@@ -428,9 +429,9 @@ cudaError_t launch_load_velocities(const double* stage, const Bodies& b, const u
 }
 
 cudaError_t launch_load_all(const double* stage, const int* stype, const Bodies& b, uint32_t* inv, int64_t n,
-                            cudaStream_t st) {
+                            double* dark_mass, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    load_all_kernel<<<grid_for(n, 256), 256, 0, st>>>(stage, stype, b, inv, n);
+    load_all_kernel<<<grid_for(n, 256), 256, 0, st>>>(stage, stype, b, inv, n, dark_mass);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -77,8 +77,9 @@ cudaError_t launch_check_upload(const double* stage, const int* stype, const Bod
                                 bool compare, int* flags, cudaStream_t st);
 cudaError_t launch_load_velocities(const double* stage, const Bodies& b, const uint32_t* inv, int64_t n,
                                    cudaStream_t st);
+// dark_mass (may stay untouched): the mass of some type-1 body among them
 cudaError_t launch_load_all(const double* stage, const int* stype, const Bodies& b, uint32_t* inv, int64_t n,
-                            cudaStream_t st);
+                            double* dark_mass, cudaStream_t st);
 // flags[0] = 1 unless in (7 lanes x n, caller order) and type equal prev_out's
 // 6 lanes, prev_in's mass lane and prev_type bit for bit (and are finite)
 cudaError_t launch_same_as_last(const double* in, const int* type, const double* prev_out, const double* prev_in,

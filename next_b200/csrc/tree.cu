@@ -34,6 +34,7 @@
 // reference-mode moments repeat src/gravity/octree.h:92-127 bit for bit.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "softening.cuh"
 
 namespace nb {
 
@@ -313,7 +314,7 @@ struct Mom {
     double m, cx, cy, cz, q[6];
 };
 
-__device__ __forceinline__ void store_moments(Tree& t, int nid, const Mom& a, double half, double rcrit,
+__device__ __forceinline__ void store_moments(Tree& t, int nid, int2 link, const Mom& a, double half, double rcrit,
                                               double G, bool accurate) {
     t.com[nid] = make_double4(a.cx, a.cy, a.cz, a.m);
     double* q64 = t.quad64 + 8 * static_cast<int64_t>(nid);
@@ -329,6 +330,13 @@ __device__ __forceinline__ void store_moments(Tree& t, int nid, const Mom& a, do
                         static_cast<float>(-G * a.q[2]), static_cast<float>(-G * a.q[3]));
         t.quad32[2 * static_cast<int64_t>(nid) + 1] =
             make_float4(static_cast<float>(-G * a.q[4]), static_cast<float>(-G * a.q[5]), static_cast<float>(G * a.m), 0.0f);
+    } else {
+        // what the reference's softening of this node has that no target changes: a cube root and,
+        // for the dark bodies of the one mass, a power, once per node instead of once per interaction
+        const double dark = *t.dark_mass;
+        t.soft[2 * static_cast<int64_t>(nid)] = make_double2(half, __hiloint2double(link.y, link.x));
+        t.soft[2 * static_cast<int64_t>(nid) + 1] =
+            make_double2(softening_base(half, a.m), dark == dark ? softening_dark(half, a.m, dark) : 0.0);
     }
 }
 
@@ -489,7 +497,7 @@ __device__ __forceinline__ void leaf_moments(const Bodies& bd, const uint64_t* _
         a.m = m; a.cx = cx; a.cy = cy; a.cz = cz;
         rcrit = rcrit_of(a, key, lvl, cube, base, half, P.theta);
     }
-    store_moments(t, static_cast<int>(n), a, half, rcrit, P.G, accurate);
+    store_moments(t, static_cast<int>(n), make_int2(first, -cnt), a, half, rcrit, P.G, accurate);
 }
 
 // Moments of internal node rec.x from its children rec.y .. rec.y + nchild
@@ -598,7 +606,7 @@ __device__ __forceinline__ void combine_children(const uint64_t* __restrict__ ke
         p.m = m; p.cx = cx; p.cy = cy; p.cz = cz;
         prc = rcrit_of(p, key, pl, pcube, base, phalf, P.theta);
     }
-    store_moments(t, nid, p, phalf, prc, P.G, accurate);
+    store_moments(t, nid, plk, p, phalf, prc, P.G, accurate);
 }
 
 // A climb record is valid when it describes a node with 1-8 children inside

@@ -16,46 +16,39 @@
 #include "common.cuh"
 #include "fp64_math.cuh"
 #include "kernels.cuh"
+#include "softening.cuh"
 
 namespace nb {
 
 namespace {
 
-__device__ __forceinline__ double dmax_like_std(double a, double b) { return (a < b) ? b : a; }
+// One accepted node in reference physics, from its separation, mass, softening
+// base, dark-matter softening (-1 for bodies it does not apply to) and
+// quadrupole: the two addends bhAccel accumulates (src/gravity/octree.h:138-172).
+struct RefTerm {
+    double mx, my, mz, qx, qy, qz;
+};
 
-// nextSoftening: src/dt/softening.h:21-35.
-__device__ __forceinline__ double next_softening(double size, double mass, double dist) {
-    const double eps_size = size * 0.015;
-    const double eps_mass = cbrt(mass) * 0.002;
-    const double taper = 1.0 / (1.0 + dist * 10.0);
-    const double eps = (eps_size + eps_mass) * taper;
-    return dmax_like_std(eps, 1e-4);
-}
-
-// One accepted node in reference physics: src/gravity/octree.h:138-172.
-__device__ __forceinline__ void ref_interact(double nm, double ncx, double ncy, double ncz, double size,
-                                             const double* Q, double xi, double yi, double zi, double mi,
-                                             int ti, double& ax, double& ay, double& az) {
-    const double dx = ncx - xi, dy = ncy - yi, dz = ncz - zi;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const double dist = sqrt(r2 + 1e-20);
-    double eps = next_softening(size, nm, dist);
-    if (ti == 1) eps = dmax_like_std(eps, 2.0 * size / pow(nm / mi, 0.333333333));
+__device__ __forceinline__ RefTerm ref_term(double nm, double dx, double dy, double dz, double r2, double base,
+                                            double dark, const double2& qa, const double2& qb, const double2& qc) {
+    const double eps = dmax_like_std(softening_at(base, sqrt(r2 + 1e-20)), dark);
     const double r2s = r2 + eps * eps;
     const double dinv = 1.0 / sqrt(r2s);
     const double inv3 = dinv * dinv * dinv;
     const double fac = 1.0 * nm * inv3;
-    ax += dx * fac; ay += dy * fac; az += dz * fac;
     const double inv5 = inv3 * (dinv * dinv);
     const double inv7 = inv5 * (dinv * dinv);
-    const double q = Q[0] * dx * dx + Q[1] * dy * dy + Q[2] * dz * dz +
-                     2.0 * (Q[3] * dx * dy + Q[4] * dx * dz + Q[5] * dy * dz);
-    const double qrx = 2.0 * (Q[0] * dx + Q[3] * dy + Q[4] * dz);
-    const double qry = 2.0 * (Q[3] * dx + Q[1] * dy + Q[5] * dz);
-    const double qrz = 2.0 * (Q[4] * dx + Q[5] * dy + Q[2] * dz);
-    ax += 0.5 * (qrx * inv5 - 5.0 * q * inv7 * dx);
-    ay += 0.5 * (qry * inv5 - 5.0 * q * inv7 * dy);
-    az += 0.5 * (qrz * inv5 - 5.0 * q * inv7 * dz);
+    const double q = qa.x * dx * dx + qa.y * dy * dy + qb.x * dz * dz +
+                     2.0 * (qb.y * dx * dy + qc.x * dx * dz + qc.y * dy * dz);
+    const double qrx = 2.0 * (qa.x * dx + qb.y * dy + qc.x * dz);
+    const double qry = 2.0 * (qb.y * dx + qa.y * dy + qc.y * dz);
+    const double qrz = 2.0 * (qc.x * dx + qc.y * dy + qb.x * dz);
+    RefTerm f;
+    f.mx = dx * fac; f.my = dy * fac; f.mz = dz * fac;
+    f.qx = 0.5 * (qrx * inv5 - 5.0 * q * inv7 * dx);
+    f.qy = 0.5 * (qry * inv5 - 5.0 * q * inv7 * dy);
+    f.qz = 0.5 * (qrz * inv5 - 5.0 * q * inv7 * dz);
+    return f;
 }
 
 __device__ __forceinline__ void add_stats(unsigned long long* stats, unsigned long long pp, unsigned long long pc) {
@@ -69,73 +62,127 @@ __device__ __forceinline__ void add_stats(unsigned long long* stats, unsigned lo
     }
 }
 
-__global__ void __launch_bounds__(128)
+// Reference physics.  The warp alternates between two phases: first every
+// lane runs its own depth-first walk with the opening tests only, until it has
+// a list of kRefList accepted nodes (or its walk is over); then all lanes
+// evaluate their lists in order.  The tests diverge but are cheap; the
+// evaluation (two square roots, two divisions, the quadrupole) runs with
+// nearly all lanes.
+//
+// Bound by FP64 latency: bhAccel's operations in bhAccel's order leave a chain
+// of four roots and divisions per interaction and no fused multiply-adds.
+// 1,048,576 bodies, a fifth of them dark matter: 5.81 -> 3.58 ms per walk (65,536
+// bodies 1.05 -> 0.63 ms) against one loop that tested and evaluated a node per
+// pass (13.7 of 32 lanes active) and took the node's cube root and the dark
+// bodies' power anew in every interaction.  Lists of 8 and 6 blocks per SM (80
+// registers) were the fastest of lists of 4-32 at 4-8 blocks; loading a sibling's
+// record while its predecessor is tested, or evaluating two entries at once,
+// cost more in registers than it hid (3.9-4.4 ms).
+constexpr int kRefThreads = 128;
+constexpr int kRefList = 8;
+constexpr unsigned kRefLeaf = 0x80000000u;                         // list entry: the node is a single body
+
+__global__ void __launch_bounds__(kRefThreads, 6)
 walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree t, Params P,
-                  unsigned long long* stats, int* err) {
+                      unsigned long long* stats, int* err) {
     if (*err & kErrAbort) return;
+    __shared__ unsigned list[kRefList][kRefThreads];
     const int64_t nodes = t.counts[1];
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const bool active = i < n && i >= P.own_lo && i < P.own_hi;
-    unsigned long long npp = 0, npc = 0;
-    if (active) {
-        const int root = sysid ? sysid[i] : 0;
-        const double xi = bd.x[i], yi = bd.y[i], zi = bd.z[i], mi = bd.m[i];
-        const int ti = bd.type[i];
-        const double theta = P.theta;
-        double ax = 0.0, ay = 0.0, az = 0.0;
-        int2 stack[kMaxLevel + 2];
-        int sp = 0;
-        int cur = root, end = root + 1;
-        for (;;) {
-            if (cur >= end) {
-                if (sp == 0) break;
+    const int64_t ii = active ? i : 0;
+    unsigned npp = 0, npc = 0;
+    const double xi = bd.x[ii], yi = bd.y[ii], zi = bd.z[ii], mi = bd.m[ii];
+    const bool dark = bd.type[ii] == 1;
+    // the mass whose dark-matter softening the upward pass stored per node
+    const bool stored = dark && mi == *t.dark_mass;
+    const double theta = P.theta, theta2 = theta * theta;
+    double ax = 0.0, ay = 0.0, az = 0.0;
+    int2 stack[kMaxLevel + 2];
+    int sp = 0;
+    int cur = sysid ? sysid[ii] : 0, end = active ? cur + 1 : cur;
+    while (__any_sync(0xffffffffu, cur < end || sp > 0)) {
+        int cnt = 0;
+        while (cnt < kRefList) {
+            while (cur >= end && sp > 0) {
                 --sp;
                 cur = stack[sp].x;
                 end = stack[sp].y;
-                continue;
             }
-            const int nd = cur++;
-            if (nd < 0 || nd >= nodes) { raise_error(err, kErrIndex); break; }
-            // the node's whole record in one round trip: centre of mass, link
-            // and the 8 moment words (quadrupole, size, critical radius), all
-            // issued before the first test uses any of them
-            const double4 c = t.com[nd];
-            const int2 lk = t.link[nd];
-            const double2* q2 = reinterpret_cast<const double2*>(t.quad64 + 8 * static_cast<int64_t>(nd));
-            const double2 qa = q2[0], qb = q2[1], qc = q2[2], qd = q2[3];
-            const double q64[8] = {qa.x, qa.y, qb.x, qb.y, qc.x, qc.y, qd.x, qd.y};
+            if (cur >= end) break;                                 // the walk is over
+            const int k = cur++;
+            if (k < 0 || k >= nodes) { raise_error(err, kErrIndex); cur = end; sp = 0; break; }
+            const double4 c = t.com[k];
+            const double2 head = t.soft[2 * static_cast<int64_t>(k)];    // half-width and link
+            const double size = head.x;
+            const int2 lk = make_int2(__double2loint(head.y), __double2hiint(head.y));
             if (c.w == 0.0) continue;
             const bool leaf = lk.y <= 0;
             if (leaf ? (lk.x < 0 || static_cast<int64_t>(lk.x) - lk.y > n) : (sp >= kMaxLevel + 1)) {
                 raise_error(err, leaf ? kErrIndex : kErrStack);
+                cur = end; sp = 0;
                 break;
             }
-            const int cnt = -lk.y;
-            if (leaf && cnt == 1 && lk.x == i) continue;          // own leaf (octree.h:135)
-            const double size = q64[6];
-            if (leaf && cnt > 1) {
+            if (!leaf) {
+                // size / dist < theta (octree.h:153), dist = sqrt(r2 + 1e-20): decided by the squares
+                // wherever they differ by more than the square root's and the division's rounding
+                // could hide, by the reference's own operations otherwise
+                const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
+                const double d2 = dx * dx + dy * dy + dz * dz + 1e-20;
+                const double s2 = size * size, t2 = theta2 * d2;
+                bool near = P.theta_squarable && s2 > t2 * (1.0 + 1e-14);
+                const bool far = P.theta_squarable && s2 < t2 * (1.0 - 1e-14);
+                if (!near && !far) near = !((size / sqrt(d2)) < theta);
+                if (near) {
+                    stack[sp++] = make_int2(cur, end);
+                    cur = lk.x;
+                    end = lk.x + lk.y;
+                } else {
+                    list[cnt++][threadIdx.x] = static_cast<unsigned>(k);
+                }
+            } else if (lk.y == -1) {
+                if (lk.x != i) list[cnt++][threadIdx.x] = static_cast<unsigned>(k) | kRefLeaf;   // not its own leaf (octree.h:135)
+            } else if (cnt > 0) {
+                --cur;                                             // a bucket follows the listed nodes: evaluate them first
+                break;
+            } else {
                 // deepest-level bucket: its bodies act as one-body leaves of this size
-                const double Z[6] = {0, 0, 0, 0, 0, 0};
-                for (int j = lk.x; j < lk.x + cnt; ++j) {
-                    if (j == i || bd.m[j] == 0.0) continue;
-                    ref_interact(bd.m[j], bd.x[j], bd.y[j], bd.z[j], size, Z, xi, yi, zi, mi, ti, ax, ay, az);
+                const double2 zero = make_double2(0.0, 0.0);
+                for (int j = lk.x; j < lk.x - lk.y; ++j) {
+                    const double mj = bd.m[j];
+                    if (j == i || mj == 0.0) continue;
+                    const double ex = bd.x[j] - xi, ey = bd.y[j] - yi, ez = bd.z[j] - zi;
+                    const double e2 = ex * ex + ey * ey + ez * ez;
+                    const RefTerm f = ref_term(mj, ex, ey, ez, e2, softening_base(size, mj),
+                                               dark ? softening_dark(size, mj, mi) : -1.0, zero, zero, zero);
+                    ax += f.mx; ay += f.my; az += f.mz;
+                    ax += f.qx; ay += f.qy; az += f.qz;
                     ++npp;
                 }
-                continue;
             }
+        }
+        __syncwarp();
+        for (int e = 0; e < cnt; ++e) {
+            const unsigned entry = list[e][threadIdx.x];
+            const bool leaf = entry & kRefLeaf;
+            const int64_t nd = entry & ~kRefLeaf;
+            const double4 c = t.com[nd];
+            const double2 soft = t.soft[2 * nd + 1];               // base and dark softening of the node
+            double2 qa = make_double2(0.0, 0.0), qb = qa, qc = qa; // a body has no quadrupole
+            const double2* q2 = reinterpret_cast<const double2*>(t.quad64 + 8 * nd);
+            if (!leaf) { qa = q2[0]; qb = q2[1]; qc = q2[2]; }
             const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            const double dist = sqrt(r2 + 1e-20);
-            if (leaf || (size / dist) < theta) {
-                const double Q[6] = {q64[0], q64[1], q64[2], q64[3], q64[4], q64[5]};
-                ref_interact(c.w, c.x, c.y, c.z, size, Q, xi, yi, zi, mi, ti, ax, ay, az);
-                if (leaf) ++npp; else ++npc;
-                continue;
-            }
-            stack[sp++] = make_int2(cur, end);
-            cur = lk.x;
-            end = lk.x + lk.y;
+            double sd = -1.0;
+            if (dark) sd = stored ? soft.y : softening_dark(t.soft[2 * nd].x, c.w, mi);
+            const RefTerm f = ref_term(c.w, dx, dy, dz, r2, soft.x, sd, qa, qb, qc);
+            ax += f.mx; ay += f.my; az += f.mz;
+            ax += f.qx; ay += f.qy; az += f.qz;
+            if (leaf) ++npp; else ++npc;
         }
+        __syncwarp();
+    }
+    if (active) {
         bd.ax[i] = ax; bd.ay[i] = ay; bd.az[i] = az;
         if (bd.pot) bd.pot[i] = 0.0;
     }
@@ -407,7 +454,7 @@ __global__ void direct_reduce_kernel(const double* __restrict__ partial, int64_t
 // The device softening law on k (size, mass, dist) triples (test support).
 __global__ void softening_kernel(const double* __restrict__ in, int64_t k, double* __restrict__ out) {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t < k) out[t] = next_softening(in[t], in[k + t], in[2 * k + t]);
+    if (t < k) out[t] = softening_at(softening_base(in[t], in[k + t]), in[2 * k + t]);
 }
 
 }  // namespace
@@ -430,8 +477,8 @@ cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int6
         auto kern = potential ? walk_accurate_kernel<true> : walk_accurate_kernel<false>;
         kern<<<blocks, 32 * kPlainWarps, 0, st>>>(bd, nsys > 1 ? offsets : nullptr, nsys, n, t, P, stats, err);
     } else {
-        const unsigned blocks = static_cast<unsigned>((n + 127) / 128);
-        walk_reference_kernel<<<blocks, 128, 0, st>>>(bd, sid, n, t, P, stats, err);
+        const unsigned blocks = static_cast<unsigned>((n + kRefThreads - 1) / kRefThreads);
+        walk_reference_kernel<<<blocks, kRefThreads, 0, st>>>(bd, sid, n, t, P, stats, err);
     }
     count_launches(1);
     return cudaGetLastError();

@@ -96,3 +96,63 @@ def test_accurate_walk_ensemble_of_odd_sizes():
             np.testing.assert_array_equal(a[c][offsets[i]:offsets[i + 1]], r[c])
         one.close()
     sim.close()
+
+
+def reference_bodies(n, seed):
+    b = ic.plummer(n, seed=seed)
+    rng = np.random.default_rng(seed)
+    b["type"][:] = rng.integers(0, 3, n)
+    return b
+
+
+@pytest.mark.parametrize("n,theta,masses", [
+    (1, 0.5, "equal"), (2, 0.5, "equal"), (9, 0.5, "equal"), (127, 0.5, "mixed"), (129, 0.3, "equal"),
+    (1001, 0.5, "mixed"), (4097, 0.5, "equal"), (4097, 0.05, "mixed"), (3000, 1.5, "equal"),
+])
+def test_reference_walk_sizes(oracle, n, theta, masses):
+    """Dark bodies of one mass (its softening stored per node) and of several (some computed per interaction),
+    lists and warps that end early: the oracle's forces up to the last bit of cbrt and pow (another opening decision
+    would move them by 1e-3 and more)."""
+    b = reference_bodies(n, n)
+    if masses == "mixed":
+        b["m"] *= np.random.default_rng(1).uniform(0.1, 3.0, n)
+        b["m"][::11] = 0.0
+    sim = Simulation("reference", "fp64", theta=theta)
+    sim.upload(b)
+    a = sim.accel()
+    r = oracle.accel(b, mode="ref", theta=theta)
+    assert sim.stats()["device_error"] == 0
+    if n > 1:
+        close(a, r, ("ax", "ay", "az"))
+    sim.close()
+
+
+def test_reference_walk_ties_and_buckets(oracle):
+    """A lattice, whose distances tie with the opening test's limit exactly, with coincident bodies among it."""
+    g = np.arange(12, dtype=np.float64) / 8.0
+    x, y, z = (v.ravel() for v in np.meshgrid(g, g, g, indexing="ij"))
+    b = reference_bodies(x.size, 3)
+    b["x"], b["y"], b["z"] = x.copy(), y.copy(), z.copy()
+    for k in ("x", "y", "z"):
+        b[k][500:520] = b[k][500]
+    for theta in (0.25, 0.5, 1.0):
+        sim = Simulation("reference", "fp64", theta=theta)
+        sim.upload(b)
+        a = sim.accel()
+        r = oracle.accel(b, mode="ref", theta=theta)
+        assert sim.stats()["device_error"] == 0
+        close(a, r, ("ax", "ay", "az"))
+        sim.close()
+
+
+def test_reference_walk_after_other_dark_masses(oracle):
+    """The stored softening follows the uploaded bodies: another upload with other masses, then one without dark bodies."""
+    sim = Simulation("reference", "fp64")
+    for seed, scale, kind in ((1, 1.0, 1), (2, 4.0, 1), (3, 0.5, 0)):
+        b = ic.plummer(600, seed=seed)
+        b["m"] *= scale
+        b["type"][::3] = kind
+        sim.upload(b)
+        a = sim.accel()
+        close(a, oracle.accel(b, mode="ref"), ("ax", "ay", "az"))
+    sim.close()
