@@ -55,9 +55,9 @@ struct Tree {
     int8_t* int_level;
     int32_t* int_bounds;   // 9 per q: child c spans [b[c], b[c+1])
     int64_t* int_packed;   // nchild | ngroups << 32 -> exclusive scan in place
-    int32_t* int_node;     // node id of q
     int32_t* counter;      // upward-pass arrivals (self-resetting)
-    int4* climb;           // node id, first child, child count | level << 8, start position
+    int4* climb;           // node id, first child, child count, parent's internal id (-1: a root)
+    double4* cell;         // centre (accurate physics) and half-width
     // per node
     int2* link;            // internal: (first child, nchild); leaf: (first body, -count)
     int32_t* parent;       // internal id of the parent (-1 for a root)
