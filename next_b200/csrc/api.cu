@@ -110,13 +110,10 @@ struct next_handle {
 
     // tree
     Tree t{};
-    void* scan_tmp = nullptr;
-    int64_t scan_tmp_elems = 0;
 
     // small device scalars
     int* err = nullptr;
     unsigned long long* stats = nullptr;   // pp, pc, max stack, spare
-    unsigned int* queue = nullptr;
     unsigned int* tickets = nullptr;       // 0: cubes, 1: dt, 2: diagnostics
     double* partial = nullptr;             // kReduceMax * 8
     double* dts = nullptr;                 // dt, dt/2
@@ -220,7 +217,7 @@ void free_tree(next_handle* h) {
     dfree(t.dlev); dfree(t.nint); dfree(t.int_start); dfree(t.int_level); dfree(t.int_bounds);
     dfree(t.int_packed); dfree(t.counter); dfree(t.climb); dfree(t.cell); dfree(t.ready); dfree(t.link); dfree(t.parent); dfree(t.level);
     dfree(t.com); dfree(t.quad64); dfree(t.box); dfree(t.quad32); dfree(t.soft); dfree(t.groups);
-    dfree(h->scan_tmp);
+    dfree(t.work);
     t.cap_int = t.cap_node = t.cap_group = 0;
 }
 
@@ -252,10 +249,7 @@ int alloc_tree(next_handle* h, int64_t cap_int) {
     if (h->P.physics == NEXT_PHYSICS_ACCURATE) { A(&t.box, t.cap_node); A(&t.quad32, 2 * t.cap_node); }
     else { A(&t.soft, 2 * t.cap_node); }
     A(&t.groups, t.cap_group);
-    h->scan_tmp_elems = scan_tile_sums_needed(std::max<int64_t>(n + 1, cap_int + 1));
-    int64_t* st64 = nullptr;
-    A(&st64, h->scan_tmp_elems);
-    h->scan_tmp = st64;
+    A(&t.work, tree_work_words(n, cap_int));
     if (e != cudaSuccess) return cuda_fail(h, e, "tree allocation");
     NB_TRY(cudaMemsetAsync(t.counter, 0, sizeof(int32_t) * cap_int, h->st), "tree counters");
     NB_TRY(cudaMemsetAsync(t.link, 0, sizeof(int2) * t.cap_node, h->st), "tree links");
@@ -360,7 +354,7 @@ int build(next_handle* h, std::vector<int>* evs) {
     NB_TRY(launch_gather_bodies(h->buf[h->cur].b, dst, sidx, n, h->inv, h->err, h->st), "reorder");
     h->cur = other;
     Bodies bd = h->cur_bodies();
-    NB_TRY(build_tree(skeys, n, bd, h->sysid, h->sys, h->d_offsets, h->P, h->t, h->scan_tmp, h->err, h->st),
+    NB_TRY(build_tree(skeys, n, bd, h->sysid, h->sys, h->d_offsets, h->P, h->t, h->sm_count, h->err, h->st),
            "tree build");
     h->forces_valid = false;
     return record(h, evs);
@@ -376,7 +370,7 @@ int walk(next_handle* h, bool potential) {
     Bodies bd = h->cur_bodies();
     if (group_walk(h)) {
         NB_TRY(launch_walk_group(bd, h->n, h->t, h->P, potential, h->prm.precision == NEXT_PRECISION_FP64_GROUP,
-                                 h->prm.walk_warps, h->prm.walk_stack, h->queue, h->stats, h->err, h->sm_count, h->st),
+                                 h->prm.walk_warps, h->prm.walk_stack, h->stats, h->err, h->sm_count, h->st),
                "group walk");
     } else {
         NB_TRY(launch_walk_plain(bd, h->sysid, h->d_offsets, h->nsys, h->n, h->t, h->P, potential, h->stats, h->err,
@@ -749,14 +743,14 @@ int next_create(const next_params* p, next_handle** out) {
     e = sort_prepare();
     if (e != cudaSuccess) return bail(e, "sort setup");
     auto A = [&](auto** q, size_t c) { if (e == cudaSuccess) e = dalloc(q, c); };
-    A(&h->err, 1); A(&h->stats, 4); A(&h->queue, 1); A(&h->tickets, 4); A(&h->partial, kReduceMax * 8);
+    A(&h->err, 1); A(&h->stats, 4); A(&h->tickets, 4); A(&h->partial, kReduceMax * 8);
     A(&h->dts, 2); A(&h->dt_out, 2); A(&h->diag, 8); A(&h->changed, 4); A(&h->fma_out, 1);
-    A(&h->t.counts, 6); A(&h->t.dark_mass, 1); A(&h->done, 1);
+    A(&h->t.counts, 4); A(&h->t.dark_mass, 1); A(&h->done, 1);
     if (e != cudaSuccess) return bail(e, "scalars");
     e = cudaMemset(h->err, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(h->tickets, 0, sizeof(unsigned int) * 4);
     if (e == cudaSuccess) e = cudaMemset(h->stats, 0, sizeof(unsigned long long) * 4);
-    if (e == cudaSuccess) e = cudaMemset(h->t.counts, 0, sizeof(int64_t) * 6);
+    if (e == cudaSuccess) e = cudaMemset(h->t.counts, 0, sizeof(int64_t) * 4);
     if (e == cudaSuccess) e = cudaMemset(h->t.dark_mass, 0xff, sizeof(double));   // NaN
     if (e == cudaSuccess) e = cudaMemset(h->done, 0, sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_dts), sizeof(double) * 2, cudaHostAllocDefault);
@@ -784,7 +778,7 @@ void next_destroy(next_handle* h) {
     nccl_comm_destroy(h->comm);
     h->comm = nullptr;
     free_bodies(h);
-    dfree(h->err); dfree(h->stats); dfree(h->queue); dfree(h->tickets); dfree(h->partial);
+    dfree(h->err); dfree(h->stats); dfree(h->tickets); dfree(h->partial);
     dfree(h->dts); dfree(h->dt_out); dfree(h->diag); dfree(h->changed); dfree(h->fma_out); dfree(h->t.counts); dfree(h->t.dark_mass);
     dfree(h->done);
     dfree(h->d_targets); dfree(h->d_targetpos); dfree(h->d_direct_partial); dfree(h->d_direct_out);

@@ -44,6 +44,8 @@ struct Systems {
 // last key level (a leaf over capacity: the keys need more levels)
 constexpr unsigned kDepthOverfull = 64;
 
+constexpr int kTreeWorkQueue = 4;      // word of Tree::work the group walk counts its groups in
+
 struct Tree {
     // capacities
     int64_t cap_int, cap_node, cap_group;
@@ -73,8 +75,9 @@ struct Tree {
     int4* groups;          // (first body, count, root node, 0)
     int32_t* ready;        // upward pass: internal ids whose children are all leaves
     // device scalars: [0] internal count, [1] node count, [2] group count,
-    // [3] deepest leaf level, [4] ready-list length
+    // [3] deepest leaf level
     int64_t* counts;
+    unsigned long long* work;  // zeroed by every build: tickets, counters, the walk's queue, look-back statuses
 };
 
 struct Params {

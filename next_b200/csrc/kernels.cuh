@@ -32,16 +32,10 @@ cudaError_t radix_sort_pairs_to(const uint64_t* keys_in, const uint32_t* vals_in
                                 uint32_t* vals_out, uint64_t* alt_keys, uint32_t* alt_vals, int64_t n, int key_bits,
                                 uint32_t* scratch, int* err, cudaStream_t st);
 
-// scan.cu
-template <typename T>
-cudaError_t exclusive_scan(const T* in, T* out, int64_t n_cap, const int64_t* count_dev, T* tile_sums,
-                           int64_t* total_dev, cudaStream_t st);
-int64_t scan_tile_sums_needed(int64_t n_cap);
-
 // tree.cu
 cudaError_t build_tree(const uint64_t* keys, int64_t n, const Bodies& bd, const int32_t* sysid, const Systems& sys,
-                       const int64_t* d_offsets, const Params& P, Tree& t, void* scan_tmp, int* err,
-                       cudaStream_t st);
+                       const int64_t* d_offsets, const Params& P, Tree& t, int sm_count, int* err, cudaStream_t st);
+int64_t tree_work_words(int64_t n, int64_t cap_int);   // words of Tree::work for n bodies and cap_int internal cells
 
 // walk_plain.cu
 cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int64_t* offsets, int nsys, int64_t n,
@@ -56,8 +50,8 @@ cudaError_t launch_direct(const Bodies& bd, int64_t n, const int64_t* targets, i
 // walk_group.cu: the warp-per-group walk, FP32-mixed or FP64 arithmetic
 size_t walk_group_smem(bool fp64, int warps, int stack_cap);
 cudaError_t launch_walk_group(const Bodies& bd, int64_t nbodies, const Tree& t, const Params& P, bool potential,
-                              bool fp64, int warps, int stack_cap, unsigned int* queue, unsigned long long* stats,
-                              int* err, int sm_count, cudaStream_t st);
+                              bool fp64, int warps, int stack_cap, unsigned long long* stats, int* err, int sm_count,
+                              cudaStream_t st);
 
 // integrate.cu
 cudaError_t launch_gather_bodies(const Bodies& src, const Bodies& dst, const uint32_t* idx, int64_t n, uint32_t* inv,

@@ -33,49 +33,127 @@
 // reference-mode moments repeat src/gravity/octree.h:92-127 bit for bit.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "scan.cuh"
 #include "softening.cuh"
 
 namespace nb {
 
 namespace {
 
-__global__ void dlev_kernel(const uint64_t* __restrict__ keys, int64_t n, int base, int levels,
-                            int8_t* __restrict__ dlev) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    dlev[s] = static_cast<int8_t>(s == 0 ? -1 : shared_levels(keys[s - 1], keys[s], base, levels));
-}
+// Words of Tree::work, zeroed at the start of every build: two tile tickets,
+// the ready-list length, the deepest leaf level, the group walk's queue, then
+// the look-back statuses of the two scans.
+constexpr int kWorkCells = 0, kWorkChildren = 1, kWorkReady = 2, kWorkDeepest = 3, kWorkStatus = 5;
+static_assert(kTreeWorkQueue == 4, "the queue's word");
 
-// Internal cells starting at each position; *deepest gets the deepest leaf
-// level (one below the deepest internal cell) of the build, or
-// kDepthOverfull if a cell at the last key level holds more than leaf_cap.
-__global__ void nint_kernel(const int8_t* __restrict__ dlev, int64_t n, int leaf_cap, int levels,
-                            int32_t* __restrict__ nint, unsigned long long* deepest) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    unsigned deep = 0;
-    if (s < n) {
-        int mb = -1;
-        if (s + leaf_cap < n) {
-            mb = 127;
-            for (int j = 1; j <= leaf_cap; ++j) mb = min(mb, static_cast<int>(dlev[s + j]));
-        }
-        const int top = min(mb, levels - 1);
-        const int c = max(0, top - static_cast<int>(dlev[s]));
-        nint[s] = c;
-        if (c > 0) deep = static_cast<unsigned>(top + 1);
-        if (mb >= levels) deep = kDepthOverfull;
+// Internal cells per position, their ids and records, in one pass: d[s] for a
+// tile of positions and the leaf_cap behind it (in shared memory), the counts,
+// their scan over the tile and the tiles before it, and the cells themselves.
+// work[kWorkDeepest] gets the deepest leaf level (one below the deepest
+// internal cell) of the build, or kDepthOverfull if a cell at the last key
+// level holds more than leaf_cap.
+//
+// Six launches (d, counts, three of a scan, cells) took 2.5-3 us each on small
+// systems and re-read their arrays on large ones.  With the child counts' scan
+// below in one launch too (five before): build 0.138 -> 0.123 ms at 16,384
+// bodies, 0.246 -> 0.228 ms at 1,048,576, 2.79 -> 2.71 ms at 16.7 M.
+constexpr int kCellThreads = 256, kCellItems = 4, kCellTile = kCellThreads * kCellItems;
+constexpr int kMaxLeafCap = 64;
+
+__global__ void __launch_bounds__(kCellThreads)
+cells_kernel(const uint64_t* __restrict__ keys, int64_t n, int base, int levels, int leaf_cap, Tree t, int* err) {
+    __shared__ int8_t d[kCellTile + kMaxLeafCap + 1];
+    __shared__ unsigned long long before;
+    __shared__ int ticket;
+    __shared__ unsigned deepest;
+    if (threadIdx.x == 0) {
+        ticket = static_cast<int>(atomicAdd(t.work + kWorkCells, 1ull));
+        deepest = 0;
     }
-    // block maximum, then one atomic per block, skipped when it cannot raise
-    // the value (one hot address: unconditional atomics cost more than the pass)
-    __shared__ unsigned warp_max[32];
-    deep = __reduce_max_sync(0xffffffffu, deep);
-    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = deep;
     __syncthreads();
+    const int tile = ticket;
+    const int64_t s0 = static_cast<int64_t>(tile) * kCellTile;
+    // positions past the last body get -1: no run of equal prefixes crosses the end
+    for (int p = threadIdx.x; p <= kCellTile + leaf_cap; p += kCellThreads) {
+        const int64_t s = s0 + p;
+        d[p] = static_cast<int8_t>(s == 0 || s >= n ? -1 : shared_levels(keys[s - 1], keys[s], base, levels));
+    }
+    __syncthreads();
+    // the thread's positions p0 .. p0 + 3; window of position p0 + i: p0 + i + 1 .. p0 + i + leaf_cap
+    const int p0 = threadIdx.x * kCellItems;
+    int own[kCellItems], cnt[kCellItems];
+#pragma unroll
+    for (int i = 0; i < kCellItems; ++i) own[i] = d[p0 + i];
+    int win[kCellItems];
+    if (leaf_cap >= kCellItems) {
+        int core = 127;                                    // what all four windows share
+        for (int p = p0 + kCellItems; p <= p0 + leaf_cap; ++p) core = min(core, static_cast<int>(d[p]));
+#pragma unroll
+        for (int i = 0; i < kCellItems; ++i) {
+            win[i] = core;
+#pragma unroll
+            for (int k = 1; k < kCellItems; ++k) {
+                if (k > i) win[i] = min(win[i], own[k]);
+                if (k <= i) win[i] = min(win[i], static_cast<int>(d[p0 + leaf_cap + k]));
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < kCellItems; ++i) {
+            win[i] = 127;
+            for (int j = 1; j <= leaf_cap; ++j) win[i] = min(win[i], static_cast<int>(d[p0 + i + j]));
+        }
+    }
+    unsigned deep = 0;
+    unsigned long long mine = 0;
+#pragma unroll
+    for (int i = 0; i < kCellItems; ++i) {
+        const int top = min(win[i], levels - 1);
+        cnt[i] = s0 + p0 + i < n ? max(0, top - own[i]) : 0;
+        mine += static_cast<unsigned>(cnt[i]);
+        if (cnt[i] > 0) deep = max(deep, static_cast<unsigned>(top + 1));
+        if (s0 + p0 + i < n && win[i] >= levels) deep = kDepthOverfull;
+    }
+    deep = __reduce_max_sync(0xffffffffu, deep);
+    if ((threadIdx.x & 31) == 0 && deep) atomicMax(&deepest, deep);
+    unsigned long long sum;
+    const unsigned long long ex = block_exclusive<kCellThreads>(mine, &sum);
     if (threadIdx.x < 32) {
-        unsigned v = threadIdx.x < (blockDim.x >> 5) ? warp_max[threadIdx.x] : 0u;
-        v = __reduce_max_sync(0xffffffffu, v);
-        if (threadIdx.x == 0 && v > *reinterpret_cast<volatile unsigned long long*>(deepest))
-            atomicMax(deepest, static_cast<unsigned long long>(v));
+        const unsigned long long b = look_back(t.work + kWorkStatus, tile, sum, err);
+        if (threadIdx.x == 0) before = b;
+    }
+    __syncthreads();
+    int64_t q = static_cast<int64_t>(before + ex);
+    int first[kCellItems];
+#pragma unroll
+    for (int i = 0; i < kCellItems; ++i) { first[i] = static_cast<int>(q); q += cnt[i]; }
+    const int64_t s = s0 + p0;
+    if (s + kCellItems <= n) {
+        *reinterpret_cast<int4*>(t.nint + s) = make_int4(first[0], first[1], first[2], first[3]);
+        *reinterpret_cast<char4*>(t.dlev + s) = make_char4(own[0], own[1], own[2], own[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kCellItems; ++i)
+            if (s + i < n) { t.nint[s + i] = first[i]; t.dlev[s + i] = static_cast<int8_t>(own[i]); }
+    }
+#pragma unroll
+    for (int i = 0; i < kCellItems; ++i) {
+        for (int k = 0; k < cnt[i]; ++k) {
+            const int64_t c = static_cast<int64_t>(first[i]) + k;
+            if (c >= t.cap_int) { raise_error(err, kErrTree); break; }
+            t.int_start[c] = static_cast<int32_t>(s + i);
+            t.int_level[c] = static_cast<int8_t>(own[i] + 1 + k);
+        }
+    }
+    if (threadIdx.x == 0) {
+        // skipped where it cannot raise the value: one hot address
+        unsigned long long* all = t.work + kWorkDeepest;
+        if (deepest > *reinterpret_cast<volatile unsigned long long*>(all))
+            atomicMax(all, static_cast<unsigned long long>(deepest));
+        if (s0 + kCellTile >= n) {
+            t.nint[n] = static_cast<int32_t>(before + sum);
+            t.counts[0] = static_cast<int64_t>(before + sum);
+        }
     }
 }
 
@@ -115,120 +193,119 @@ __device__ int pack_groups(const int32_t* b, int level, int levels, int leaf_cap
     return ng;
 }
 
-// Internal cell ids: position s starts the cells q = int_base[s] + k at
-// levels dlev[s] + 1 + k.  Compacts them so the search kernel below runs one
-// thread per cell rather than per position.
-__global__ void cell_starts_kernel(const int8_t* __restrict__ dlev, const int32_t* __restrict__ int_base,
-                                   int64_t n, Tree t, int* err) {
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const int q0 = int_base[s];
-    const int cnt = int_base[s + 1] - q0;
-    if (cnt == 0) return;
-    const int d = dlev[s];
-    for (int k = 0; k < cnt; ++k) {
-        const int64_t q = static_cast<int64_t>(q0) + k;
-        if (q >= t.cap_int) { raise_error(err, kErrTree); return; }
-        t.int_start[q] = static_cast<int32_t>(s);
-        t.int_level[q] = static_cast<int8_t>(d + 1 + k);
-    }
-}
-
 // Child boundaries of every internal cell (l, s): the cell ends at the first
 // key above its prefix, and child c starts at the first key >= prefix | c at
 // level l+1.  All eight are lower bounds over the same range [s, system end),
 // run together with one shared step sequence (the range halves every step
 // whatever the comparisons give), so a thread has eight independent loads in
-// flight per step and no divergence.
+// flight per step and no divergence.  The counts of children and walk groups
+// are scanned here too (tiles of cells by ticket, look-back between them); the
+// last tile checks the totals.
 #ifndef NB_INT_SCAN
 #define NB_INT_SCAN 128
 #endif
-__global__ void __launch_bounds__(256)
+// The child bounds of cell q, stored, and its counts of children and groups.
+__device__ __forceinline__ void find_children(const uint64_t* __restrict__ keys, int64_t n,
+                                              const int32_t* __restrict__ sysid, const int64_t* __restrict__ offsets,
+                                              int base, int levels, int leaf_cap, int group_cap, int64_t q, Tree& t,
+                                              int* err, int* nchild, int* ngroups) {
+    const int s = t.int_start[q];
+    const int l = t.int_level[q];
+    if (s < 0 || s >= n || l < 0 || l >= levels) { raise_error(err, kErrIndex); return; }
+    const int64_t hi = offsets ? offsets[(sysid ? sysid[s] : 0) + 1] : n;
+    const uint64_t ks = keys[s];
+    const int sh = base - 3 * l;                       // bits below level l's digits
+    const uint64_t low = (sh >= 64) ? ~0ull : ((1ull << sh) - 1ull);
+    const uint64_t prefix = ks & ~low;
+    const int csh = sh - 3;
+    uint64_t v[8];
+    v[0] = (prefix | low) + 1ull;                      // end of the cell
+#pragma unroll
+    for (int c = 1; c < 8; ++c) v[c] = prefix | (static_cast<uint64_t>(c) << csh);
+    // A small cell's end is the first p > s whose key shares fewer than l
+    // digits with its predecessor (dlev[p] < l): found by reading dlev
+    // forward, 16 positions per round trip, for up to NB_INT_SCAN
+    // positions; the children's searches then run over the cell only.
+    int64_t e = -1;
+    if (NB_INT_SCAN > 0) {
+        const int64_t lim = hi < static_cast<int64_t>(s) + 1 + NB_INT_SCAN ? hi : static_cast<int64_t>(s) + 1 + NB_INT_SCAN;
+        for (int64_t p0 = static_cast<int64_t>(s) + 1; p0 < lim && e < 0; p0 += 16) {
+            int dv[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dv[j] = p0 + j < lim ? t.dlev[p0 + j] : 127;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (e < 0 && dv[j] < l) e = p0 + j;
+        }
+        if (e < 0 && lim == hi) e = hi;
+    }
+    int64_t pos[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) pos[c] = s;
+    int64_t len = (e >= 0 ? e : hi) - s;
+    while (len > 1) {
+        const int64_t half = len >> 1;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) pos[c] = __ldg(keys + pos[c] + half) < v[c] ? pos[c] + half : pos[c];
+        len -= half;
+    }
+    int32_t b[9];
+    b[0] = s;
+#pragma unroll
+    for (int c = 1; c < 8; ++c) b[c] = static_cast<int32_t>(pos[c] + (__ldg(keys + pos[c]) < v[c] ? 1 : 0));
+    b[8] = e >= 0 ? static_cast<int32_t>(e) : static_cast<int32_t>(pos[0] + (__ldg(keys + pos[0]) < v[0] ? 1 : 0));
+    for (int c = 0; c < 8; ++c) *nchild += b[c + 1] > b[c];
+    if (b[8] - b[0] > group_cap)
+        *ngroups = pack_groups(b, l, levels, leaf_cap, group_cap, [](int, int) {});
+    for (int c = 0; c < 9; ++c) t.int_bounds[9 * q + c] = b[c];
+}
+
+constexpr int kChildThreads = 256;
+__global__ void __launch_bounds__(kChildThreads)
 internal_kernel(const uint64_t* __restrict__ keys, int64_t n, const int32_t* __restrict__ sysid,
-                const int64_t* __restrict__ offsets, int base, int levels, int leaf_cap, int group_cap, Tree t,
-                int* err) {
-    if (*err & kErrAbort) return;
+                const int64_t* __restrict__ offsets, int nsys, int base, int levels, int leaf_cap, int group_cap,
+                int64_t status_at, Tree t, int* err) {
+    if (*err & kErrAbort) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            t.counts[1] = t.counts[2] = nsys;
+            t.counts[3] = static_cast<int64_t>(t.work[kWorkDeepest]);
+        }
+        return;
+    }
+    __shared__ unsigned long long before;
+    __shared__ int ticket;
     const int64_t m = t.counts[0] < t.cap_int ? t.counts[0] : t.cap_int;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
-        const int s = t.int_start[q];
-        const int l = t.int_level[q];
-        if (s < 0 || s >= n || l < 0 || l >= levels) { raise_error(err, kErrIndex); continue; }
-        const int64_t hi = offsets ? offsets[(sysid ? sysid[s] : 0) + 1] : n;
-        const uint64_t ks = keys[s];
-        const int sh = base - 3 * l;                       // bits below level l's digits
-        const uint64_t low = (sh >= 64) ? ~0ull : ((1ull << sh) - 1ull);
-        const uint64_t prefix = ks & ~low;
-        const int csh = sh - 3;
-        uint64_t v[8];
-        v[0] = (prefix | low) + 1ull;                      // end of the cell
-#pragma unroll
-        for (int c = 1; c < 8; ++c) v[c] = prefix | (static_cast<uint64_t>(c) << csh);
-        // A small cell's end is the first p > s whose key shares fewer than l
-        // digits with its predecessor (dlev[p] < l): found by reading dlev
-        // forward, 16 positions per round trip, for up to NB_INT_SCAN
-        // positions; the children's searches then run over the cell only.
-        int64_t e = -1;
-        if (NB_INT_SCAN > 0) {
-            const int64_t lim = hi < static_cast<int64_t>(s) + 1 + NB_INT_SCAN ? hi : static_cast<int64_t>(s) + 1 + NB_INT_SCAN;
-            for (int64_t p0 = static_cast<int64_t>(s) + 1; p0 < lim && e < 0; p0 += 16) {
-                int dv[16];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) dv[j] = p0 + j < lim ? t.dlev[p0 + j] : 127;
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (e < 0 && dv[j] < l) e = p0 + j;
-            }
-            if (e < 0 && lim == hi) e = hi;
+    for (;;) {
+        __syncthreads();
+        if (threadIdx.x == 0) ticket = static_cast<int>(atomicAdd(t.work + kWorkChildren, 1ull));
+        __syncthreads();
+        const int tile = ticket;
+        const int64_t q0 = static_cast<int64_t>(tile) * kChildThreads;
+        if (q0 >= m && tile > 0) break;
+        const int64_t q = q0 + threadIdx.x;
+        int nchild = 0, ngroups = 0;
+        if (q < m)
+            find_children(keys, n, sysid, offsets, base, levels, leaf_cap, group_cap, q, t, err, &nchild, &ngroups);
+        unsigned long long sum;
+        const unsigned long long ex = block_exclusive<kChildThreads>(
+            static_cast<unsigned long long>(nchild) | (static_cast<unsigned long long>(ngroups) << 32), &sum);
+        if (threadIdx.x < 32) {
+            const unsigned long long b = look_back(t.work + status_at, tile, sum, err);
+            if (threadIdx.x == 0) before = b;
         }
-        int64_t pos[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) pos[c] = s;
-        int64_t len = (e >= 0 ? e : hi) - s;
-        while (len > 1) {
-            const int64_t half = len >> 1;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) pos[c] = __ldg(keys + pos[c] + half) < v[c] ? pos[c] + half : pos[c];
-            len -= half;
+        __syncthreads();
+        if (q < m) t.int_packed[q] = static_cast<int64_t>(before + ex);
+        if (threadIdx.x == 0 && q0 + kChildThreads >= m) {
+            const unsigned long long all = before + sum;
+            t.int_packed[m] = static_cast<int64_t>(all);
+            const int64_t nodes = nsys + static_cast<int64_t>(all & 0xffffffffull);
+            const int64_t groups = nsys + static_cast<int64_t>(all >> 32);
+            if (nodes > t.cap_node || groups > t.cap_group) raise_error(err, kErrTree);
+            t.counts[1] = nodes < t.cap_node ? nodes : t.cap_node;
+            t.counts[2] = groups < t.cap_group ? groups : t.cap_group;
+            t.counts[3] = static_cast<int64_t>(t.work[kWorkDeepest]);
         }
-        int32_t b[9];
-        b[0] = s;
-#pragma unroll
-        for (int c = 1; c < 8; ++c) b[c] = static_cast<int32_t>(pos[c] + (__ldg(keys + pos[c]) < v[c] ? 1 : 0));
-        b[8] = e >= 0 ? static_cast<int32_t>(e) : static_cast<int32_t>(pos[0] + (__ldg(keys + pos[0]) < v[0] ? 1 : 0));
-        int nchild = 0;
-        for (int c = 0; c < 8; ++c) nchild += b[c + 1] > b[c];
-        int ngroups = 0;
-        if (b[8] - b[0] > group_cap)
-            ngroups = pack_groups(b, l, levels, leaf_cap, group_cap, [](int, int) {});
-        for (int c = 0; c < 9; ++c) t.int_bounds[9 * q + c] = b[c];
-        t.int_packed[q] = static_cast<int64_t>(nchild) | (static_cast<int64_t>(ngroups) << 32);
     }
-}
-
-__global__ void check_counts_kernel(int nsys, Tree t, int* err) {
-    const int64_t m = t.counts[0];
-    if (m > t.cap_int) { raise_error(err, kErrTree); t.counts[1] = nsys; t.counts[2] = nsys; return; }
-    const int64_t packed = t.int_packed[m];
-    const int64_t nodes = nsys + (packed & 0xffffffffll);
-    const int64_t groups = nsys + (packed >> 32);
-    if (nodes > t.cap_node || groups > t.cap_group) raise_error(err, kErrTree);
-    t.counts[1] = nodes < t.cap_node ? nodes : t.cap_node;
-    t.counts[2] = groups < t.cap_group ? groups : t.cap_group;
-}
-
-__global__ void roots_kernel(const int64_t* __restrict__ offsets, int64_t n, int nsys, int leaf_cap,
-                             int group_cap, Tree t) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsys) return;
-    const int64_t b = offsets ? offsets[s] : 0;
-    const int64_t e = offsets ? offsets[s + 1] : n;
-    const int cnt = static_cast<int>(e - b);
-    if (cnt <= leaf_cap) {
-        t.link[s] = make_int2(static_cast<int>(b), -cnt);
-        t.parent[s] = -1;
-        t.level[s] = 0;
-    }
-    t.groups[s] = make_int4(static_cast<int>(b), cnt <= group_cap ? cnt : 0, s, 0);
 }
 
 // Geometric centre of the level-l cell holding `key` (the reference's child
@@ -248,9 +325,22 @@ __device__ double3 cell_centre(uint64_t key, int level, double4 cube, int base) 
 
 __global__ void children_kernel(const uint64_t* __restrict__ keys, const int8_t* __restrict__ dlev,
                                 const int32_t* __restrict__ int_base, const int32_t* __restrict__ sysid,
-                                const double4* __restrict__ cubes, int nsys, int base, int levels, int leaf_cap,
-                                int group_cap, bool accurate, Tree t, int* err) {
+                                const int64_t* __restrict__ offsets, const double4* __restrict__ cubes, int64_t n,
+                                int nsys, int base, int levels, int leaf_cap, int group_cap, bool accurate, Tree t,
+                                int* err) {
     if (*err & kErrAbort) return;
+    // the system roots: leaves here, internal ones by their cell below
+    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < nsys; s += gridDim.x * blockDim.x) {
+        const int64_t b = offsets ? offsets[s] : 0;
+        const int64_t e = offsets ? offsets[s + 1] : n;
+        const int cnt = static_cast<int>(e - b);
+        if (cnt <= leaf_cap) {
+            t.link[s] = make_int2(static_cast<int>(b), -cnt);
+            t.parent[s] = -1;
+            t.level[s] = 0;
+        }
+        t.groups[s] = make_int4(static_cast<int>(b), cnt <= group_cap ? cnt : 0, s, 0);
+    }
     const int64_t m = t.counts[0];
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
         const int l = t.int_level[q];
@@ -617,7 +707,7 @@ upward_leaves_kernel(Bodies bd, int64_t nbodies, const uint64_t* __restrict__ ke
         if (!climb_record_check(nodes, rec, err)) continue;
         if (atomicAdd(t.counter + q, 1) == rec.z - 1) {
             t.counter[q] = 0;
-            const unsigned long long slot = atomicAdd(reinterpret_cast<unsigned long long*>(t.counts + 4), 1ull);
+            const unsigned long long slot = atomicAdd(t.work + kWorkReady, 1ull);
             if (slot < static_cast<unsigned long long>(t.cap_int)) t.ready[slot] = q;
             else raise_error(err, kErrIndex);
         }
@@ -642,7 +732,8 @@ upward_climb_kernel(Params P, Tree t, int* err) {
     if (*err & kErrAbort) return;
     const int64_t nodes = t.counts[1];
     const int64_t ninternal = t.counts[0];
-    const int64_t nready = t.counts[4] < t.cap_int ? t.counts[4] : t.cap_int;
+    const int64_t listed = static_cast<int64_t>(t.work[kWorkReady]);
+    const int64_t nready = listed < t.cap_int ? listed : t.cap_int;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nready;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int q = t.ready[i];
@@ -652,39 +743,31 @@ upward_climb_kernel(Params P, Tree t, int* err) {
 }
 }  // namespace
 
+int64_t tree_work_words(int64_t n, int64_t cap_int) {
+    return kWorkStatus + n / kCellTile + 1 + cap_int / kChildThreads + 1;
+}
+
 cudaError_t build_tree(const uint64_t* keys, int64_t n, const Bodies& bd, const int32_t* sysid,
-                       const Systems& sys, const int64_t* d_offsets, const Params& P, Tree& t,
-                       void* scan_tmp, int* err, cudaStream_t st) {
+                       const Systems& sys, const int64_t* d_offsets, const Params& P, Tree& t, int sm_count, int* err,
+                       cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
     const int threads = 256;
-    const unsigned blocks = static_cast<unsigned>((n + threads - 1) / threads);
     const int leaf_cap = P.physics == NEXT_PHYSICS_REFERENCE ? 1 : P.leaf_cap;
     const int group_cap = P.group_cap < leaf_cap ? leaf_cap : P.group_cap;
     const int32_t* sid = sys.n > 1 ? sysid : nullptr;
     const int64_t* offs = sys.n > 1 ? d_offsets : nullptr;
-    cudaError_t e0 = cudaMemsetAsync(t.counts + 3, 0, 2 * sizeof(int64_t), st);
-    if (e0 != cudaSuccess) return e0;
-    if (n > 0) {
-        dlev_kernel<<<blocks, threads, 0, st>>>(keys, n, sys.base, sys.levels, t.dlev);
-        nint_kernel<<<blocks, threads, 0, st>>>(t.dlev, n, leaf_cap, sys.levels, t.nint,
-                                                reinterpret_cast<unsigned long long*>(t.counts + 3));
-    }
-    cudaError_t e = exclusive_scan<int32_t>(t.nint, t.nint, n, nullptr, static_cast<int32_t*>(scan_tmp),
-                                            t.counts + 0, st);
+    cudaError_t e = cudaMemsetAsync(t.work, 0, sizeof(unsigned long long) * tree_work_words(n, t.cap_int), st);
     if (e != cudaSuccess) return e;
-    if (n > 0) {
-        cell_starts_kernel<<<blocks, threads, 0, st>>>(t.dlev, t.nint, n, t, err);
-        const unsigned iblocks = static_cast<unsigned>((t.cap_int + threads - 1) / threads);
-        internal_kernel<<<iblocks < 4096u ? (iblocks ? iblocks : 1u) : 4096u, threads, 0, st>>>(
-            keys, n, sid, offs, sys.base, sys.levels, leaf_cap, group_cap, t, err);
-    }
-    e = exclusive_scan<int64_t>(t.int_packed, t.int_packed, t.cap_int, t.counts + 0,
-                                static_cast<int64_t*>(scan_tmp), nullptr, st);
-    if (e != cudaSuccess) return e;
-    check_counts_kernel<<<1, 1, 0, st>>>(sys.n, t, err);
-    roots_kernel<<<(sys.n + 127) / 128, 128, 0, st>>>(offs, n, sys.n, leaf_cap, group_cap, t);
+    const unsigned tiles = static_cast<unsigned>((n + kCellTile - 1) / kCellTile);
+    cells_kernel<<<tiles, kCellThreads, 0, st>>>(keys, n, sys.base, sys.levels, leaf_cap, t, err);
+    const int64_t itiles = (t.cap_int + kChildThreads - 1) / kChildThreads;
+    const int64_t resident = 4 * static_cast<int64_t>(sm_count);
+    const int64_t status_at = kWorkStatus + n / kCellTile + 1;
+    internal_kernel<<<static_cast<unsigned>(itiles < resident ? (itiles ? itiles : 1) : resident), kChildThreads, 0, st>>>(
+        keys, n, sid, offs, sys.n, sys.base, sys.levels, leaf_cap, group_cap, status_at, t, err);
     const unsigned cblocks = static_cast<unsigned>((t.cap_int + threads - 1) / threads);
     children_kernel<<<cblocks < 4096u ? (cblocks ? cblocks : 1u) : 4096u, threads, 0, st>>>(
-        keys, t.dlev, t.nint, sid, sys.cube, sys.n, sys.base, sys.levels, leaf_cap, group_cap,
+        keys, t.dlev, t.nint, sid, offs, sys.cube, n, sys.n, sys.base, sys.levels, leaf_cap, group_cap,
         P.physics == NEXT_PHYSICS_ACCURATE, t, err);
     const unsigned ublocks = static_cast<unsigned>((t.cap_node + threads - 1) / threads);
     Params Pu = P;
@@ -698,8 +781,7 @@ cudaError_t build_tree(const uint64_t* keys, int64_t n, const Bodies& bd, const 
     const unsigned cgrid = static_cast<unsigned>(cl < 8192 ? (cl ? cl : 1) : 8192);
     if (acc) upward_climb_kernel<true><<<cgrid, kClimbThreads, 0, st>>>(Pu, t, err);
     else upward_climb_kernel<false><<<cgrid, kClimbThreads, 0, st>>>(Pu, t, err);
-    count_launches(1);
-    count_launches(n > 0 ? 9 : 5);
+    count_launches(5);
     return cudaGetLastError();
 }
 

@@ -647,8 +647,9 @@ struct Fp64Arith {
 template <class A>
 __global__ void __launch_bounds__(128, A::kMinBlocks)
 walk_group_kernel(Bodies bd, int64_t nbodies, Tree t, typename A::Scalar G, typename A::Scalar eps2, int stack_cap,
-                  unsigned int* queue, unsigned long long* stats, int* err, int64_t own_lo, int64_t own_hi) {
+                  unsigned long long* stats, int* err, int64_t own_lo, int64_t own_hi) {
     if (*err & kErrAbort) return;
+    unsigned int* queue = reinterpret_cast<unsigned int*>(t.work + kTreeWorkQueue);   // zeroed by the build
     using WarpLists = WarpListsT<A::kStageBytes>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -881,8 +882,7 @@ walk_group_kernel(Bodies bd, int64_t nbodies, Tree t, typename A::Scalar G, type
 
 template <class A>
 cudaError_t launch_variant(const Bodies& bd, int64_t nbodies, const Tree& t, const Params& P, int warps, int stack_cap,
-                           unsigned int* queue, unsigned long long* stats, int* err, int sm_count,
-                           cudaStream_t st) {
+                           unsigned long long* stats, int* err, int sm_count, cudaStream_t st) {
     auto kern = walk_group_kernel<A>;
     const size_t smem = (sizeof(WarpListsT<A::kStageBytes>) + sizeof(int) * stack_cap) * warps;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
@@ -891,11 +891,9 @@ cudaError_t launch_variant(const Bodies& bd, int64_t nbodies, const Tree& t, con
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    e = cudaMemsetAsync(queue, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return e;
     using S = typename A::Scalar;
     kern<<<per_sm * sm_count, 32 * warps, smem, st>>>(bd, nbodies, t, static_cast<S>(P.G),
-                                                     static_cast<S>(P.eps * P.eps), stack_cap, queue, stats, err,
+                                                     static_cast<S>(P.eps * P.eps), stack_cap, stats, err,
                                                      P.own_lo, P.own_hi);
     count_launches(1);
     return cudaGetLastError();
@@ -903,12 +901,11 @@ cudaError_t launch_variant(const Bodies& bd, int64_t nbodies, const Tree& t, con
 
 template <template <bool, bool, bool> class Arith>
 cudaError_t launch_arith(const Bodies& bd, int64_t nbodies, const Tree& t, const Params& P, bool potential, int warps,
-                         int stack_cap, unsigned int* queue, unsigned long long* stats, int* err, int sm_count,
-                         cudaStream_t st) {
+                         int stack_cap, unsigned long long* stats, int* err, int sm_count, cudaStream_t st) {
     const bool soft = P.eps > 0.0;
 #define NB_WALK_CASE(Q, S, POT)                                                                                  \
     if (P.quad == Q && soft == S && potential == POT)                                                            \
-        return launch_variant<Arith<Q, S, POT>>(bd, nbodies, t, P, warps, stack_cap, queue, stats, err, sm_count, st);
+        return launch_variant<Arith<Q, S, POT>>(bd, nbodies, t, P, warps, stack_cap, stats, err, sm_count, st);
     NB_WALK_CASE(true, true, false)
     NB_WALK_CASE(true, true, true)
     NB_WALK_CASE(true, false, false)
@@ -930,11 +927,11 @@ size_t walk_group_smem(bool fp64, int warps, int stack_cap) {
 }
 
 cudaError_t launch_walk_group(const Bodies& bd, int64_t nbodies, const Tree& t, const Params& P, bool potential,
-                              bool fp64, int warps, int stack_cap, unsigned int* queue, unsigned long long* stats,
-                              int* err, int sm_count, cudaStream_t st) {
+                              bool fp64, int warps, int stack_cap, unsigned long long* stats, int* err, int sm_count,
+                              cudaStream_t st) {
     if (fp64)
-        return launch_arith<Fp64Arith>(bd, nbodies, t, P, potential, warps, stack_cap, queue, stats, err, sm_count, st);
-    return launch_arith<MixedArith>(bd, nbodies, t, P, potential, warps, stack_cap, queue, stats, err, sm_count, st);
+        return launch_arith<Fp64Arith>(bd, nbodies, t, P, potential, warps, stack_cap, stats, err, sm_count, st);
+    return launch_arith<MixedArith>(bd, nbodies, t, P, potential, warps, stack_cap, stats, err, sm_count, st);
 }
 
 }  // namespace nb

@@ -1,0 +1,54 @@
+"""The one-pass cell and child scans at the edges of their tiles (1,024 positions, 256 cells), for every way a leaf
+size meets the four positions a thread owns: the exported tree equals the oracle's node for node (levels, bodies,
+half-widths and masses of single bodies exactly; masses of cells to the rounding of a sum, 1e-14)."""
+import numpy as np
+import pytest
+
+from next_b200 import ic
+from next_b200.native import Simulation
+
+pytestmark = pytest.mark.gpu
+
+LEVEL, MASS, HALF, LEAF, COUNT = 0, 1, 5, 12, 15
+
+
+@pytest.mark.parametrize("n,leaf_cap", [(1, 1), (2, 1), (5, 3), (255, 4), (257, 5), (1023, 1), (1024, 2), (1025, 3), (1027, 4),
+                                        (2047, 16), (2049, 64), (4097, 5), (33000, 1), (70001, 16)])
+def test_tree_at_tile_edges(oracle, n, leaf_cap):
+    b = ic.plummer(n, seed=n) if n % 2 else ic.uniform_sphere(n, seed=n)
+    sim = Simulation("accurate", "fp64", leaf_cap=leaf_cap)
+    sim.upload(b)
+    t, r = sim.debug_tree(), oracle.tree(b, mode="accurate", leaf_cap=leaf_cap)
+    assert t.shape == r.shape
+    for c in (LEVEL, HALF, LEAF):
+        np.testing.assert_array_equal(t[:, c], r[:, c])
+    leaves = r[:, LEAF] == 1                        # the device exports the body counts of leaves
+    np.testing.assert_array_equal(t[leaves, COUNT], r[leaves, COUNT])
+    np.testing.assert_allclose(t[:, MASS], r[:, MASS], rtol=1e-14, atol=0)
+    assert sim.stats()["device_error"] == 0
+    sim.close()
+
+
+def test_build_of_coincident_bodies_and_many_systems(oracle):
+    """Long chains of cells at one position, and systems that start and end inside a tile: every system's forces
+    equal its own."""
+    sizes = [700, 1, 0, 1500, 3, 900]
+    parts = [ic.plummer(k, seed=i + 20) for i, k in enumerate(sizes) if k]
+    for k in ("x", "y", "z"):
+        parts[0][k][10:60] = parts[0][k][10]
+    b = {c: np.concatenate([p[c] for p in parts]) for c in parts[0]}
+    offsets = np.concatenate([[0], np.cumsum(sizes)])
+    sim = Simulation("accurate", "fp64", leaf_cap=2)
+    sim.upload(b, offsets)
+    a, j = sim.accel(), 0
+    for i, k in enumerate(sizes):
+        if k == 0:
+            continue
+        one = Simulation("accurate", "fp64", leaf_cap=2)
+        one.upload(parts[j])
+        r = one.accel()
+        for c in ("ax", "ay", "az"):
+            np.testing.assert_array_equal(a[c][offsets[i]:offsets[i + 1]], r[c])
+        one.close()
+        j += 1
+    sim.close()
