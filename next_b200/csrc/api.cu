@@ -337,11 +337,12 @@ int build(next_handle* h, std::vector<int>* evs) {
         NB_TRY(launch_root_cubes(src, n, h->sys, h->d_offsets, h->partial, kReduceMax, h->tickets + 0, h->st),
                "root cube");
     h->cube_fresh = false;
-    NB_TRY(launch_keys(src, h->sysid, n, h->sys, h->keys, h->idx, h->st), "keys");
+    NB_TRY(sort_begin(n, h->key_bits, h->sort_scratch, h->st), "sort scratch");
+    NB_TRY(launch_keys(src, h->sysid, n, h->sys, h->keys, h->idx, h->key_bits, h->sort_scratch, h->st), "keys");
     rc0 = record(h, evs);
     if (rc0) return rc0;
     bool in_alt = false;
-    NB_TRY(radix_sort_pairs(h->keys, h->idx, h->keys_alt, h->idx_alt, n, h->key_bits, h->sort_scratch, h->err, &in_alt,
+    NB_TRY(radix_sort_pairs(h->keys, h->idx, h->keys_alt, h->idx_alt, n, h->key_bits, h->sort_scratch, true, h->err, &in_alt,
                             h->st),
            "radix sort");
     h->sorted_in_alt = in_alt;
@@ -1425,7 +1426,7 @@ int next_debug_keys(next_handle* h, uint64_t* keys, double* cube4) {
     if (rc) return rc;
     Bodies b = h->cur_bodies();
     NB_TRY(launch_root_cubes(b, h->n, h->sys, h->d_offsets, h->partial, kReduceMax, h->tickets + 0, h->st), "root cube");
-    NB_TRY(launch_keys(b, h->sysid, h->n, h->sys, h->keys, h->idx, h->st), "keys");
+    NB_TRY(launch_keys(b, h->sysid, h->n, h->sys, h->keys, h->idx, 0, nullptr, h->st), "keys");
     std::vector<uint64_t> kw(h->n);
     std::vector<uint32_t> ids(h->n);
     NB_TRY(cudaMemcpyAsync(kw.data(), h->keys, sizeof(uint64_t) * h->n, cudaMemcpyDeviceToHost, h->st), "keys");
@@ -1512,7 +1513,7 @@ int next_sort_pairs(next_handle* h, int64_t n, const uint64_t* keys_in, const ui
     if (e == cudaSuccess) e = cudaMemsetAsync(h->err, 0, sizeof(int), h->st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(k0, keys_in, sizeof(uint64_t) * n, cudaMemcpyHostToDevice, h->st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(v0, vals_in, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, h->st);
-    if (e == cudaSuccess) e = radix_sort_pairs(k0, v0, k1, v1, n, key_bits, scr, h->err, &in_alt, h->st);
+    if (e == cudaSuccess) e = radix_sort_pairs(k0, v0, k1, v1, n, key_bits, scr, false, h->err, &in_alt, h->st);
     if (e == cudaSuccess && keys_out)
         e = cudaMemcpyAsync(keys_out, in_alt ? k1 : k0, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess && vals_out)

@@ -12,8 +12,9 @@ int64_t launches_so_far();
 // keys.cu
 cudaError_t launch_root_cubes(const Bodies& b, int64_t n, const Systems& sys, const int64_t* d_offsets,
                               double* partial, int partial_blocks, unsigned int* ticket, cudaStream_t st);
+// hist (may be NULL): digit counts of the keys' low key_bits bits, added
 cudaError_t launch_keys(const Bodies& b, const int32_t* sysid, int64_t n, const Systems& sys, uint64_t* keys,
-                        uint32_t* idx, cudaStream_t st);
+                        uint32_t* idx, int key_bits, uint32_t* hist, cudaStream_t st);
 
 // sort.cu
 #ifndef NB_SORT_ITEMS
@@ -24,10 +25,13 @@ constexpr int64_t sort_scratch_words_for(int64_t n) {
     return 2 * 8 * 256 + 8 + 8 * ((n + kSortTile - 1) / kSortTile) * 256;
 }
 size_t sort_scratch_words(int64_t n);
-size_t sort_smem_bytes();
 cudaError_t sort_prepare();
+// Clears a sort's scratch; its first 8 x 256 words then take the digit counts
+// (sort_digits.cuh) of the keys, from the kernel that makes them or sort_count.
+cudaError_t sort_begin(int64_t n, int key_bits, uint32_t* scratch, cudaStream_t st);
+// counted: sort_begin and the counting have been queued already
 cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* alt_keys, uint32_t* alt_vals, int64_t n,
-                             int key_bits, uint32_t* scratch, int* err, bool* in_alt, cudaStream_t st);
+                             int key_bits, uint32_t* scratch, bool counted, int* err, bool* in_alt, cudaStream_t st);
 cudaError_t radix_sort_pairs_to(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
                                 uint32_t* vals_out, uint64_t* alt_keys, uint32_t* alt_vals, int64_t n, int key_bits,
                                 uint32_t* scratch, int* err, cudaStream_t st);

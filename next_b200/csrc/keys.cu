@@ -13,6 +13,7 @@
 #include "box.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "sort_digits.cuh"
 
 namespace nb {
 
@@ -74,39 +75,52 @@ system_cubes_kernel(const double* __restrict__ x, const double* __restrict__ y,
     }
 }
 
-// Bodies per thread (two: more independent descents in flight per thread;
-// 16.7 M-body halo 2.00 -> 1.96 ms build less sort).
-#ifndef NB_KEYS_PER_THREAD
-#define NB_KEYS_PER_THREAD 2
-#endif
-__global__ void __launch_bounds__(256)
+// Two bodies per thread and round (more independent descents in flight per
+// thread; 16.7 M-body halo 2.00 -> 1.96 ms build less sort).  The block also
+// counts the digits of its keys for the sort that follows (hist), which saves
+// that pass over the keys.
+constexpr int kKeysPerThread = 2;
+constexpr int kKeyThreads = 256;
+constexpr int64_t kCountingBlocks = 740;    // 296 to 1,480 measured the same
+__global__ void __launch_bounds__(kKeyThreads)
 keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
             const double* __restrict__ z, const int32_t* __restrict__ sysid, int64_t n,
             const double4* __restrict__ cubes, int base, int levels,
-            uint64_t* __restrict__ keys, uint32_t* __restrict__ idx) {
-    const int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * NB_KEYS_PER_THREAD;
+            uint64_t* __restrict__ keys, uint32_t* __restrict__ idx, int key_bits, uint32_t* __restrict__ hist) {
+    __shared__ uint32_t local[8 * kSortRadix];
+    const int passes = hist ? (key_bits + 7) / 8 : 0;
+    for (int i = threadIdx.x; i < passes * kSortRadix; i += kKeyThreads) local[i] = 0;
+    __syncthreads();
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * kKeyThreads * kKeysPerThread;
+    for (int64_t i0 = (blockIdx.x * (int64_t)kKeyThreads + threadIdx.x) * kKeysPerThread; i0 < n; i0 += stride) {
 #pragma unroll
-    for (int u = 0; u < NB_KEYS_PER_THREAD; ++u) {
-        const int64_t i = i0 + u;
-        if (i >= n) return;
-        const int s = sysid ? sysid[i] : 0;
-        const double4 c = cubes[s];
-        const double px = x[i], py = y[i], pz = z[i];
-        double cx = c.x, cy = c.y, cz = c.z, h = c.w;
-        uint64_t key = base < 64 ? (static_cast<uint64_t>(s) << base) : 0ull;
-        for (int l = 1; l <= levels; ++l) {
-            const bool bx = px > cx, by = py > cy, bz = pz > cz;
-            const uint64_t oct = static_cast<uint64_t>(bx) | (static_cast<uint64_t>(by) << 1) |
-                                 (static_cast<uint64_t>(bz) << 2);
-            key |= oct << (base - 3 * l);
-            const double hs = h * 0.5;
-            cx = cx + (bx ? hs : -hs);
-            cy = cy + (by ? hs : -hs);
-            cz = cz + (bz ? hs : -hs);
-            h = hs;
+        for (int u = 0; u < kKeysPerThread; ++u) {
+            const int64_t i = i0 + u;
+            if (i >= n) break;
+            const int s = sysid ? sysid[i] : 0;
+            const double4 c = cubes[s];
+            const double px = x[i], py = y[i], pz = z[i];
+            double cx = c.x, cy = c.y, cz = c.z, h = c.w;
+            uint64_t key = base < 64 ? (static_cast<uint64_t>(s) << base) : 0ull;
+            for (int l = 1; l <= levels; ++l) {
+                const bool bx = px > cx, by = py > cy, bz = pz > cz;
+                const uint64_t oct = static_cast<uint64_t>(bx) | (static_cast<uint64_t>(by) << 1) |
+                                     (static_cast<uint64_t>(bz) << 2);
+                key |= oct << (base - 3 * l);
+                const double hs = h * 0.5;
+                cx = cx + (bx ? hs : -hs);
+                cy = cy + (by ? hs : -hs);
+                cz = cz + (bz ? hs : -hs);
+                h = hs;
+            }
+            keys[i] = key;
+            idx[i] = static_cast<uint32_t>(i);
+            if (hist) count_digits(key, key_bits, local);
         }
-        keys[i] = key;
-        idx[i] = static_cast<uint32_t>(i);
+    }
+    if (hist) {
+        __syncthreads();
+        add_digit_counts<kKeyThreads>(local, passes, hist);
     }
 }
 
@@ -130,11 +144,13 @@ cudaError_t launch_root_cubes(const Bodies& b, int64_t n, const Systems& sys, co
 }
 
 cudaError_t launch_keys(const Bodies& b, const int32_t* sysid, int64_t n, const Systems& sys,
-                        uint64_t* keys, uint32_t* idx, cudaStream_t st) {
+                        uint64_t* keys, uint32_t* idx, int key_bits, uint32_t* hist, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const int blocks = static_cast<int>((n + 256 * NB_KEYS_PER_THREAD - 1) / (256 * NB_KEYS_PER_THREAD));
-    keys_kernel<<<blocks, 256, 0, st>>>(b.x, b.y, b.z, sys.n > 1 ? sysid : nullptr, n, sys.cube,
-                                        sys.base, sys.levels, keys, idx);
+    // with counts, fewer and longer blocks: each adds its counts to the sort's once
+    const int64_t all = (n + kKeyThreads * kKeysPerThread - 1) / (kKeyThreads * kKeysPerThread);
+    const unsigned blocks = static_cast<unsigned>(hist && all > kCountingBlocks ? kCountingBlocks : all);
+    keys_kernel<<<blocks, kKeyThreads, 0, st>>>(b.x, b.y, b.z, sys.n > 1 ? sysid : nullptr, n, sys.cube, sys.base,
+                                                sys.levels, keys, idx, key_bits, hist);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -1,15 +1,16 @@
-// Stable LSD radix sort of (uint64 key, uint32 value) pairs: one histogram
-// pass over the keys for all digits, then one "onesweep" pass per 8-bit
-// digit.  A onesweep pass works on tiles of 256 x 15 pairs:
+// Stable LSD radix sort of (uint64 key, uint32 value) pairs: one count of all
+// digits over the keys (made with the keys in a tree build), then one "onesweep" pass per 8-bit
+// digit.  A onesweep pass works on tiles of pairs (see Layout):
 //   1. load the tile, count its digits per warp (ballot peer masks, kept in
 //      shared memory for the ranking; one shared add per digit group) and
 //      publish the per-digit tile counts in a status array (flag + count
 //      packed in one 32-bit word);
-//   2. read the statuses of the 8 preceding tiles (decoupled look-back),
-//      and while those loads are in flight scan the counts and rank and
-//      scatter the tile into shared memory in digit order;
-//   3. finish the look-back, publish the inclusive counts, and write the
-//      tile out, each digit run to its global offset,
+//   2. scan the counts and rank and scatter the tile into shared memory in
+//      digit order;
+//   3. add up the counts of the tiles before it -- all at once where there are
+//      at most as many tiles as SMs, else by a decoupled look-back over 8 tiles
+//      at a time that was started before the ranking -- and write the tile
+//      out, each digit run to its global offset,
 // so a pass reads and writes every pair exactly once.  Tiles are numbered
 // in the order blocks start (an atomic ticket), so every tile a block waits
 // on is already running; each wait is still bounded and raises
@@ -18,89 +19,52 @@
 // Memory bound: per pass 12 B read + 12 B written per pair.
 #include "common.cuh"
 #include "kernels.cuh"
+#include "sort_digits.cuh"
 
 namespace nb {
 
 namespace {
 
 constexpr int kRadix = 256;
-constexpr int kThreads = 256;
-constexpr int kWarps = kThreads / 32;
-constexpr int kItems = NB_SORT_ITEMS;
-constexpr int kTile = kThreads * kItems;
+constexpr int kHistThreads = 256;
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagInc = 2u << 30;
 constexpr uint32_t kCountMask = (1u << 30) - 1;
 constexpr int kSpinLimit = 1 << 20;
 constexpr int kLookWindow = 8;   // earlier tiles whose status one look-back step reads
 
-// Digit mask of pass p for keys of key_bits significant bits: bits at and
-// above key_bits take no part in the ordering.
-__host__ __device__ __forceinline__ uint32_t pass_mask(int key_bits, int p) {
-    const int left = key_bits - 8 * p;
-    return left >= 8 ? 0xffu : (1u << left) - 1u;
-}
-
-__global__ void __launch_bounds__(kThreads)
+// Digit counts of all passes.  Four keys per thread and round, their loads in
+// flight together; small sorts get a block per 1,024 keys.
+__global__ void __launch_bounds__(kHistThreads)
 histogram_kernel(const uint64_t* __restrict__ keys, int64_t n, int key_bits, uint32_t* __restrict__ hist) {
     const int passes = (key_bits + 7) / 8;
-    __shared__ uint32_t local[8][kRadix];
-    for (int i = threadIdx.x; i < 8 * kRadix; i += kThreads) (&local[0][0])[i] = 0;
+    __shared__ uint32_t local[8 * kRadix];
+    for (int i = threadIdx.x; i < passes * kRadix; i += kHistThreads) local[i] = 0;
     __syncthreads();
-    for (int64_t i = blockIdx.x * (int64_t)kThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kThreads) {
-        const uint64_t k = keys[i];
-        for (int p = 0; p < passes; ++p) atomicAdd(&local[p][(k >> (8 * p)) & pass_mask(key_bits, p)], 1u);
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * kHistThreads;
+    for (int64_t i = blockIdx.x * (int64_t)kHistThreads + threadIdx.x; i < n; i += 4 * stride) {
+        uint64_t k[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * stride < n) k[u] = keys[i + u * stride];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i + u * stride < n) count_digits(k[u], key_bits, local);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < passes * kRadix; i += kThreads) {
-        const uint32_t v = (&local[0][0])[i];
-        if (v) atomicAdd(hist + i, v);
-    }
+    add_digit_counts<kHistThreads>(local, passes, hist);
 }
 
-// Exclusive scan of each pass's 256 digit counts (one block per pass).
-__global__ void __launch_bounds__(kRadix) digit_offsets_kernel(const uint32_t* hist, uint32_t* offsets) {
-    __shared__ uint32_t s[kRadix];
-    const int p = blockIdx.x, t = threadIdx.x;
-    s[t] = hist[p * kRadix + t];
-    __syncthreads();
-    for (int o = 1; o < kRadix; o <<= 1) {
-        const uint32_t v = t >= o ? s[t - o] : 0u;
-        __syncthreads();
-        s[t] += v;
-        __syncthreads();
-    }
-    offsets[p * kRadix + t] = s[t] - hist[p * kRadix + t];
-}
-
-template <int ITEMS>
+template <int THREADS, int ITEMS>
 struct SortSmemT {
-    uint32_t warp_hist[kWarps][kRadix];
+    uint32_t warp_hist[THREADS / 32][kRadix];
     uint32_t global_delta[kRadix];
-    uint32_t warp_total[kWarps];
-    uint64_t keys[kThreads * ITEMS];
-    uint32_t vals[kThreads * ITEMS];
-    uint32_t peers[ITEMS][kThreads];   // the count pass's peer masks, reused by the ranking
+    uint32_t warp_total[kRadix / 32];
+    uint64_t keys[THREADS * ITEMS];
+    uint32_t vals[THREADS * ITEMS];
+    uint32_t peers[ITEMS][THREADS];   // the count pass's peer masks, reused by the ranking
     int tile;
 };
-using SortSmem = SortSmemT<kItems>;
-
-// Sorts of at most NB_SORT_SMALL_N pairs (the build's, not the allocation-
-// free entry point's) use tiles of kThreads x NB_SORT_SMALL_ITEMS pairs: a
-// few tiles make such a pass, so its time is about one tile's latency, which
-// shorter tiles cut (16,384 pairs: sort 0.048 -> 0.039 ms).  At 1,048,576
-// pairs the longer look-back chain of twice the tiles costs more than that
-// (0.072 -> 0.079 ms), so larger sorts keep kTile.
-#ifndef NB_SORT_SMALL_N
-#define NB_SORT_SMALL_N 262144
-#endif
-#ifndef NB_SORT_SMALL_ITEMS
-#define NB_SORT_SMALL_ITEMS 8
-#endif
-#ifndef NB_SORT_SMALL_MINB
-#define NB_SORT_SMALL_MINB 4
-#endif
-constexpr int kSmallItems = NB_SORT_SMALL_ITEMS;
 
 // Lanes of the warp whose 8-bit digit equals this lane's: eight ballots,
 // one per digit bit (cheaper than a match-any on this part).  Written as one
@@ -123,20 +87,14 @@ __device__ __forceinline__ uint32_t digit_peers(int dig) {
     return peers;
 }
 
-// Three resident blocks per SM (80 registers, 69 KB of shared memory with
-// the stashed peer masks): the phases of one tile wait on memory and on
-// earlier tiles, so occupancy matters as much as instruction count here.
-#ifndef NB_SORT_MINB
-#define NB_SORT_MINB 3
-#endif
 // Tile loads into registers: item k of lane l of warp w is pair
 // tile_base + (w * kItems + k) * 32 + l; pairs past n are padding keys that
 // rank after every real key of the tile and are never written out.
-template <int ITEMS>
+template <int THREADS, int ITEMS>
 __device__ __forceinline__ void load_tile(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                                           int64_t n, int tile, int w, int lane, uint64_t (&key)[ITEMS],
                                           uint32_t (&val)[ITEMS]) {
-    const int64_t warp_base = static_cast<int64_t>(tile) * (kThreads * ITEMS) + static_cast<int64_t>(w) * ITEMS * 32;
+    const int64_t warp_base = static_cast<int64_t>(tile) * (THREADS * ITEMS) + static_cast<int64_t>(w) * ITEMS * 32;
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
         const int64_t g = warp_base + k * 32 + lane;
@@ -145,31 +103,54 @@ __device__ __forceinline__ void load_tile(const uint64_t* __restrict__ keys_in, 
     }
 }
 
+// Four digits' status words of one tile, past L1 (another block may be about to write them).
+__device__ __forceinline__ uint4 load_status(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+
 // Persistent: a block takes tiles by ticket until none is left.  Once a
 // tile's pairs sit ranked in shared memory, the block takes its next ticket
 // and loads that tile into the registers the ranking has freed, so the load
 // runs while this tile waits on its look-back and writes itself out.
-template <int ITEMS, int MINB>
-__global__ void __launch_bounds__(kThreads, MINB)
+template <int THREADS, int ITEMS, int MINB, bool DIRECT>
+__global__ void __launch_bounds__(THREADS, MINB)
 onesweep_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                 uint64_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int64_t n, int shift,
-                uint32_t dmask, const uint32_t* __restrict__ digit_offsets, uint32_t* status, unsigned int* tile_ticket,
+                uint32_t dmask, const uint32_t* __restrict__ hist, uint32_t* status, unsigned int* tile_ticket,
                 int* err) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SortSmemT<ITEMS>& S = *reinterpret_cast<SortSmemT<ITEMS>*>(smem_raw);
+    SortSmemT<THREADS, ITEMS>& S = *reinterpret_cast<SortSmemT<THREADS, ITEMS>*>(smem_raw);
+    constexpr int kWarps = THREADS / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int ntiles = static_cast<int>((n + (kThreads * ITEMS) - 1) / (kThreads * ITEMS));
+    const int d = threadIdx.x;                 // the thread's digit, below kRadix
+    const int ntiles = static_cast<int>((n + (THREADS * ITEMS) - 1) / (THREADS * ITEMS));
     if (threadIdx.x == 0) S.tile = static_cast<int>(atomicAdd(tile_ticket, 1u));
-    __syncthreads();
+    // first output position of each digit: the pass's counts, scanned over the digits
+    uint32_t digit_first = 0;
+    {
+        const uint32_t c = d < kRadix ? hist[d] : 0u;
+        uint32_t inc = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (d < kRadix && lane == 31) S.warp_total[w] = inc;
+        __syncthreads();
+        digit_first = inc - c;
+        for (int ww = 0; ww < w && ww < kRadix / 32; ++ww) digit_first += S.warp_total[ww];
+    }
     int tile = S.tile;
     // Digits are re-extracted from the keys where needed: holding them (or
     // anything derived from them) across the passes costs more registers.
     uint64_t key[ITEMS];
     uint32_t val[ITEMS];
-    if (tile < ntiles) load_tile(keys_in, vals_in, n, tile, w, lane, key, val);
+    if (tile < ntiles) load_tile<THREADS, ITEMS>(keys_in, vals_in, n, tile, w, lane, key, val);
     while (tile < ntiles) {
-        const int64_t tile_base = static_cast<int64_t>(tile) * (kThreads * ITEMS);
-        for (int i = threadIdx.x; i < kWarps * kRadix; i += kThreads) (&S.warp_hist[0][0])[i] = 0;
+        const int64_t tile_base = static_cast<int64_t>(tile) * (THREADS * ITEMS);
+        for (int i = threadIdx.x; i < kWarps * kRadix; i += THREADS) (&S.warp_hist[0][0])[i] = 0;
         __syncthreads();
         // Per-warp digit counts first (fire-and-forget shared adds by each digit's
         // lowest lane), so the tile's counts are published before the ranking.
@@ -185,21 +166,24 @@ onesweep_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict
         // Per digit d: exclusive prefix over warps and the tile count, published
         // at once; the first look-back window is read now and consumed after the
         // local scan and the ranking, which do not need it.
-        const int d = threadIdx.x;
         uint32_t count = 0;
-        for (int ww = 0; ww < kWarps; ++ww) {
-            const uint32_t c = S.warp_hist[ww][d];
-            S.warp_hist[ww][d] = count;
-            count += c;
-        }
         volatile uint32_t* vstat = status;
-        if (tile == 0) vstat[d] = kFlagInc | count;
-        else vstat[static_cast<int64_t>(tile) * kRadix + d] = kFlagAgg | count;
         uint32_t win[kLookWindow];
+        if (d < kRadix) {
+            for (int ww = 0; ww < kWarps; ++ww) {
+                const uint32_t c = S.warp_hist[ww][d];
+                S.warp_hist[ww][d] = count;
+                count += c;
+            }
+            if (!DIRECT && tile == 0) vstat[d] = kFlagInc | count;
+            else vstat[static_cast<int64_t>(tile) * kRadix + d] = kFlagAgg | count;
+            if (!DIRECT) {
 #pragma unroll
-        for (int j = 0; j < kLookWindow; ++j)
-            win[j] = tile - 1 - j >= 0 ? vstat[static_cast<int64_t>(tile - 1 - j) * kRadix + d]
-                                       : static_cast<uint32_t>(kFlagInc);
+                for (int j = 0; j < kLookWindow; ++j)
+                    win[j] = tile - 1 - j >= 0 ? vstat[static_cast<int64_t>(tile - 1 - j) * kRadix + d]
+                                               : static_cast<uint32_t>(kFlagInc);
+            }
+        }
         // Exclusive scan of the tile counts over digits: warp scans + warp totals.
         uint32_t inc = count;
 #pragma unroll
@@ -207,12 +191,14 @@ onesweep_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict
             const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
             if (lane >= o) inc += u;
         }
-        if (lane == 31) S.warp_total[w] = inc;
+        if (d < kRadix && lane == 31) S.warp_total[w] = inc;
         __syncthreads();
         uint32_t tile_start = inc - count;
-        for (int ww = 0; ww < w; ++ww) tile_start += S.warp_total[ww];
-        // warp_hist[w][d] becomes the first local slot of warp w's digit-d keys
-        for (int ww = 0; ww < kWarps; ++ww) S.warp_hist[ww][d] += tile_start;
+        if (d < kRadix) {
+            for (int ww = 0; ww < w; ++ww) tile_start += S.warp_total[ww];
+            // warp_hist[w][d] becomes the first local slot of warp w's digit-d keys
+            for (int ww = 0; ww < kWarps; ++ww) S.warp_hist[ww][d] += tile_start;
+        }
         __syncthreads();
         // Warp-level multisplit in item order (stable: item k of every lane
         // precedes item k+1, lanes in order within an item), scattering each key
@@ -234,12 +220,43 @@ onesweep_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict
         if (threadIdx.x == 0) S.tile = static_cast<int>(atomicAdd(tile_ticket, 1u));
         __syncthreads();
         const int next = S.tile;
-        if (next < ntiles) load_tile(keys_in, vals_in, n, next, w, lane, key, val);
+        if (next < ntiles) load_tile<THREADS, ITEMS>(keys_in, vals_in, n, next, w, lane, key, val);
         // Decoupled look-back for digit d over the earlier tiles, a window of
         // statuses per step: entries are taken in order, an entry without a
         // flag yet is re-read alone (bounded), the first inclusive one ends it.
         uint32_t excl = 0;
-        if (tile > 0) {
+        if (DIRECT) {
+            // the counts of all earlier tiles, summed at once: 64 threads take four digits each of every
+            // (THREADS / 64)-th tile, four tiles' loads in flight, and the block adds up their shares
+            constexpr int kGroups = THREADS / 64;
+            uint4* part = reinterpret_cast<uint4*>(&S.warp_hist[0][0]);      // free once the tile is ranked
+            const int g = threadIdx.x >> 6, c4 = threadIdx.x & 63;
+            const uint4* st4 = reinterpret_cast<const uint4*>(status) + c4;
+            uint4 sum = make_uint4(0, 0, 0, 0);
+            bool timed_out = false;
+            for (int t0 = g; t0 < tile; t0 += 4 * kGroups) {
+                uint4 v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    v[j] = t0 + j * kGroups < tile ? load_status(st4 + (t0 + j * kGroups) * (kRadix / 4))
+                                                   : make_uint4(kFlagAgg, kFlagAgg, kFlagAgg, kFlagAgg);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    int spins = 0;
+                    while ((v[j].x & v[j].y & v[j].z & v[j].w & kFlagAgg) == 0) {
+                        if (++spins > kSpinLimit) { timed_out = true; break; }
+                        v[j] = load_status(st4 + (t0 + j * kGroups) * (kRadix / 4));
+                    }
+                    sum.x += v[j].x & kCountMask; sum.y += v[j].y & kCountMask;
+                    sum.z += v[j].z & kCountMask; sum.w += v[j].w & kCountMask;
+                }
+            }
+            if (timed_out) raise_error(err, kErrSort);
+            part[g * 64 + c4] = sum;
+            __syncthreads();
+            if (d < kRadix)
+                for (int k = 0; k < kGroups; ++k) excl += (&S.warp_hist[0][0])[k * kRadix + d];
+        } else if (d < kRadix && tile > 0) {
             int pred = tile - 1;
             bool done = false, timed_out = false;
             while (!done) {
@@ -266,12 +283,12 @@ onesweep_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict
             vstat[static_cast<int64_t>(tile) * kRadix + d] = kFlagInc | ((excl + count) & kCountMask);
         }
         // global position of local slot i with digit d: global_delta[d] + i
-        S.global_delta[d] = digit_offsets[d] + excl - tile_start;
+        if (d < kRadix) S.global_delta[d] = digit_first + excl - tile_start;
         __syncthreads();
-        const int64_t valid = n - tile_base < (kThreads * ITEMS) ? n - tile_base : (kThreads * ITEMS);
+        const int64_t valid = n - tile_base < (THREADS * ITEMS) ? n - tile_base : (THREADS * ITEMS);
 #pragma unroll
         for (int k = 0; k < ITEMS; ++k) {
-            const int i = k * kThreads + threadIdx.x;
+            const int i = k * THREADS + threadIdx.x;
             if (i < valid) {
                 const uint64_t kk = S.keys[i];
                 const int dd = static_cast<int>((kk >> shift) & dmask);
@@ -286,66 +303,130 @@ onesweep_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict
     }
 }
 
-}  // namespace
+// Tile layouts.  Up to 148 x 512 x 15 = 1,136,640 pairs the smallest layout is
+// taken that gives every SM at most one tile: a pass then lasts one tile, and a
+// tile sums the counts of all earlier ones at once (DIRECT) instead of
+// following a chain of look-backs.  Above that, tiles of 256 x 15, three blocks
+// per SM, whose phases overlap, with the look-back.  Whole sorts of 63-bit keys
+// by the entry point for device buffers, host call included, against 256 x 8
+// up to 262,144 pairs and 256 x 15 above: 16,384 pairs 97 -> 72 us, 262,144 117 ->
+// 106 us, 1,048,576 164 -> 143 us.  A pass is bound there by the ballots and the
+// ranking of an SM's own tile.
+struct Layout {
+    int pairs;                 // per tile
+    void (*launch)(int64_t n, const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int shift,
+                   uint32_t dmask, const uint32_t* hist, uint32_t* status, unsigned int* ticket, int* err,
+                   cudaStream_t st);
+    cudaError_t (*prepare)();
+};
 
-// Pairs per tile of radix_sort_pairs for n pairs.
-static int64_t tile_pairs(int64_t n) {
-    return n <= NB_SORT_SMALL_N ? static_cast<int64_t>(kThreads) * kSmallItems : kTile;
-}
-
-// Scratch words for sorts of up to n pairs with either entry point: hist +
-// offsets (8 x 256 each), tile tickets (8), status (8 x tiles x 256) for the
-// larger of the two tile layouts any such sort can use.
-size_t sort_scratch_words(int64_t n) {
-    const int64_t small_n = n < NB_SORT_SMALL_N ? n : static_cast<int64_t>(NB_SORT_SMALL_N);
-    const int64_t small_tile = static_cast<int64_t>(kThreads) * kSmallItems;
-    const int64_t small_tiles = small_n > 0 ? (small_n + small_tile - 1) / small_tile : 0;
-    const size_t small = static_cast<size_t>(2 * 8 * kRadix + 8 + 8 * small_tiles * kRadix);
-    const size_t big = static_cast<size_t>(sort_scratch_words_for(n));
-    return small > big ? small : big;
-}
-
-size_t sort_smem_bytes() { return sizeof(SortSmem); }
-
-#ifndef NB_SORT_PERSISTENT
-#define NB_SORT_PERSISTENT 1
-#endif
-
-// Blocks of one onesweep pass: every tile's own block, or (persistent) no
-// more than fit on the device at once, each taking tiles until none is left.
-template <int ITEMS, int MINB>
-static unsigned onesweep_grid(int64_t tiles) {
-    if (!NB_SORT_PERSISTENT) return static_cast<unsigned>(tiles);
+// Blocks of one pass: no more than fit on the device at once, each taking
+// tiles until none is left.
+template <int THREADS, int ITEMS, int MINB, bool DIRECT>
+unsigned onesweep_grid(int64_t tiles) {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, onesweep_kernel<ITEMS, MINB>, kThreads,
-                                                      sizeof(SortSmemT<ITEMS>)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, onesweep_kernel<THREADS, ITEMS, MINB, DIRECT>, THREADS,
+                                                      sizeof(SortSmemT<THREADS, ITEMS>)) != cudaSuccess ||
         per_sm < 1 || sms < 1)
         return static_cast<unsigned>(tiles);
     const int64_t resident = static_cast<int64_t>(per_sm) * sms;
     return static_cast<unsigned>(tiles < resident ? tiles : resident);
 }
 
-// One pass with tiles of kThreads x ITEMS pairs.
-template <int ITEMS, int MINB>
-static void launch_pass(int64_t n, const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int shift,
-                        uint32_t dmask, const uint32_t* offs, uint32_t* status, unsigned int* ticket, int* err,
-                        cudaStream_t st) {
-    const int64_t tiles = (n + kThreads * ITEMS - 1) / (kThreads * ITEMS);
-    onesweep_kernel<ITEMS, MINB><<<onesweep_grid<ITEMS, MINB>(tiles), kThreads, sizeof(SortSmemT<ITEMS>), st>>>(
-        ki, vi, ko, vo, n, shift, dmask, offs, status, ticket, err);
+template <int THREADS, int ITEMS, int MINB, bool DIRECT>
+constexpr Layout layout() {
+    return {THREADS * ITEMS,
+            [](int64_t n, const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int shift, uint32_t dmask,
+               const uint32_t* hist, uint32_t* status, unsigned int* ticket, int* err, cudaStream_t st) {
+                const int64_t tiles = (n + THREADS * ITEMS - 1) / (THREADS * ITEMS);
+                onesweep_kernel<THREADS, ITEMS, MINB, DIRECT>
+                    <<<onesweep_grid<THREADS, ITEMS, MINB, DIRECT>(tiles), THREADS, sizeof(SortSmemT<THREADS, ITEMS>), st>>>(
+                        ki, vi, ko, vo, n, shift, dmask, hist, status, ticket, err);
+            },
+            []() {
+                return cudaFuncSetAttribute(onesweep_kernel<THREADS, ITEMS, MINB, DIRECT>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            static_cast<int>(sizeof(SortSmemT<THREADS, ITEMS>)));
+            }};
+}
+
+constexpr Layout kOneTile[] = {layout<256, 4, 1, true>(), layout<256, 8, 1, true>(), layout<512, 8, 1, true>(),
+                               layout<512, 15, 1, true>()};
+constexpr Layout kManyTiles = layout<256, NB_SORT_ITEMS, 3, false>();
+constexpr int64_t kOneTileBlocks = 148;
+
+const Layout& layout_for(int64_t n) {
+    for (const Layout& l : kOneTile)
+        if (n <= kOneTileBlocks * l.pairs) return l;
+    return kManyTiles;
+}
+
+int64_t tiles_for(int64_t n) { return (n + layout_for(n).pairs - 1) / layout_for(n).pairs; }
+
+}  // namespace
+
+static_assert(kSortTile == kManyTiles.pairs, "tile size shared with the scratch-size formula");
+
+// Scratch words for sorts of up to n pairs: digit counts (8 x 256; twice that
+// is reserved), tile tickets (8), status (8 x tiles x 256) for the layout with
+// the most tiles any such sort can use.
+size_t sort_scratch_words(int64_t n) {
+    const int64_t one = (n + kOneTile[0].pairs - 1) / kOneTile[0].pairs;
+    const size_t few = static_cast<size_t>(2 * 8 * kRadix + 8 + 8 * kRadix * (one < kOneTileBlocks ? one : kOneTileBlocks));
+    const size_t many = static_cast<size_t>(sort_scratch_words_for(n));
+    return few > many ? few : many;
 }
 
 cudaError_t sort_prepare() {
-    cudaError_t e = cudaFuncSetAttribute(onesweep_kernel<kItems, NB_SORT_MINB>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(sizeof(SortSmemT<kItems>)));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(onesweep_kernel<kSmallItems, NB_SORT_SMALL_MINB>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(sizeof(SortSmemT<kSmallItems>)));
+    cudaError_t e = kManyTiles.prepare();
+    for (const Layout& l : kOneTile)
+        if (e == cudaSuccess) e = l.prepare();
     return e;
+}
+
+// Clears the scratch of a sort of n pairs; the digit counts (the scratch's
+// first 8 x 256 words) can be added to from then on.
+cudaError_t sort_begin(int64_t n, int key_bits, uint32_t* scratch, cudaStream_t st) {
+    const size_t words = static_cast<size_t>(2 * 8 * kRadix + 8 + ((key_bits + 7) / 8) * tiles_for(n) * kRadix);
+    return cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * words, st);
+}
+
+cudaError_t sort_count(const uint64_t* keys, int64_t n, int key_bits, uint32_t* scratch, cudaStream_t st) {
+    int64_t blocks = (n + kHistThreads * 4 - 1) / (kHistThreads * 4);
+    if (blocks > 592) blocks = 592;
+    histogram_kernel<<<static_cast<unsigned>(blocks), kHistThreads, 0, st>>>(keys, n, key_bits, scratch);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+// The passes of a counted sort, from (keys_in, vals_in), which are left
+// untouched unless they are also the other half of the ping-pong, to
+// (keys_out, vals_out): the passes alternate between the outputs and
+// (alt_keys, alt_vals), starting on whichever side makes the last pass land
+// in the outputs.
+cudaError_t sort_passes(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out, uint32_t* vals_out,
+                        uint64_t* alt_keys, uint32_t* alt_vals, int64_t n, int key_bits, uint32_t* scratch, int* err,
+                        cudaStream_t st) {
+    const int passes = (key_bits + 7) / 8;
+    const Layout& l = layout_for(n);
+    const int64_t tiles = tiles_for(n);
+    unsigned int* tickets = scratch + 16 * kRadix;
+    uint32_t* status = scratch + 16 * kRadix + 8;
+    const uint64_t* src_k = keys_in;
+    const uint32_t* src_v = vals_in;
+    for (int p = 0; p < passes; ++p) {
+        const bool to_out = ((passes - 1 - p) & 1) == 0;
+        uint64_t* dst_k = to_out ? keys_out : alt_keys;
+        uint32_t* dst_v = to_out ? vals_out : alt_vals;
+        l.launch(n, src_k, src_v, dst_k, dst_v, 8 * p, pass_mask(key_bits, p), scratch + p * kRadix,
+                 status + static_cast<int64_t>(p) * tiles * kRadix, tickets + p, err, st);
+        src_k = dst_k;
+        src_v = dst_v;
+    }
+    count_launches(passes);
+    return cudaGetLastError();
 }
 
 // Sorts (keys, vals) of length n using (alt_keys, alt_vals) as the other
@@ -353,52 +434,23 @@ cudaError_t sort_prepare() {
 // of passes is even, else in (alt_keys, alt_vals); *in_alt tells which.
 // scratch holds sort_scratch_words(n) words.
 cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* alt_keys, uint32_t* alt_vals,
-                             int64_t n, int key_bits, uint32_t* scratch, int* err, bool* in_alt,
+                             int64_t n, int key_bits, uint32_t* scratch, bool counted, int* err, bool* in_alt,
                              cudaStream_t st) {
     *in_alt = false;
     if (n <= 1) return cudaSuccess;
-    const int passes = (key_bits + 7) / 8;
-    const int64_t tiles = (n + tile_pairs(n) - 1) / tile_pairs(n);
-    const bool small = tile_pairs(n) != kTile;
-    uint32_t* hist = scratch;
-    uint32_t* offsets = scratch + 8 * kRadix;
-    unsigned int* tickets = scratch + 16 * kRadix;
-    uint32_t* status = scratch + 16 * kRadix + 8;
-    const size_t words = static_cast<size_t>(2 * 8 * kRadix + 8 + 8 * tiles * kRadix);
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * words, st);
-    if (e != cudaSuccess) return e;
-    int hblocks = static_cast<int>((n + kThreads * 16 - 1) / (kThreads * 16));
-    if (hblocks > 1184) hblocks = 1184;
-    histogram_kernel<<<hblocks, kThreads, 0, st>>>(keys, n, key_bits, hist);
-    digit_offsets_kernel<<<passes, kRadix, 0, st>>>(hist, offsets);
-    uint64_t* src_k = keys; uint32_t* src_v = vals;
-    uint64_t* dst_k = alt_keys; uint32_t* dst_v = alt_vals;
-    for (int p = 0; p < passes; ++p) {
-        uint32_t* pst = status + static_cast<int64_t>(p) * tiles * kRadix;
-        if (small)
-            launch_pass<kSmallItems, NB_SORT_SMALL_MINB>(n, src_k, src_v, dst_k, dst_v, 8 * p, pass_mask(key_bits, p),
-                                                         offsets + p * kRadix, pst, tickets + p, err, st);
-        else
-            launch_pass<kItems, NB_SORT_MINB>(n, src_k, src_v, dst_k, dst_v, 8 * p, pass_mask(key_bits, p),
-                                              offsets + p * kRadix, pst, tickets + p, err, st);
-        uint64_t* tk = src_k; src_k = dst_k; dst_k = tk;
-        uint32_t* tv = src_v; src_v = dst_v; dst_v = tv;
+    cudaError_t e = cudaSuccess;
+    if (!counted) {
+        e = sort_begin(n, key_bits, scratch, st);
+        if (e == cudaSuccess) e = sort_count(keys, n, key_bits, scratch, st);
+        if (e != cudaSuccess) return e;
     }
-    *in_alt = (passes & 1) != 0;
-    count_launches(2 + passes);
-    return cudaGetLastError();
+    *in_alt = (((key_bits + 7) / 8) & 1) != 0;
+    return *in_alt ? sort_passes(keys, vals, alt_keys, alt_vals, keys, vals, n, key_bits, scratch, err, st)
+                   : sort_passes(keys, vals, keys, vals, alt_keys, alt_vals, n, key_bits, scratch, err, st);
 }
 
-}  // namespace nb
-
-namespace nb {
-
-static_assert(kSortTile == kTile, "tile size shared with the scratch-size formula");
-
 // Sorts n pairs from (keys_in, vals_in) into (keys_out, vals_out), never
-// writing the inputs: the passes alternate between the outputs and
-// (alt_keys, alt_vals), starting on whichever side makes the last pass land
-// in the outputs.  scratch holds sort_scratch_words(n) words, err one word.
+// writing the inputs.  scratch holds sort_scratch_words(n) words, err one word.
 cudaError_t radix_sort_pairs_to(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out,
                                 uint32_t* vals_out, uint64_t* alt_keys, uint32_t* alt_vals, int64_t n, int key_bits,
                                 uint32_t* scratch, int* err, cudaStream_t st) {
@@ -408,32 +460,10 @@ cudaError_t radix_sort_pairs_to(const uint64_t* keys_in, const uint32_t* vals_in
         if (e == cudaSuccess) e = cudaMemcpyAsync(vals_out, vals_in, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
         return e;
     }
-    const int passes = (key_bits + 7) / 8;
-    const int64_t tiles = (n + kTile - 1) / kTile;
-    uint32_t* hist = scratch;
-    uint32_t* offsets = scratch + 8 * kRadix;
-    unsigned int* tickets = scratch + 16 * kRadix;
-    uint32_t* status = scratch + 16 * kRadix + 8;
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * static_cast<size_t>(sort_scratch_words_for(n)), st);
+    cudaError_t e = sort_begin(n, key_bits, scratch, st);
+    if (e == cudaSuccess) e = sort_count(keys_in, n, key_bits, scratch, st);
     if (e != cudaSuccess) return e;
-    int hblocks = static_cast<int>((n + kThreads * 16 - 1) / (kThreads * 16));
-    if (hblocks > 1184) hblocks = 1184;
-    histogram_kernel<<<hblocks, kThreads, 0, st>>>(keys_in, n, key_bits, hist);
-    digit_offsets_kernel<<<passes, kRadix, 0, st>>>(hist, offsets);
-    const uint64_t* src_k = keys_in;
-    const uint32_t* src_v = vals_in;
-    for (int p = 0; p < passes; ++p) {
-        const bool to_out = ((passes - 1 - p) & 1) == 0;
-        uint64_t* dst_k = to_out ? keys_out : alt_keys;
-        uint32_t* dst_v = to_out ? vals_out : alt_vals;
-        launch_pass<kItems, NB_SORT_MINB>(n, src_k, src_v, dst_k, dst_v, 8 * p, pass_mask(key_bits, p),
-                                          offsets + p * kRadix, status + static_cast<int64_t>(p) * tiles * kRadix,
-                                          tickets + p, err, st);
-        src_k = dst_k;
-        src_v = dst_v;
-    }
-    count_launches(2 + passes);
-    return cudaGetLastError();
+    return sort_passes(keys_in, vals_in, keys_out, vals_out, alt_keys, alt_vals, n, key_bits, scratch, err, st);
 }
 
 }  // namespace nb

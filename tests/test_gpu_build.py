@@ -52,3 +52,20 @@ def test_build_of_coincident_bodies_and_many_systems(oracle):
         one.close()
         j += 1
     sim.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 1023, 1024, 1025, 148 * 1024, 148 * 1024 + 1, 148 * 2048, 148 * 2048 + 1, 148 * 4096,
+                               148 * 4096 + 1, 148 * 7680, 148 * 7680 + 1])
+def test_sort_at_the_layouts_edges(n):
+    """Pairs at the sizes where the tile layout changes, most keys equal in most digits: stable order, bit for bit."""
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, 1 << 62, n, dtype=np.uint64)
+    keys[rng.random(n) < 0.5] &= np.uint64(0xff00ff)
+    vals = np.arange(n, dtype=np.uint32)
+    sim = Simulation("accurate", "mixed")
+    for bits in (17, 63):
+        ko, vo = sim.sort_pairs(keys, vals, bits)
+        order = np.argsort(keys & np.uint64((1 << bits) - 1), kind="stable")
+        np.testing.assert_array_equal(vo, vals[order])
+        np.testing.assert_array_equal(ko, keys[order])
+    sim.close()
