@@ -65,6 +65,27 @@ struct BodyBuf {
 
 constexpr int kReduceMax = 1024;
 
+// The device scalars the host reads, side by side: one copy brings them all.
+struct Status {
+    unsigned long long stats[4];   // pp, pc, max stack, spare
+    int64_t counts[4];             // Tree::counts
+    int err;
+    unsigned int done;             // closing kicks completed by graph replays (next_steps)
+};
+
+// Results of at most this many bytes are gathered straight into page-locked
+// memory of the handle and copied on by the host: one launch instead of one
+// copy engine transfer per lane (1,024 bodies, six lanes: 48 -> 33 us; from
+// 16,384 bodies on the transfers are as fast).
+constexpr int64_t kSmallExportBytes = 400 << 10;
+
+struct HostBlock {
+    Status status;
+    double dts[2];
+    int flags[4];                  // upload check: changed, non-finite, negative mass; next_step_host's check
+    double lanes[kSmallExportBytes / sizeof(double)];
+};
+
 }  // namespace
 
 struct next_handle {
@@ -112,24 +133,19 @@ struct next_handle {
     Tree t{};
 
     // small device scalars
-    int* err = nullptr;
-    unsigned long long* stats = nullptr;   // pp, pc, max stack, spare
+    Status* status = nullptr;
+    int* err = nullptr;                    // in *status, as the next one
+    unsigned long long* stats = nullptr;
     unsigned int* tickets = nullptr;       // 0: cubes, 1: dt, 2: diagnostics
     double* partial = nullptr;             // kReduceMax * 8
     double* dts = nullptr;                 // dt, dt/2
-    double* dt_out = nullptr;              // adaptive dt, half
     double* diag = nullptr;                // 8
     int* changed = nullptr;
     float* fma_out = nullptr;
-    unsigned int* done = nullptr;          // closing kicks completed by graph replays (next_steps)
+    unsigned int* done = nullptr;          // in *status
 
     // pinned host scalars
-    double* h_dts = nullptr;
-    int* h_err = nullptr;
-    int* h_flags = nullptr;                // upload check: changed, non-finite, negative mass
-    int64_t* h_counts = nullptr;           // internal, nodes, groups
-    unsigned long long* h_stats = nullptr;
-    unsigned int* h_done = nullptr;
+    HostBlock* host = nullptr;
 
     // direct summation scratch
     int64_t* d_targets = nullptr;
@@ -437,16 +453,14 @@ bool adaptive_depth(const next_handle* h) {
 }
 
 int read_device_error(next_handle* h, int* bits) {
-    NB_TRY(cudaMemcpyAsync(h->h_err, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->st), "error word");
-    NB_TRY(cudaMemcpyAsync(h->h_counts, h->t.counts, sizeof(int64_t) * 4, cudaMemcpyDeviceToHost, h->st), "counts");
-    NB_TRY(cudaMemcpyAsync(h->h_stats, h->stats, sizeof(unsigned long long) * 4, cudaMemcpyDeviceToHost, h->st), "stats");
+    NB_TRY(cudaMemcpyAsync(&h->host->status, h->status, sizeof(Status), cudaMemcpyDeviceToHost, h->st), "status");
     NB_TRY(cudaStreamSynchronize(h->st), "sync");
-    *bits = *h->h_err;
+    *bits = h->host->status.err;
     // the first build after an upload measured the tree depth: later builds
     // keep three levels of margin below it.  A tree that outgrows them gets
     // leaves of more than leaf_cap bodies at the last level (still exact,
     // slower): seen here, the keys get three more levels.
-    const int64_t deepest = h->h_counts[3];
+    const int64_t deepest = h->host->status.counts[3];
     if (h->depth_seen == h->builds) return NEXT_OK;   // no build since the last look
     h->depth_seen = h->builds;
     if (*bits == 0 && deepest > 0 && adaptive_depth(h)) {
@@ -468,7 +482,7 @@ int recover(next_handle* h, int bits) {
         return fail(h, NEXT_ERR_DEVICE, "device error word " + std::to_string(bits) +
                                             " (sort look-back timeout or failed index check)");
     if (bits & kErrTree) {
-        const int64_t need = std::max<int64_t>(h->h_counts[0] + h->h_counts[0] / 2 + 1024, 2 * h->t.cap_int);
+        const int64_t need = std::max<int64_t>(h->host->status.counts[0] + h->host->status.counts[0] / 2 + 1024, 2 * h->t.cap_int);
         int rc = alloc_tree(h, need);
         if (rc) return rc;
     }
@@ -496,8 +510,9 @@ int forces_checked(next_handle* h, bool potential) {
     return fail(h, NEXT_ERR_DEVICE, "force phase kept overflowing");
 }
 
+// dt for the kernels that follow; the count of completed replays starts at zero
 int set_dt(next_handle* h, double dt) {
-    NB_TRY(launch_set_dt(h->dts, dt, h->st), "dt upload");
+    NB_TRY(launch_set_dt(h->dts, dt, h->done, h->st), "dt upload");
     return NEXT_OK;
 }
 
@@ -654,13 +669,13 @@ int add_graph_timing(next_handle* h, int parity, const std::vector<int>& evs) {
 
 // Grow capacities that the last build came close to (before a graph capture).
 int grow_if_tight(next_handle* h) {
-    const int64_t internal = h->h_counts[0], nodes = h->h_counts[1];
+    const int64_t internal = h->host->status.counts[0], nodes = h->host->status.counts[1];
     if (!h->fixed_tree_cap && (4 * internal > 3 * h->t.cap_int || 4 * nodes > 3 * h->t.cap_node)) {
         int rc = alloc_tree(h, std::max<int64_t>(2 * internal + 1024, h->t.cap_int));
         if (rc) return rc;
         h->forces_valid = false;
     }
-    if (group_walk(h) && 4 * static_cast<int64_t>(h->h_stats[2]) > 3 * h->prm.walk_stack &&
+    if (group_walk(h) && 4 * static_cast<int64_t>(h->host->status.stats[2]) > 3 * h->prm.walk_stack &&
         h->prm.walk_stack < (1 << 14)) {
         h->prm.walk_stack *= 2;
         drop_graphs(h);
@@ -744,22 +759,18 @@ int next_create(const next_params* p, next_handle** out) {
     e = sort_prepare();
     if (e != cudaSuccess) return bail(e, "sort setup");
     auto A = [&](auto** q, size_t c) { if (e == cudaSuccess) e = dalloc(q, c); };
-    A(&h->err, 1); A(&h->stats, 4); A(&h->tickets, 4); A(&h->partial, kReduceMax * 8);
-    A(&h->dts, 2); A(&h->dt_out, 2); A(&h->diag, 8); A(&h->changed, 4); A(&h->fma_out, 1);
-    A(&h->t.counts, 4); A(&h->t.dark_mass, 1); A(&h->done, 1);
+    A(&h->status, 1); A(&h->tickets, 4); A(&h->partial, kReduceMax * 8);
+    A(&h->dts, 2); A(&h->diag, 8); A(&h->changed, 4); A(&h->fma_out, 1);
+    A(&h->t.dark_mass, 1);
     if (e != cudaSuccess) return bail(e, "scalars");
-    e = cudaMemset(h->err, 0, sizeof(int));
+    h->err = &h->status->err;
+    h->stats = h->status->stats;
+    h->done = &h->status->done;
+    h->t.counts = h->status->counts;
+    e = cudaMemset(h->status, 0, sizeof(Status));
     if (e == cudaSuccess) e = cudaMemset(h->tickets, 0, sizeof(unsigned int) * 4);
-    if (e == cudaSuccess) e = cudaMemset(h->stats, 0, sizeof(unsigned long long) * 4);
-    if (e == cudaSuccess) e = cudaMemset(h->t.counts, 0, sizeof(int64_t) * 4);
     if (e == cudaSuccess) e = cudaMemset(h->t.dark_mass, 0xff, sizeof(double));   // NaN
-    if (e == cudaSuccess) e = cudaMemset(h->done, 0, sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_dts), sizeof(double) * 2, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_err), sizeof(int) * 2, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_flags), sizeof(int) * 4, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_counts), sizeof(int64_t) * 4, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_stats), sizeof(unsigned long long) * 4, cudaHostAllocDefault);
-    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->h_done), sizeof(unsigned int), cudaHostAllocDefault);
+    if (e == cudaSuccess) e = cudaHostAlloc(reinterpret_cast<void**>(&h->host), sizeof(HostBlock), cudaHostAllocDefault);
     if (e != cudaSuccess) return bail(e, "pinned scalars");
     *out = h;
     return NEXT_OK;
@@ -779,18 +790,12 @@ void next_destroy(next_handle* h) {
     nccl_comm_destroy(h->comm);
     h->comm = nullptr;
     free_bodies(h);
-    dfree(h->err); dfree(h->stats); dfree(h->tickets); dfree(h->partial);
-    dfree(h->dts); dfree(h->dt_out); dfree(h->diag); dfree(h->changed); dfree(h->fma_out); dfree(h->t.counts); dfree(h->t.dark_mass);
-    dfree(h->done);
+    dfree(h->status); dfree(h->tickets); dfree(h->partial);
+    dfree(h->dts); dfree(h->diag); dfree(h->changed); dfree(h->fma_out); dfree(h->t.dark_mass);
     dfree(h->d_targets); dfree(h->d_targetpos); dfree(h->d_direct_partial); dfree(h->d_direct_out);
     if (h->flush) cudaFree(h->flush);
     for (auto ev : h->ev_pool) cudaEventDestroy(ev);
-    if (h->h_dts) cudaFreeHost(h->h_dts);
-    if (h->h_err) cudaFreeHost(h->h_err);
-    if (h->h_flags) cudaFreeHost(h->h_flags);
-    if (h->h_counts) cudaFreeHost(h->h_counts);
-    if (h->h_stats) cudaFreeHost(h->h_stats);
-    if (h->h_done) cudaFreeHost(h->h_done);
+    if (h->host) cudaFreeHost(h->host);
     if (h->ev_out) cudaEventDestroy(h->ev_out);
     if (h->st_out) cudaStreamDestroy(h->st_out);
     if (h->st) cudaStreamDestroy(h->st);
@@ -859,11 +864,11 @@ static int upload_staged(next_handle* h, int64_t n_systems, const int64_t* offse
     Bodies b = h->cur_bodies();
     NB_TRY(cudaMemsetAsync(h->changed, 0, sizeof(int) * 3, h->st), "upload flags");
     NB_TRY(launch_check_upload(stage, stype, b, h->inv, n, same_layout, h->changed, h->st), "upload check");
-    NB_TRY(cudaMemcpyAsync(h->h_flags, h->changed, sizeof(int) * 3, cudaMemcpyDeviceToHost, h->st), "upload flags");
+    NB_TRY(cudaMemcpyAsync(h->host->flags, h->changed, sizeof(int) * 3, cudaMemcpyDeviceToHost, h->st), "upload flags");
     NB_TRY(cudaStreamSynchronize(h->st), "sync");
-    if (h->h_flags[1]) return fail(h, NEXT_ERR_INVALID_ARGUMENT, "non-finite body data");
-    if (h->h_flags[2]) return fail(h, NEXT_ERR_INVALID_ARGUMENT, "negative mass");
-    if (same_layout && h->h_flags[0] == 0) {
+    if (h->host->flags[1]) return fail(h, NEXT_ERR_INVALID_ARGUMENT, "non-finite body data");
+    if (h->host->flags[2]) return fail(h, NEXT_ERR_INVALID_ARGUMENT, "negative mass");
+    if (same_layout && h->host->flags[0] == 0) {
         NB_TRY(launch_load_velocities(stage, b, h->inv, n, h->st), "velocities");
         return NEXT_OK;   // same positions: tree order and cached forces stay valid
     }
@@ -889,6 +894,23 @@ int next_upload(next_handle* h, int64_t n, const double* x, const double* y, con
     return next_upload_systems(h, 1, offs, x, y, z, vx, vy, vz, m, type);
 }
 
+// `cnt` lanes of the working state to the caller's arrays, in the caller's
+// order (a NULL array is skipped); returns when they have arrived.
+static int download_lanes(next_handle* h, const double* const* lanes, double* const* outs, int cnt) {
+    const int64_t n = h->n;
+    const bool small = static_cast<int64_t>(sizeof(double)) * n * cnt <= kSmallExportBytes;
+    double* staged = small ? h->host->lanes : h->stage;
+    NB_TRY(launch_gather_out(lanes, cnt, h->inv, n, staged, h->st), "gather out");
+    for (int c = 0; c < cnt && !small; ++c)
+        if (outs[c])
+            NB_TRY(cudaMemcpyAsync(outs[c], staged + c * n, sizeof(double) * n, cudaMemcpyDeviceToHost, h->st),
+                   "download");
+    NB_TRY(cudaStreamSynchronize(h->st), "sync");
+    for (int c = 0; c < cnt && small; ++c)
+        if (outs[c]) std::memcpy(outs[c], staged + c * n, sizeof(double) * n);
+    return NEXT_OK;
+}
+
 int next_download(next_handle* h, double* x, double* y, double* z, double* vx, double* vy, double* vz) {
     int rc = check_ready(h);
     if (rc) return rc;
@@ -901,12 +923,7 @@ int next_download(next_handle* h, double* x, double* y, double* z, double* vx, d
     for (int c = 0; c < 6; ++c)
         if (dst[c]) { lanes[cnt] = src[c]; outs[cnt] = dst[c]; ++cnt; }
     if (cnt == 0) return NEXT_OK;
-    NB_TRY(launch_gather_out(lanes, cnt, h->inv, h->n, h->stage, h->st), "gather out");
-    for (int c = 0; c < cnt; ++c)
-        NB_TRY(cudaMemcpyAsync(outs[c], h->stage + c * h->n, sizeof(double) * h->n, cudaMemcpyDeviceToHost, h->st),
-               "download");
-    NB_TRY(cudaStreamSynchronize(h->st), "sync");
-    return NEXT_OK;
+    return download_lanes(h, lanes, outs, cnt);
 }
 
 int next_step(next_handle* h, double dt) {
@@ -1108,7 +1125,7 @@ int next_step_host(next_handle* h, double dt, int64_t n, double* x, double* y, d
     NB_TRY(cudaMemsetAsync(h->io_flag, 0, sizeof(int), h->st_in), "io flag");
     NB_TRY(launch_same_as_last(in, h->io_type[k], h->io_out[p], h->io_in[p], h->io_type[p], n, h->io_flag, h->st_in),
            "upload check");
-    NB_TRY(cudaMemcpyAsync(h->h_flags + 3, h->io_flag, sizeof(int), cudaMemcpyDeviceToHost, h->st_in), "io flag");
+    NB_TRY(cudaMemcpyAsync(h->host->flags + 3, h->io_flag, sizeof(int), cudaMemcpyDeviceToHost, h->st_in), "io flag");
     NB_TRY(cudaStreamWaitEvent(h->st_out, h->ev_out, 0), "export wait");
     NB_TRY(cudaStreamWaitEvent(h->st_out, h->ev_in_pos, 0), "upload wait");
     for (int c = 0; c < 3; ++c)
@@ -1122,7 +1139,7 @@ int next_step_host(next_handle* h, double dt, int64_t n, double* x, double* y, d
     if (ei != cudaSuccess) return cuda_fail(h, ei, "upload");
     if (eo != cudaSuccess) return cuda_fail(h, eo, "position copies");
     if (es != cudaSuccess) return cuda_fail(h, es, "sync");
-    if (h->h_flags[3] == 0) {
+    if (h->host->flags[3] == 0) {
         h->io_cur = k;
         h->io_ready = true;
         return NEXT_OK;
@@ -1140,9 +1157,9 @@ int next_step_host(next_handle* h, double dt, int64_t n, double* x, double* y, d
     Bodies b = h->cur_bodies();
     NB_TRY(cudaMemsetAsync(h->changed, 0, sizeof(int) * 3, h->st), "upload flags");
     NB_TRY(launch_check_upload(in, h->io_type[k], b, h->inv, n, false, h->changed, h->st), "upload check");
-    NB_TRY(cudaMemcpyAsync(h->h_flags, h->changed, sizeof(int) * 3, cudaMemcpyDeviceToHost, h->st), "upload flags");
+    NB_TRY(cudaMemcpyAsync(h->host->flags, h->changed, sizeof(int) * 3, cudaMemcpyDeviceToHost, h->st), "upload flags");
     NB_TRY(cudaStreamSynchronize(h->st), "sync");
-    const bool invalid = h->h_flags[1] || h->h_flags[2];
+    const bool invalid = h->host->flags[1] || h->host->flags[2];
     if (invalid) {
         // back to the state the previous call returned
         for (int c = 0; c < 6; ++c)
@@ -1166,7 +1183,7 @@ int next_step_host(next_handle* h, double dt, int64_t n, double* x, double* y, d
                                    sizeof(double) * n, cudaMemcpyDeviceToHost, h->st), "restore");
         NB_TRY(cudaStreamSynchronize(h->st), "sync");
         h->io_ready = true;       // the held state is again what the previous call returned
-        return fail(h, NEXT_ERR_INVALID_ARGUMENT, h->h_flags[1] ? "non-finite body data" : "negative mass");
+        return fail(h, NEXT_ERR_INVALID_ARGUMENT, h->host->flags[1] ? "non-finite body data" : "negative mass");
     }
     rc = step_and_export(h, x, y, z, vx, vy, vz, out, true, &pending);
     const cudaError_t es2 = cudaStreamSynchronize(h->st_out);
@@ -1192,7 +1209,6 @@ int next_steps(next_handle* h, double dt, int nsteps) {
     int done = 0;            // steps completed
     int base = 0;            // `done` when the device's count of completed replays was last zeroed
     int since_check = 0;     // replays launched since the error word was last read
-    if (use_graph) NB_TRY(cudaMemsetAsync(h->done, 0, sizeof(unsigned int), h->st), "replay count");
     // Reads the error word of the replays launched since the last look.  A
     // replay that overflowed a capacity stopped after its kick-drift (every
     // later kernel of it, and of the replays after it, skipped its work but
@@ -1202,13 +1218,11 @@ int next_steps(next_handle* h, double dt, int nsteps) {
     auto check = [&]() -> int {
         if (since_check == 0) return NEXT_OK;
         since_check = 0;
-        NB_TRY(cudaMemcpyAsync(h->h_done, h->done, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->st),
-               "replay count");
         int bits = 0;
         int r = read_device_error(h, &bits);
         if (r) return r;
         if (bits == 0) return grow_if_tight(h);
-        const int completed = static_cast<int>(*h->h_done);
+        const int completed = static_cast<int>(h->host->status.done);
         r = recover(h, bits);
         if (r) return r;
         r = forces_checked(h, false);
@@ -1294,12 +1308,8 @@ int next_accel(next_handle* h, double* ax, double* ay, double* az, double* pot) 
     const double* lanes[4] = {h->ax, h->ay, h->az, h->pot};
     double* outs[4] = {ax, ay, az, pot};
     const int cnt = want_pot ? 4 : 3;
-    NB_TRY(launch_gather_out(lanes, cnt, h->inv, h->n, h->stage, h->st), "gather out");
-    for (int c = 0; c < cnt; ++c)
-        if (outs[c])
-            NB_TRY(cudaMemcpyAsync(outs[c], h->stage + c * h->n, sizeof(double) * h->n, cudaMemcpyDeviceToHost, h->st),
-                   "download");
-    NB_TRY(cudaStreamSynchronize(h->st), "sync");
+    rc = download_lanes(h, lanes, outs, cnt);
+    if (rc) return rc;
     if (pot && !want_pot) std::memset(pot, 0, sizeof(double) * h->n);
     return NEXT_OK;
 }
@@ -1308,10 +1318,9 @@ int next_adaptive_dt(next_handle* h, double base_dt, double* dt_out) {
     int rc = check_ready(h);
     if (rc) return rc;
     if (!dt_out) return fail(h, NEXT_ERR_INVALID_ARGUMENT, "NULL output");
-    NB_TRY(launch_adaptive_dt(h->cur_bodies(), h->n, base_dt, h->partial, h->tickets + 1, h->dt_out, h->st), "adaptive dt");
-    NB_TRY(cudaMemcpyAsync(h->h_dts, h->dt_out, sizeof(double), cudaMemcpyDeviceToHost, h->st), "dt");
+    NB_TRY(launch_adaptive_dt(h->cur_bodies(), h->n, base_dt, h->partial, h->tickets + 1, h->host->dts, h->st), "adaptive dt");
     NB_TRY(cudaStreamSynchronize(h->st), "sync");
-    *dt_out = h->h_dts[0];
+    *dt_out = h->host->dts[0];
     return NEXT_OK;
 }
 
@@ -1378,14 +1387,14 @@ int next_stats_get(next_handle* h, next_stats* s) {
         rc = resolve_timers(h);
         if (rc) return rc;
         s->device_error = bits;
-        s->n_internal = h->h_counts[0];
-        s->n_nodes = h->h_counts[1];
-        s->n_groups = h->h_counts[2];
+        s->n_internal = h->host->status.counts[0];
+        s->n_nodes = h->host->status.counts[1];
+        s->n_groups = h->host->status.counts[2];
         s->key_levels = h->sys.levels;
         s->recoveries = static_cast<int32_t>(h->recoveries);
-        s->pp_interactions = static_cast<int64_t>(h->h_stats[0]);
-        s->pc_interactions = static_cast<int64_t>(h->h_stats[1]);
-        s->max_stack = static_cast<int64_t>(h->h_stats[2]);
+        s->pp_interactions = static_cast<int64_t>(h->host->status.stats[0]);
+        s->pc_interactions = static_cast<int64_t>(h->host->status.stats[1]);
+        s->max_stack = static_cast<int64_t>(h->host->status.stats[2]);
     }
     s->steps = static_cast<int32_t>(h->timed_steps);
     s->ms_step = h->acc_step;
@@ -1458,7 +1467,7 @@ int next_debug_tree(next_handle* h, double* rows, int64_t cap, int64_t* n_rows) 
     if (rc) return rc;
     rc = forces_checked(h, false);
     if (rc) return rc;
-    const int64_t nn = h->h_counts[1];
+    const int64_t nn = h->host->status.counts[1];
     std::vector<int2> link(nn);
     std::vector<int8_t> level(nn);
     std::vector<double4> com(nn);
@@ -1518,9 +1527,9 @@ int next_sort_pairs(next_handle* h, int64_t n, const uint64_t* keys_in, const ui
         e = cudaMemcpyAsync(keys_out, in_alt ? k1 : k0, sizeof(uint64_t) * n, cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess && vals_out)
         e = cudaMemcpyAsync(vals_out, in_alt ? v1 : v0, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, h->st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h->h_err, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h->host->status.err, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-    const int bits = e == cudaSuccess ? *h->h_err : 0;
+    const int bits = e == cudaSuccess ? h->host->status.err : 0;
     dfree(k0); dfree(k1); dfree(v0); dfree(v1); dfree(scr);
     if (e != cudaSuccess) return cuda_fail(h, e, "sort");
     if (bits & kErrSort) return fail(h, NEXT_ERR_DEVICE, "sort look-back timeout");
@@ -1626,7 +1635,7 @@ int next_autotune(next_handle* h, next_tune_result* out) {
         if (ms < best_ms) {
             best_ms = ms;
             best = c;
-            best_stack = static_cast<int64_t>(h->h_stats[2]);
+            best_stack = static_cast<int64_t>(h->host->status.stats[2]);
         }
     }
     cudaEventDestroy(a);

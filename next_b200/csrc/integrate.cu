@@ -329,7 +329,8 @@ __global__ void ids_to_positions_kernel(const int64_t* __restrict__ ids, const u
     if (t < k) pos[t] = inv[ids[t]];
 }
 
-__global__ void set_dt_kernel(double* dts, double dt) {
+__global__ void set_dt_kernel(double* dts, double dt, unsigned int* done) {
+    *done = 0u;
     dts[0] = dt;
     dts[1] = dt * 0.5;
 }
@@ -463,8 +464,8 @@ cudaError_t launch_ids_to_positions(const int64_t* ids, const uint32_t* inv, int
     return cudaGetLastError();
 }
 
-cudaError_t launch_set_dt(double* dts, double dt, cudaStream_t st) {
-    set_dt_kernel<<<1, 1, 0, st>>>(dts, dt);
+cudaError_t launch_set_dt(double* dts, double dt, unsigned int* done, cudaStream_t st) {
+    set_dt_kernel<<<1, 1, 0, st>>>(dts, dt, done);
     count_launches(1);
     return cudaGetLastError();
 }

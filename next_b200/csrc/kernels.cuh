@@ -88,7 +88,7 @@ cudaError_t launch_gather_out(const double* const* lanes, int count, const uint3
                               cudaStream_t st);
 cudaError_t launch_ids_to_positions(const int64_t* ids, const uint32_t* inv, int64_t k, int64_t* pos,
                                     cudaStream_t st);
-cudaError_t launch_set_dt(double* dts, double dt, cudaStream_t st);
+cudaError_t launch_set_dt(double* dts, double dt, unsigned int* done, cudaStream_t st);   // *done = 0
 cudaError_t launch_fma_peak(float* out, int blocks, int iters, cudaStream_t st);
 
 }  // namespace nb
