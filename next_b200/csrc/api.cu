@@ -390,7 +390,7 @@ int walk(next_handle* h, bool potential) {
                                  h->prm.walk_warps, h->prm.walk_stack, h->stats, h->err, h->sm_count, h->st),
                "group walk");
     } else {
-        NB_TRY(launch_walk_plain(bd, h->sysid, h->d_offsets, h->nsys, h->n, h->t, h->P, potential, h->stats, h->err,
+        NB_TRY(launch_walk_plain(bd, h->sysid, h->d_offsets, h->sys, h->n, h->t, h->P, potential, h->stats, h->err,
                                  h->st),
                "plain walk");
     }

@@ -42,8 +42,8 @@ cudaError_t build_tree(const uint64_t* keys, int64_t n, const Bodies& bd, const 
 int64_t tree_work_words(int64_t n, int64_t cap_int);   // words of Tree::work for n bodies and cap_int internal cells
 
 // walk_plain.cu
-cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int64_t* offsets, int nsys, int64_t n,
-                              const Tree& t, const Params& P, bool potential, unsigned long long* stats, int* err,
+cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int64_t* d_offsets, const Systems& sys,
+                              int64_t n, const Tree& t, const Params& P, bool potential, unsigned long long* stats, int* err,
                               cudaStream_t st);
 int direct_slices(int64_t n, int64_t k);
 // in: k sizes, k masses, k distances; out: k softening lengths (reference law)

@@ -200,13 +200,16 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
 // data wavefronts at 87-93% of their peak, 17 of 32 lanes active); here a record
 // is read once for W bodies, mostly with its siblings beside it, and small
 // systems have 1 / W of a warp per body instead of 1 / 32.  1,048,576 bodies
-// (theta 0.5, one body per leaf): 21.7 -> 9.25 ms per walk, 16,384 bodies 1.95 ->
-// 0.23 ms.  Bound now by the issue of the FP64 chains and the selects around
-// them (62% of issue slots, FP64 pipe 41%).  W = 4: the bodies of a warp open
-// different cells, so a larger W spends more lanes on nodes one body wants (W =
-// 6: 9.5 ms, 8: 10.1 ms) and a smaller one reads and tests more nodes per body
-// (3: 9.9 ms, 2: 12.5 ms, 1: 19 ms); 120 registers, 4 blocks per SM (5 spill: 15 ms).
-constexpr int kPlainW = 4;
+// (theta 0.5, one body per leaf): 21.7 -> 8.3 ms per walk, 16,384 bodies 1.95 ->
+// 0.21 ms.  Bound by the issue of the FP64 chains and what surrounds them (62%
+// of issue slots).  The targets' coordinates lie in shared memory and a node
+// that gives no force is switched off by its inverse distance alone: with the
+// coordinates in registers and a select per component the loop had room for
+// four bodies (9.25 ms).  W = 7: the bodies of a warp open different cells, so a
+// larger W spends more lanes on nodes few of them want (8: 8.4 ms, 9: 9.0 ms)
+// and a smaller one reads and tests more nodes per body (6: 8.4 ms, 4: 9.1 ms);
+// 128 registers, 4 blocks per SM (5: 9.3 ms and more).
+constexpr int kPlainW = 7;
 constexpr int kPlainWarps = 4;
 // Popping k nodes adds at most 7 k entries, and one node at a time never more
 // than 7 per level: rounds are cut short so that 7 * kMaxLevel + 8 entries stay
@@ -218,11 +221,16 @@ constexpr int kPlainList = 32 + 32 * kPlainChunk;
 struct PlainShared {
     int2 stack[kPlainStack];                             // node, mask of the bodies that opened its parent
     int2 list[kPlainList];                               // body, mask of the bodies that opened its leaf
+    double pos[kPlainW][4];
 };
+
+// a target's coordinate, read where it is used: held in registers the targets would cost the loop its overlap
+__device__ __forceinline__ double at(const double& v) { return *reinterpret_cast<const volatile double*>(&v); }
 
 template <bool POT>
 __global__ void __launch_bounds__(32 * kPlainWarps, 4)
-walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, int64_t n, Tree t, Params P,
+walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, const double4* __restrict__ cubes,
+                     int64_t n, Tree t, Params P,
                      unsigned long long* stats, int* err) {
     if (*err & kErrAbort) return;
     __shared__ PlainShared shared[kPlainWarps];
@@ -256,13 +264,18 @@ walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, i
     }
     if (own) {                                           // warp-uniform
         const unsigned nodes = static_cast<unsigned>(t.counts[1]), nbodies = static_cast<unsigned>(n);
-        const double eps2 = P.eps * P.eps, G = P.G;
-        double x[kPlainW], y[kPlainW], z[kPlainW], ax[kPlainW], ay[kPlainW], az[kPlainW], pot[kPlainW];
+        // Lengths of a system far from 1 are scaled by a power of two, which rounds nothing, so that fifth
+        // powers of distances stay in range.
+        const int ex = static_cast<int>((__double_as_longlong(cubes[sys].w) >> 52) & 0x7ff) - 1023;
+        const bool scaled = ex > 150 || ex < -150;
+        const double S1 = scaled ? scalbn(1.0, -ex) : 1.0;
+        const double eps2 = (P.eps * S1) * (P.eps * S1);
+        double ax[kPlainW], ay[kPlainW], az[kPlainW], pot[kPlainW];
         int sp = 1, pn = 0;
 #pragma unroll
         for (int b = 0; b < kPlainW; ++b) {
             const int64_t i = first + b < last ? first + b : first;
-            x[b] = bd.x[i]; y[b] = bd.y[i]; z[b] = bd.z[i];
+            if (lane == b) { S.pos[b][0] = bd.x[i] * S1; S.pos[b][1] = bd.y[i] * S1; S.pos[b][2] = bd.z[i] * S1; }
             ax[b] = ay[b] = az[b] = pot[b] = 0.0;
         }
         if (lane == 0) S.stack[0] = make_int2(sys, static_cast<int>(bodies));
@@ -295,32 +308,36 @@ walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, i
                 if (!ok) raise_error(err, kErrIndex);
                 if (!ok || c.w == 0.0) mask = 0;
             }
+            if (scaled) {                                 // warp-uniform
+                c.x *= S1; c.y *= S1; c.z *= S1;
+                qd.y *= S1;
+                qa.x = qa.x * S1 * S1; qa.y = qa.y * S1 * S1; qb.x = qb.x * S1 * S1;
+                qb.y = qb.y * S1 * S1; qc.x = qc.x * S1 * S1; qc.y = qc.y * S1 * S1;
+            }
             const double rc2 = qd.y * qd.y;
             unsigned opened = 0;
             // no branch in this loop: the bodies' chains of dependent FP64 operations interleave
 #pragma unroll
             for (int b = 0; b < kPlainW; ++b) {
                 const bool mine = mask >> b & 1u;
-                const double dx = c.x - x[b], dy = c.y - y[b], dz = c.z - z[b];
+                const double dx = c.x - at(S.pos[b][0]), dy = c.y - at(S.pos[b][1]), dz = c.z - at(S.pos[b][2]);
                 const double r2 = dx * dx + dy * dy + dz * dz;
                 const bool open = mine && r2 < rc2, use = mine && !open;
                 opened |= static_cast<unsigned>(open) << b;
                 const double r2s = away_from_ends(r2 + eps2);
-                const double rinv = rsqrt_fast(r2s);
+                const double rinv = use ? rsqrt_fast(r2s) : 0.0;    // zero: no force from this node
                 const double rinv2 = rinv * rinv;
-                // a = G rinv5 ((m r2 + 2.5 d.Q.d rinv2) d - Q d); Q = 0 in monopole walks
+                // a = rinv5 ((m r2 + 2.5 d.Q.d rinv2) d - Q d), times G at the end; Q = 0 in monopole walks
                 const double qx = fma(qc.x, dz, fma(qb.y, dy, qa.x * dx));
                 const double qy = fma(qc.y, dz, fma(qa.y, dy, qb.y * dx));
                 const double qz = fma(qb.x, dz, fma(qc.y, dy, qc.x * dx));
                 const double q = fma(dz, qz, fma(dy, qy, dx * qx));
-                const double g5 = G * rinv * (rinv2 * rinv2);
+                const double rinv5 = rinv * (rinv2 * rinv2);
                 const double k = fma(2.5 * q, rinv2, c.w * r2s);
-                const double fx = fma(g5, fma(k, dx, -qx), ax[b]), fy = fma(g5, fma(k, dy, -qy), ay[b]),
-                             fz = fma(g5, fma(k, dz, -qz), az[b]);
-                ax[b] = use ? fx : ax[b];
-                ay[b] = use ? fy : ay[b];
-                az[b] = use ? fz : az[b];
-                if (POT) pot[b] = use ? pot[b] - fma(0.5 * q, g5, G * c.w * rinv) : pot[b];
+                ax[b] = fma(rinv5, fma(k, dx, -qx), ax[b]);
+                ay[b] = fma(rinv5, fma(k, dy, -qy), ay[b]);
+                az[b] = fma(rinv5, fma(k, dz, -qz), az[b]);
+                if (POT) pot[b] -= fma(0.5 * q, rinv5, c.w * rinv);
             }
             npc += __popc(mask & ~opened & own);
             // children of opened cells -> stack
@@ -366,14 +383,15 @@ walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, i
                     const int j = pe.x;
                     const unsigned jm = static_cast<unsigned>(pe.y);
                     pn = k;
-                    double xj = 0.0, yj = 0.0, zj = 0.0, gm = 0.0;
-                    if (jm) { xj = bd.x[j]; yj = bd.y[j]; zj = bd.z[j]; gm = G * bd.m[j]; }
+                    double xj = 0.0, yj = 0.0, zj = 0.0, mj = 0.0;
+                    if (jm) { xj = bd.x[j]; yj = bd.y[j]; zj = bd.z[j]; mj = bd.m[j]; }
+                    if (scaled) { xj *= S1; yj *= S1; zj *= S1; }
 #pragma unroll
                     for (int b = 0; b < kPlainW; ++b) {
                         if (!(jm >> b & 1u) || j == first + b) continue;
-                        const double dx = xj - x[b], dy = yj - y[b], dz = zj - z[b];
+                        const double dx = xj - at(S.pos[b][0]), dy = yj - at(S.pos[b][1]), dz = zj - at(S.pos[b][2]);
                         const double rinv = rsqrt(dx * dx + dy * dy + dz * dz + eps2);
-                        const double mr = gm * rinv, mr3 = mr * rinv * rinv;
+                        const double mr = mj * rinv, mr3 = mr * rinv * rinv;
                         ax[b] = fma(mr3, dx, ax[b]);
                         ay[b] = fma(mr3, dy, ay[b]);
                         az[b] = fma(mr3, dz, az[b]);
@@ -395,8 +413,9 @@ walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, i
             }
             const int64_t i = first + b;
             if (lane == 0 && (own >> b & 1u)) {
-                bd.ax[i] = ax[b]; bd.ay[i] = ay[b]; bd.az[i] = az[b];
-                if (POT) bd.pot[i] = pot[b];
+                const double g = P.G * S1;
+                bd.ax[i] = g * ax[b] * S1; bd.ay[i] = g * ay[b] * S1; bd.az[i] = g * az[b] * S1;
+                if (POT) bd.pot[i] = g * pot[b];
             }
         }
     }
@@ -466,16 +485,16 @@ cudaError_t launch_softening_eval(const double* in, int64_t k, double* out, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int64_t* offsets, int nsys, int64_t n,
-                              const Tree& t, const Params& P, bool potential, unsigned long long* stats, int* err,
+cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int64_t* d_offsets, const Systems& sys,
+                              int64_t n, const Tree& t, const Params& P, bool potential, unsigned long long* stats, int* err,
                               cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const int32_t* sid = nsys > 1 ? sysid : nullptr;
+    const int32_t* sid = sys.n > 1 ? sysid : nullptr;
     if (P.physics == NEXT_PHYSICS_ACCURATE) {
-        const int64_t warps = (n + kPlainW - 1) / kPlainW + (nsys > 1 ? nsys : 0);
+        const int64_t warps = (n + kPlainW - 1) / kPlainW + (sys.n > 1 ? sys.n : 0);
         const unsigned blocks = static_cast<unsigned>((warps + kPlainWarps - 1) / kPlainWarps);
         auto kern = potential ? walk_accurate_kernel<true> : walk_accurate_kernel<false>;
-        kern<<<blocks, 32 * kPlainWarps, 0, st>>>(bd, nsys > 1 ? offsets : nullptr, nsys, n, t, P, stats, err);
+        kern<<<blocks, 32 * kPlainWarps, 0, st>>>(bd, sys.n > 1 ? d_offsets : nullptr, sys.n, sys.cube, n, t, P, stats, err);
     } else {
         const unsigned blocks = static_cast<unsigned>((n + kRefThreads - 1) / kRefThreads);
         walk_reference_kernel<<<blocks, kRefThreads, 0, st>>>(bd, sid, n, t, P, stats, err);

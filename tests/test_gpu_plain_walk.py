@@ -1,6 +1,6 @@
 """The plain FP64 walks at the edges of their warps, lists and stacks.
 
-The accurate walk takes four bodies of one system per warp and sums a body's
+The accurate walk takes seven bodies of one system per warp and sums a body's
 terms in another order than the oracle: at most a few thousand terms, each
 rounded a few times, so forces and potentials agree to 1e-12 of the largest one
 (2^-53 times the term count leaves a factor of two); the opening decisions are
@@ -156,3 +156,21 @@ def test_reference_walk_after_other_dark_masses(oracle):
         a = sim.accel()
         close(a, oracle.accel(b, mode="ref"), ("ax", "ay", "az"))
     sim.close()
+
+
+@pytest.mark.parametrize("length", [2.0 ** -400, 2.0 ** 400])
+def test_accurate_walk_far_from_unit_lengths(length):
+    """Lengths scaled by a power of two round nothing: forces and potentials scale exactly, where the distances'
+    own fifth powers would leave the range."""
+    b = ic.plummer(999, seed=4)
+    c = dict(b, **{k: b[k] * length for k in ("x", "y", "z")})
+    out = []
+    for bodies, eps in ((b, 0.01), (c, 0.01 * length)):
+        sim = Simulation("accurate", "fp64", theta=0.5, eps=eps)
+        sim.upload(bodies)
+        out.append(sim.accel(potential=True))
+        assert sim.stats()["device_error"] == 0
+        sim.close()
+    for k in ("ax", "ay", "az"):
+        np.testing.assert_array_equal(out[1][k] * length * length, out[0][k])
+    np.testing.assert_array_equal(out[1]["pot"] * length, out[0]["pot"])
