@@ -110,6 +110,7 @@ struct next_handle {
     int32_t* sysid = nullptr;
     int64_t* d_offsets = nullptr;
     double4* cubes = nullptr;
+    unsigned long long* boxes = nullptr;   // 6 per system, several systems only
     uint32_t* sort_scratch = nullptr;
     size_t sort_words = 0;
     double* stage = nullptr;          // 7 x n staging lanes (upload) / up to 10 x n (download)
@@ -294,7 +295,7 @@ void free_bodies(next_handle* h) {
     for (auto& b : h->buf) b.free_all();
     dfree(h->ax); dfree(h->ay); dfree(h->az); dfree(h->pot);
     dfree(h->keys); dfree(h->keys_alt); dfree(h->idx); dfree(h->idx_alt); dfree(h->inv);
-    dfree(h->sysid); dfree(h->d_offsets); dfree(h->cubes); dfree(h->sort_scratch);
+    dfree(h->sysid); dfree(h->d_offsets); dfree(h->cubes); dfree(h->boxes); dfree(h->sort_scratch);
     dfree(h->stage); dfree(h->stype);
     free_tree(h);
     h->cap_n = 0;
@@ -311,6 +312,7 @@ int alloc_bodies(next_handle* h, int64_t n) {
     A(&h->ax, padded); A(&h->ay, padded); A(&h->az, padded); A(&h->pot, padded);
     A(&h->keys, n); A(&h->keys_alt, n); A(&h->idx, n); A(&h->idx_alt, n); A(&h->inv, n);
     A(&h->sysid, n); A(&h->d_offsets, h->nsys + 1); A(&h->cubes, h->nsys);
+    if (h->nsys > 1) A(&h->boxes, 6 * static_cast<size_t>(h->nsys));
     h->sort_words = sort_scratch_words(n);
     A(&h->sort_scratch, h->sort_words);
     A(&h->stage, 10 * n); A(&h->stype, n);
@@ -350,7 +352,7 @@ int build(next_handle* h, std::vector<int>* evs) {
     if (rc0) return rc0;
     ++h->builds;
     if (!h->cube_fresh)
-        NB_TRY(launch_root_cubes(src, n, h->sys, h->d_offsets, h->partial, kReduceMax, h->tickets + 0, h->st),
+        NB_TRY(launch_root_cubes(src, h->sysid, n, h->sys, h->partial, kReduceMax, h->tickets + 0, h->st),
                "root cube");
     h->cube_fresh = false;
     NB_TRY(sort_begin(n, h->key_bits, h->sort_scratch, h->st), "sort scratch");
@@ -516,12 +518,12 @@ int set_dt(next_handle* h, double dt) {
     return NEXT_OK;
 }
 
-// The opening half-kick and the drift; with one system the same pass boxes
-// the new positions, and the next build takes that root cube.
+// The opening half-kick and the drift; the same pass boxes the new positions,
+// and the next build takes those root cubes.
 cudaError_t kick_drift_step(next_handle* h, const Bodies& bd) {
-    if (h->sys.n != 1) return launch_kick_drift(bd, h->n, h->dts, h->err, h->st);
-    const cudaError_t e = launch_kick_drift_box(bd, h->n, h->dts, h->err, h->partial, kReduceMax, h->tickets + 0,
-                                                h->sys.cube, h->st);
+    const cudaError_t e = h->sys.n != 1 ? launch_system_boxes(bd, h->sysid, h->n, h->sys, h->dts, h->err, h->tickets + 0, h->st)
+                                        : launch_kick_drift_box(bd, h->n, h->dts, h->err, h->partial, kReduceMax,
+                                                                h->tickets + 0, h->sys.cube, h->st);
     h->cube_fresh = e == cudaSuccess;
     return e;
 }
@@ -838,6 +840,8 @@ static int upload_staged(next_handle* h, int64_t n_systems, const int64_t* offse
         h->depth_decided = false;
         S.offsets = h->d_offsets;
         S.cube = h->cubes;
+        S.boxes = h->boxes;
+        if (h->nsys > 1) NB_TRY(launch_reset_boxes(S, h->st), "boxes");
         set_share(h);
         NB_TRY(cudaMemcpyAsync(h->d_offsets, offsets, sizeof(int64_t) * (n_systems + 1), cudaMemcpyHostToDevice, h->st),
                "offsets");
@@ -1434,7 +1438,7 @@ int next_debug_keys(next_handle* h, uint64_t* keys, double* cube4) {
     int rc = check_ready(h);
     if (rc) return rc;
     Bodies b = h->cur_bodies();
-    NB_TRY(launch_root_cubes(b, h->n, h->sys, h->d_offsets, h->partial, kReduceMax, h->tickets + 0, h->st), "root cube");
+    NB_TRY(launch_root_cubes(b, h->sysid, h->n, h->sys, h->partial, kReduceMax, h->tickets + 0, h->st), "root cube");
     NB_TRY(launch_keys(b, h->sysid, h->n, h->sys, h->keys, h->idx, 0, nullptr, h->st), "keys");
     std::vector<uint64_t> kw(h->n);
     std::vector<uint32_t> ids(h->n);

@@ -45,4 +45,13 @@ __device__ __forceinline__ double4 cube_from_box(const double lo[3], const doubl
     return c;
 }
 
+// Doubles as unsigned integers of the same order, for atomic minima and maxima.
+__device__ __forceinline__ unsigned long long box_encode(double v) {
+    const long long b = __double_as_longlong(v);
+    return static_cast<unsigned long long>(b) ^ (b < 0 ? ~0ull : 0x8000000000000000ull);
+}
+__device__ __forceinline__ double box_decode(unsigned long long u) {
+    return __longlong_as_double(static_cast<long long>(u ^ (u >> 63 ? 0x8000000000000000ull : ~0ull)));
+}
+
 }  // namespace nb

@@ -34,6 +34,7 @@ struct Systems {
     int levels;          // octant levels per key (base / 3)
     const int64_t* offsets;   // n + 1
     double4* cube;       // cx, cy, cz, half
+    unsigned long long* boxes;   // 6 per system (several systems): bounds being collected, see box.cuh
 };
 
 // Tree in sibling-contiguous layout.  Nodes 0..nsys-1 are the system roots;

@@ -49,21 +49,129 @@ __global__ void inv_scatter_kernel(const uint32_t* __restrict__ id, int64_t n, u
     if (k < n) inv[k] = static_cast<uint32_t>(p);
 }
 
-__global__ void kick_drift_kernel(Bodies b, int64_t n, const double* __restrict__ dts, const int* err) {
-    if (*err & kErrAbort) return;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double dt = dts[0], half = dts[1];
-    // all loads before the first store (the lanes may alias as far as the
-    // compiler knows)
-    const double vx0 = b.vx[i], vy0 = b.vy[i], vz0 = b.vz[i], ax = b.ax[i], ay = b.ay[i], az = b.az[i];
-    const double x0 = b.x[i], y0 = b.y[i], z0 = b.z[i];
-    const double vx = vx0 + ax * half, vy = vy0 + ay * half, vz = vz0 + az * half;
-    b.vx[i] = vx; b.vy[i] = vy; b.vz[i] = vz;
-    b.x[i] = x0 + vx * dt; b.y[i] = y0 + vy * dt; b.z[i] = z0 + vz * dt;
+// The opening half-kick and the drift (KICK) of bodies of many systems, and
+// the bounds of every system's (drifted) positions.  A warp takes SPAN * 32
+// consecutive bodies: they mostly belong to one system, whose bounds it keeps
+// in registers and adds to the system's with six atomics when the system ends.
+// The last block to finish turns the bounds into cubes (up to kBoxLast
+// systems; a launch of its own above).
+//
+// Memory bound: the kick-drift's 120 B per body (without it 28 B).  A block per
+// system took as long as its largest system: 256 systems of 1,024-65,536
+// bodies, 160 us for the boxes beside 66 us for the kick-drift -> NB_BOX us for
+// both.
+constexpr int kBoxLast = 4096;
+constexpr int64_t kBoxShort = 262144;  // up to here a warp takes 64 bodies, above 256 (fewer atomics)
+struct Bounds {
+    double lo[3], hi[3];
+    __device__ __forceinline__ void clear() {
+        for (int a = 0; a < 3; ++a) { lo[a] = 1e30; hi[a] = -1e30; }
+    }
+    __device__ __forceinline__ void add(double x, double y, double z) {
+        lo[0] = fmin(lo[0], x); hi[0] = fmax(hi[0], x);
+        lo[1] = fmin(lo[1], y); hi[1] = fmax(hi[1], y);
+        lo[2] = fmin(lo[2], z); hi[2] = fmax(hi[2], z);
+    }
+    __device__ __forceinline__ void merge(unsigned long long* box) const {
+        for (int a = 0; a < 3; ++a) {
+            atomicMin(box + a, box_encode(lo[a]));
+            atomicMax(box + 3 + a, box_encode(hi[a]));
+        }
+    }
+};
+
+// A system's root cube from its bounds, which are cleared for the next time.
+__device__ __forceinline__ void take_cube(unsigned long long* box, double4* cube) {
+    double lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = box_decode(__ldcg(box + a));
+        hi[a] = box_decode(__ldcg(box + 3 + a));
+        box[a] = box_encode(1e30);
+        box[3 + a] = box_encode(-1e30);
+    }
+    *cube = cube_from_box(lo, hi);
 }
 
-// The same kick-drift over a grid-stride loop that also boxes the drifted
+__global__ void box_cubes_kernel(unsigned long long* boxes, int nsys, double4* cube) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s < nsys) take_cube(boxes + 6 * static_cast<int64_t>(s), cube + s);
+}
+
+template <bool KICK, int SPAN>
+__global__ void __launch_bounds__(kBoxThreads)
+system_boxes_kernel(Bodies b, const int32_t* __restrict__ sysid, int64_t n, const double* __restrict__ dts,
+                    const int* err, unsigned long long* __restrict__ boxes, int nsys, unsigned int* ticket,
+                    double4* __restrict__ cube) {
+    if (KICK && (*err & kErrAbort)) return;
+    const double dt = KICK ? dts[0] : 0.0, half = KICK ? dts[1] : 0.0;
+    const int lane = threadIdx.x & 31;
+    const int64_t first = ((blockIdx.x * (int64_t)kBoxThreads + threadIdx.x) >> 5) * (32 * SPAN);
+    int cur = -1;                      // the system whose bounds are collected (warp-uniform)
+    Bounds bounds;
+    bounds.clear();
+    const auto flush = [&]() {
+        if (cur >= 0) {
+            for (int a = 0; a < 3; ++a) warp_minmax(bounds.lo[a], bounds.hi[a]);
+            if (lane == 0) bounds.merge(boxes + 6 * static_cast<int64_t>(cur));
+        }
+        bounds.clear();
+    };
+    for (int k0 = 0; k0 < SPAN; k0 += 2) {
+        // two rounds' loads before the first store (the lanes may alias as far as the compiler knows)
+        double x[2], y[2], z[2], vx[2], vy[2], vz[2], ax[2], ay[2], az[2];
+        int s[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = first + 32 * (k0 + u) + lane;
+            s[u] = -1;
+            if (i < n) {
+                s[u] = sysid[i];
+                x[u] = b.x[i]; y[u] = b.y[i]; z[u] = b.z[i];
+                if (KICK) {
+                    vx[u] = b.vx[i]; vy[u] = b.vy[i]; vz[u] = b.vz[i];
+                    ax[u] = b.ax[i]; ay[u] = b.ay[i]; az[u] = b.az[i];
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t i = first + 32 * (k0 + u) + lane;
+            if (KICK && i < n) {
+                const double wx = vx[u] + ax[u] * half, wy = vy[u] + ay[u] * half, wz = vz[u] + az[u] * half;
+                b.vx[i] = wx; b.vy[i] = wy; b.vz[i] = wz;
+                x[u] = x[u] + wx * dt; y[u] = y[u] + wy * dt; z[u] = z[u] + wz * dt;
+                b.x[i] = x[u]; b.y[i] = y[u]; b.z[i] = z[u];
+            }
+            const int s0 = __shfl_sync(0xffffffffu, s[u], 0);
+            if (__all_sync(0xffffffffu, s[u] == s0 || s[u] < 0)) {
+                if (s0 != cur) { flush(); cur = s0; }
+                if (s[u] >= 0) bounds.add(x[u], y[u], z[u]);
+            } else {                   // systems meet inside the 32 bodies: each lane adds its own
+                flush();
+                cur = -1;
+                if (s[u] >= 0) {
+                    Bounds mine;
+                    mine.clear();
+                    mine.add(x[u], y[u], z[u]);
+                    mine.merge(boxes + 6 * static_cast<int64_t>(s[u]));
+                }
+            }
+        }
+    }
+    flush();
+    if (nsys > kBoxLast) return;
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int s = threadIdx.x; s < nsys; s += kBoxThreads) take_cube(boxes + 6 * static_cast<int64_t>(s), cube + s);
+    if (threadIdx.x == 0) *ticket = 0u;
+}
+
+// One system's kick-drift over a grid-stride loop that also boxes the drifted
 // positions: the last block to finish folds the block boxes into the root
 // cube the next build needs (one system), saving the build a pass over x, y, z.
 #ifndef NB_KDB_BATCH
@@ -376,11 +484,22 @@ cudaError_t launch_gather_bodies(const Bodies& src, const Bodies& dst, const uin
     return cudaGetLastError();
 }
 
-cudaError_t launch_kick_drift(const Bodies& b, int64_t n, const double* dts, const int* err, cudaStream_t st) {
-    if (n <= 0) return cudaSuccess;
-    kick_drift_kernel<<<grid_for(n, 256), 256, 0, st>>>(b, n, dts, err);
+cudaError_t launch_reset_boxes(const Systems& sys, cudaStream_t st) {
+    box_cubes_kernel<<<grid_for(sys.n, 128), 128, 0, st>>>(sys.boxes, sys.n, sys.cube);
     count_launches(1);
     return cudaGetLastError();
+}
+
+cudaError_t launch_system_boxes(const Bodies& b, const int32_t* sysid, int64_t n, const Systems& sys, const double* dts,
+                                const int* err, unsigned int* ticket, cudaStream_t st) {
+    if (n <= 0) return cudaSuccess;
+    const bool shorter = n <= kBoxShort;
+    auto kern = dts ? (shorter ? system_boxes_kernel<true, 2> : system_boxes_kernel<true, 8>)
+                    : (shorter ? system_boxes_kernel<false, 2> : system_boxes_kernel<false, 8>);
+    kern<<<grid_for(n, kBoxThreads * (shorter ? 2 : 8)), kBoxThreads, 0, st>>>(b, sysid, n, dts, err, sys.boxes, sys.n,
+                                                                              ticket, sys.cube);
+    count_launches(1);
+    return sys.n > kBoxLast ? launch_reset_boxes(sys, st) : cudaGetLastError();
 }
 
 cudaError_t launch_kick_drift_box(const Bodies& b, int64_t n, const double* dts, const int* err, double* partial,

@@ -10,8 +10,8 @@ void count_launches(int k);
 int64_t launches_so_far();
 
 // keys.cu
-cudaError_t launch_root_cubes(const Bodies& b, int64_t n, const Systems& sys, const int64_t* d_offsets,
-                              double* partial, int partial_blocks, unsigned int* ticket, cudaStream_t st);
+cudaError_t launch_root_cubes(const Bodies& b, const int32_t* sysid, int64_t n, const Systems& sys, double* partial,
+                              int partial_blocks, unsigned int* ticket, cudaStream_t st);
 // hist (may be NULL): digit counts of the keys' low key_bits bits, added
 cudaError_t launch_keys(const Bodies& b, const int32_t* sysid, int64_t n, const Systems& sys, uint64_t* keys,
                         uint32_t* idx, int key_bits, uint32_t* hist, cudaStream_t st);
@@ -60,7 +60,10 @@ cudaError_t launch_walk_group(const Bodies& bd, int64_t nbodies, const Tree& t, 
 // integrate.cu
 cudaError_t launch_gather_bodies(const Bodies& src, const Bodies& dst, const uint32_t* idx, int64_t n, uint32_t* inv,
                                  int* err, cudaStream_t st);
-cudaError_t launch_kick_drift(const Bodies& b, int64_t n, const double* dts, const int* err, cudaStream_t st);
+// root cubes of many systems; with dts, the kick-drift first, in the same pass
+cudaError_t launch_system_boxes(const Bodies& b, const int32_t* sysid, int64_t n, const Systems& sys, const double* dts,
+                                const int* err, unsigned int* ticket, cudaStream_t st);
+cudaError_t launch_reset_boxes(const Systems& sys, cudaStream_t st);
 // kick-drift that also writes the root cube of the drifted bodies (one system)
 cudaError_t launch_kick_drift_box(const Bodies& b, int64_t n, const double* dts, const int* err, double* partial,
                                   int partial_blocks, unsigned int* ticket, double4* cube, cudaStream_t st);

@@ -56,25 +56,6 @@ root_cube_kernel(const double* __restrict__ x, const double* __restrict__ y,
     }
 }
 
-// Many systems: one block per system.
-__global__ void __launch_bounds__(kBoxThreads)
-system_cubes_kernel(const double* __restrict__ x, const double* __restrict__ y,
-                    const double* __restrict__ z, const int64_t* __restrict__ offsets,
-                    int nsys, double4* cube) {
-    for (int s = blockIdx.x; s < nsys; s += gridDim.x) {
-        double lo[3] = {1e30, 1e30, 1e30}, hi[3] = {-1e30, -1e30, -1e30};
-        for (int64_t i = offsets[s] + threadIdx.x; i < offsets[s + 1]; i += blockDim.x) {
-            const double px = x[i], py = y[i], pz = z[i];
-            lo[0] = fmin(lo[0], px); hi[0] = fmax(hi[0], px);
-            lo[1] = fmin(lo[1], py); hi[1] = fmax(hi[1], py);
-            lo[2] = fmin(lo[2], pz); hi[2] = fmax(hi[2], pz);
-        }
-        block_minmax3(lo, hi);
-        if (threadIdx.x == 0) cube[s] = cube_from_box(lo, hi);
-        __syncthreads();
-    }
-}
-
 // Two bodies per thread and round (more independent descents in flight per
 // thread; 16.7 M-body halo 2.00 -> 1.96 ms build less sort).  The block also
 // counts the digits of its keys for the sort that follows (hist), which saves
@@ -126,20 +107,14 @@ keys_kernel(const double* __restrict__ x, const double* __restrict__ y,
 
 }  // namespace
 
-cudaError_t launch_root_cubes(const Bodies& b, int64_t n, const Systems& sys, const int64_t* d_offsets,
-                              double* partial, int partial_blocks, unsigned int* ticket,
-                              cudaStream_t st) {
-    if (sys.n == 1) {
-        int blocks = static_cast<int>((n + kBoxThreads - 1) / kBoxThreads);
-        if (blocks > partial_blocks) blocks = partial_blocks;
-        if (blocks < 1) blocks = 1;
-        root_cube_kernel<<<blocks, kBoxThreads, 0, st>>>(b.x, b.y, b.z, n, partial, ticket, sys.cube);
-        count_launches(1);
-    } else {
-        int blocks = sys.n < 4096 ? sys.n : 4096;
-        system_cubes_kernel<<<blocks, kBoxThreads, 0, st>>>(b.x, b.y, b.z, d_offsets, sys.n, sys.cube);
-        count_launches(1);
-    }
+cudaError_t launch_root_cubes(const Bodies& b, const int32_t* sysid, int64_t n, const Systems& sys, double* partial,
+                              int partial_blocks, unsigned int* ticket, cudaStream_t st) {
+    if (sys.n != 1) return launch_system_boxes(b, sysid, n, sys, nullptr, nullptr, ticket, st);
+    int blocks = static_cast<int>((n + kBoxThreads - 1) / kBoxThreads);
+    if (blocks > partial_blocks) blocks = partial_blocks;
+    if (blocks < 1) blocks = 1;
+    root_cube_kernel<<<blocks, kBoxThreads, 0, st>>>(b.x, b.y, b.z, n, partial, ticket, sys.cube);
+    count_launches(1);
     return cudaGetLastError();
 }
 

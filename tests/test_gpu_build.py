@@ -69,3 +69,27 @@ def test_sort_at_the_layouts_edges(n):
         np.testing.assert_array_equal(vo, vals[order])
         np.testing.assert_array_equal(ko, keys[order])
     sim.close()
+
+
+@pytest.mark.parametrize("systems,top", [(3, 400), (40, 60), (5000, 6)])
+def test_steps_of_many_systems(systems, top):
+    """Root cubes boxed by the kick-drift (several systems in a warp's bodies, more systems than the last block
+    takes): two steps of the batch equal two steps of a system alone."""
+    rng = np.random.default_rng(systems)
+    sizes = rng.integers(1, top, systems)
+    b = ic.plummer(int(sizes.sum()), seed=systems)
+    offsets = np.concatenate([[0], np.cumsum(sizes)])
+    sim = Simulation("accurate", "fp64", eps=0.05)
+    sim.upload(b, offsets)
+    sim.steps(1e-3, 2)
+    s = sim.download()
+    for i in (0, 1, systems // 2, systems - 1):
+        at = slice(offsets[i], offsets[i + 1])
+        one = Simulation("accurate", "fp64", eps=0.05)
+        one.upload({k: v[at] for k, v in b.items()})
+        one.steps(1e-3, 2)
+        o = one.download()
+        for k in s:
+            np.testing.assert_array_equal(s[k][at], o[k])
+        one.close()
+    sim.close()
