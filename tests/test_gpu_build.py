@@ -93,3 +93,31 @@ def test_steps_of_many_systems(systems, top):
             np.testing.assert_array_equal(s[k][at], o[k])
         one.close()
     sim.close()
+
+
+@pytest.mark.parametrize("kind", ["random", "lattice", "offset", "narrow", "plane", "huge"])
+def test_keys_by_cell_number_equal_the_descent(oracle, kind):
+    """Keys from cell numbers, with the level-by-level descent where a body is too near a cell boundary: on
+    boundaries (lattice), far from the origin, with extents near the coordinates' rounding, in a plane, at 1e200."""
+    rng = np.random.default_rng(11)
+    n = 20011
+    p = rng.uniform(-1.0, 1.0, (3, n))
+    if kind == "lattice":
+        p = np.round(p * 64.0) / 64.0
+    elif kind == "offset":
+        p = p * 1e-3 + np.array([[1e6], [-3e5], [7.0]])
+    elif kind == "narrow":
+        p = 1.0 + p * 1e-14
+    elif kind == "plane":
+        p[2] = 0.25
+    elif kind == "huge":
+        p = p * 1e200
+    b = {"x": p[0].copy(), "y": p[1].copy(), "z": p[2].copy(), "m": np.full(n, 1.0 / n)}
+    for k in ("vx", "vy", "vz"):
+        b[k] = np.zeros(n)
+    sim = Simulation("reference", "fp64")
+    sim.upload(b)
+    keys, cube = sim.debug_keys()
+    np.testing.assert_array_equal(cube, oracle.root_cube(b))
+    np.testing.assert_array_equal(keys, oracle.keys(b))
+    sim.close()
