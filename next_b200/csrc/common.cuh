@@ -45,7 +45,9 @@ struct Systems {
 // last key level (a leaf over capacity: the keys need more levels)
 constexpr unsigned kDepthOverfull = 64;
 
-constexpr int kTreeWorkQueue = 4;      // word of Tree::work the group walk counts its groups in
+constexpr int kTreeWorkQueue = 4;      // word of Tree::work the group walk counts its groups in,
+constexpr int kTreeWorkSms = 2, kTreeWorkSmCount = 512;  // from its 2nd 32-bit half on, its blocks per SM
+constexpr int kTreeWorkWalk = 1 + kTreeWorkSmCount / 2;  // words of the walk
 
 struct Tree {
     // capacities

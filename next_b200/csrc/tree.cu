@@ -41,9 +41,10 @@ namespace nb {
 namespace {
 
 // Words of Tree::work, zeroed at the start of every build: two tile tickets,
-// the ready-list length, the deepest leaf level, the group walk's queue, then
-// the look-back statuses of the two scans.
-constexpr int kWorkCells = 0, kWorkChildren = 1, kWorkReady = 2, kWorkDeepest = 3, kWorkStatus = 5;
+// the ready-list length, the deepest leaf level, the group walk's queue and
+// blocks per SM, then the look-back statuses of the two scans.
+constexpr int kWorkCells = 0, kWorkChildren = 1, kWorkReady = 2, kWorkDeepest = 3,
+              kWorkStatus = kTreeWorkQueue + kTreeWorkWalk;
 static_assert(kTreeWorkQueue == 4, "the queue's word");
 
 // Internal cells per position, their ids and records, in one pass: d[s] for a

@@ -23,7 +23,8 @@
 // sums them in FP64.
 //
 // Scheduling: persistent blocks (SM count x resident blocks) pull groups
-// from a global atomic work queue.  All waits are warp-synchronous; there
+// from a global atomic work queue; with few groups, only as many warps of each
+// SM as its share of them (warps_per_sm below).  All waits are warp-synchronous; there
 // are no inter-block waits.  Stack or list overflow raises an error bit and
 // abandons the group.
 //
@@ -646,10 +647,28 @@ struct Fp64Arith {
     }
 };
 
+// Warps of an SM that take part.  With fewer groups than the GPU holds warps,
+// whoever came first took them, up to a block's worth on some SMs while others
+// had none, and a launch lasts as long as its fullest SM.  So a block counts
+// itself in on its SM, and the SM works with its share of the groups: one warp
+// each up to four, then a multiple of four (a warp per scheduler), to the
+// nearest, since a few groups left over cost less than an uneven SM.  From
+// about 18 groups per SM on, every resident warp takes part.  Walk, against all
+// warps taking part: 1,024 bodies (58 groups) 40 -> 35 us; 16,384 in groups of
+// 8 (2,616) 147 -> 135 us; collapse of 32,768 in groups of 32 (1,205) 212 ->
+// 136 us; of 65,536 (2,874, past the line) 250 us both; 1,048,576 unchanged.
+// Rounding down instead ran 101 us against 91 us at 2,800 groups of 8, rounding
+// up 150 us against 136 us at 2,616.
+__device__ __forceinline__ int64_t warps_per_sm(int64_t ngroups, int sm_count) {
+    const int64_t whole = (ngroups + sm_count - 1) / sm_count;
+    if (whole <= 4) return whole;
+    return (ngroups + 2 * sm_count) / (4 * sm_count) * 4;
+}
+
 template <class A>
 __global__ void __launch_bounds__(128, A::kMinBlocks)
 walk_group_kernel(Bodies bd, int64_t nbodies, Tree t, typename A::Scalar G, typename A::Scalar eps2, int stack_cap,
-                  unsigned long long* stats, int* err, int64_t own_lo, int64_t own_hi) {
+                  unsigned long long* stats, int* err, int sm_count, int64_t own_lo, int64_t own_hi) {
     if (*err & kErrAbort) return;
     unsigned int* queue = reinterpret_cast<unsigned int*>(t.work + kTreeWorkQueue);   // zeroed by the build
     using WarpLists = WarpListsT<A::kStageBytes>;
@@ -660,6 +679,14 @@ walk_group_kernel(Bodies bd, int64_t nbodies, Tree t, typename A::Scalar G, type
     int* stack = reinterpret_cast<int*>(smem_raw + sizeof(WarpLists) * nwarps) + w * stack_cap;
     const uint32_t lt = (1u << lane) - 1u;
     const int64_t ngroups = t.counts[2];
+    __shared__ unsigned int block_of_sm;
+    if (threadIdx.x == 0) {
+        unsigned int sm;
+        asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
+        block_of_sm = atomicAdd(queue + kTreeWorkSms + sm % kTreeWorkSmCount, 1u);
+    }
+    __syncthreads();
+    if (static_cast<int64_t>(block_of_sm) * nwarps + w >= warps_per_sm(ngroups, sm_count)) return;
     const unsigned nnodes32 = static_cast<unsigned>(t.counts[1]);
     const unsigned nbodies32 = static_cast<unsigned>(nbodies);
     unsigned long long npp = 0, npc = 0;
@@ -895,7 +922,7 @@ cudaError_t launch_variant(const Bodies& bd, int64_t nbodies, const Tree& t, con
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     using S = typename A::Scalar;
     kern<<<per_sm * sm_count, 32 * warps, smem, st>>>(bd, nbodies, t, static_cast<S>(P.G),
-                                                     static_cast<S>(P.eps * P.eps), stack_cap, stats, err,
+                                                     static_cast<S>(P.eps * P.eps), stack_cap, stats, err, sm_count,
                                                      P.own_lo, P.own_hi);
     count_launches(1);
     return cudaGetLastError();
