@@ -356,7 +356,9 @@ int build(next_handle* h, std::vector<int>* evs) {
                "root cube");
     h->cube_fresh = false;
     NB_TRY(sort_begin(n, h->key_bits, h->sort_scratch, h->st), "sort scratch");
-    NB_TRY(launch_keys(src, h->sysid, n, h->sys, h->keys, h->idx, h->key_bits, h->sort_scratch, h->st), "keys");
+    NB_TRY(launch_keys(src, h->sysid, n, h->sys, h->keys, h->idx, h->key_bits,
+                       sort_counts_digits(n) ? h->sort_scratch : nullptr, h->st),
+           "keys");
     rc0 = record(h, evs);
     if (rc0) return rc0;
     bool in_alt = false;

@@ -28,6 +28,7 @@ size_t sort_scratch_words(int64_t n);
 cudaError_t sort_prepare();
 // Clears a sort's scratch; its first 8 x 256 words then take the digit counts
 // (sort_digits.cuh) of the keys, from the kernel that makes them or sort_count.
+bool sort_counts_digits(int64_t n);                   // false: small sorts count for themselves
 cudaError_t sort_begin(int64_t n, int key_bits, uint32_t* scratch, cudaStream_t st);
 // counted: sort_begin and the counting have been queued already
 cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* alt_keys, uint32_t* alt_vals, int64_t n,

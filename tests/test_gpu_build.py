@@ -4,7 +4,7 @@ half-widths and masses of single bodies exactly; masses of cells to the rounding
 import numpy as np
 import pytest
 
-from next_b200 import ic
+from next_b200 import ic, native
 from next_b200.native import Simulation
 
 pytestmark = pytest.mark.gpu
@@ -69,6 +69,31 @@ def test_sort_at_the_layouts_edges(n):
         np.testing.assert_array_equal(vo, vals[order])
         np.testing.assert_array_equal(ko, keys[order])
     sim.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097])
+@pytest.mark.parametrize("bits", [1, 8, 13, 24, 63, 64])
+def test_sort_in_one_block(n, bits):
+    """Small sorts at the edges of their blocks and with partial last digits, among them keys of all ones (as the padding
+    behind the pairs): stable order by the low bits, bit for bit, by both entry points."""
+    rng = np.random.default_rng(n + bits)
+    keys = rng.integers(0, 2 ** 64, n, dtype=np.uint64, endpoint=False)
+    keys[rng.random(n) < 0.3] = np.uint64(2 ** 64 - 1)
+    vals = rng.integers(0, 2 ** 32, n, dtype=np.uint32)
+    order = np.argsort(keys & np.uint64(2 ** bits - 1), kind="stable")
+    sim = Simulation("accurate", "mixed")
+    k, v = sim.sort_pairs(keys, vals, bits)
+    np.testing.assert_array_equal(k, keys[order])
+    np.testing.assert_array_equal(v, vals[order])
+    sim.close()
+    torch = pytest.importorskip("torch")
+    src = torch.from_numpy(keys.view(np.int64)).cuda(), torch.from_numpy(vals.view(np.int32)).cuda()
+    out = torch.empty_like(src[0]), torch.empty_like(src[1])
+    rc = native.load().next_sort_pairs_noalloc(src[0].data_ptr(), src[1].data_ptr(), out[0].data_ptr(), out[1].data_ptr(), n,
+                                               bits, torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    np.testing.assert_array_equal(out[0].cpu().numpy().view(np.uint64), keys[order])
+    np.testing.assert_array_equal(out[1].cpu().numpy().view(np.uint32), vals[order])
 
 
 @pytest.mark.parametrize("systems,top", [(3, 400), (40, 60), (5000, 6)])
