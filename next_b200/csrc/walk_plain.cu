@@ -1,7 +1,7 @@
 // Plain FP64 force walks: every body opens the tree by its own distance.
 //
-// Reference physics: one thread per target body, depth-first over the tree in
-// octant order 0..7 -- the order bhAccel recurses (src/gravity/octree.h:176-178)
+// Reference physics: one thread per target body (several lanes in small
+// systems), depth-first over the tree in octant order 0..7 -- the order bhAccel recurses (src/gravity/octree.h:176-178)
 // -- with a per-level (next sibling, end) stack instead of recursion, and
 // bhAccel's arithmetic (octree.h:134-173, softening.h:21-35) operation for
 // operation.  Accurate physics (Plummer softening, full-width opening test,
@@ -60,6 +60,35 @@ __device__ __forceinline__ void add_stats(unsigned long long* stats, unsigned lo
         if (pp) atomicAdd(stats + 0, pp);
         if (pc) atomicAdd(stats + 1, pc);
     }
+}
+
+// The reference's opening test, size / dist < theta with dist = sqrt(r2 + 1e-20) (octree.h:153): decided by
+// the squares wherever they differ by more than the square root's and the division's rounding could hide, by
+// the reference's own operations otherwise.
+__device__ __forceinline__ bool ref_opens(const double4& c, double size, double xi, double yi, double zi, double theta,
+                                          double theta2, bool squarable) {
+    const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
+    const double d2 = dx * dx + dy * dy + dz * dz + 1e-20;
+    const double s2 = size * size, t2 = theta2 * d2;
+    bool near = squarable && s2 > t2 * (1.0 + 1e-14);
+    const bool far = squarable && s2 < t2 * (1.0 - 1e-14);
+    if (!near && !far) near = !((size / sqrt(d2)) < theta);
+    return near;
+}
+
+// A listed node's addends for a target at (xi, yi, zi).
+__device__ __forceinline__ RefTerm ref_entry(const Tree& t, int64_t nd, bool leaf, double xi, double yi, double zi,
+                                             double mi, bool dark, bool stored) {
+    const double4 c = t.com[nd];
+    const double2 soft = t.soft[2 * nd + 1];               // base and dark softening of the node
+    double2 qa = make_double2(0.0, 0.0), qb = qa, qc = qa; // a body has no quadrupole
+    const double2* q2 = reinterpret_cast<const double2*>(t.quad64 + 8 * nd);
+    if (!leaf) { qa = q2[0]; qb = q2[1]; qc = q2[2]; }
+    const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    double sd = -1.0;
+    if (dark) sd = stored ? soft.y : softening_dark(t.soft[2 * nd].x, c.w, mi);
+    return ref_term(c.w, dx, dy, dz, r2, soft.x, sd, qa, qb, qc);
 }
 
 // Reference physics.  The warp alternates between two phases: first every
@@ -124,16 +153,7 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
                 break;
             }
             if (!leaf) {
-                // size / dist < theta (octree.h:153), dist = sqrt(r2 + 1e-20): decided by the squares
-                // wherever they differ by more than the square root's and the division's rounding
-                // could hide, by the reference's own operations otherwise
-                const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
-                const double d2 = dx * dx + dy * dy + dz * dz + 1e-20;
-                const double s2 = size * size, t2 = theta2 * d2;
-                bool near = P.theta_squarable && s2 > t2 * (1.0 + 1e-14);
-                const bool far = P.theta_squarable && s2 < t2 * (1.0 - 1e-14);
-                if (!near && !far) near = !((size / sqrt(d2)) < theta);
-                if (near) {
+                if (ref_opens(c, size, xi, yi, zi, theta, theta2, P.theta_squarable)) {
                     stack[sp++] = make_int2(cur, end);
                     cur = lk.x;
                     end = lk.x + lk.y;
@@ -165,17 +185,7 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
         for (int e = 0; e < cnt; ++e) {
             const unsigned entry = list[e][threadIdx.x];
             const bool leaf = entry & kRefLeaf;
-            const int64_t nd = entry & ~kRefLeaf;
-            const double4 c = t.com[nd];
-            const double2 soft = t.soft[2 * nd + 1];               // base and dark softening of the node
-            double2 qa = make_double2(0.0, 0.0), qb = qa, qc = qa; // a body has no quadrupole
-            const double2* q2 = reinterpret_cast<const double2*>(t.quad64 + 8 * nd);
-            if (!leaf) { qa = q2[0]; qb = q2[1]; qc = q2[2]; }
-            const double dx = c.x - xi, dy = c.y - yi, dz = c.z - zi;
-            const double r2 = dx * dx + dy * dy + dz * dz;
-            double sd = -1.0;
-            if (dark) sd = stored ? soft.y : softening_dark(t.soft[2 * nd].x, c.w, mi);
-            const RefTerm f = ref_term(c.w, dx, dy, dz, r2, soft.x, sd, qa, qb, qc);
+            const RefTerm f = ref_entry(t, entry & ~kRefLeaf, leaf, xi, yi, zi, mi, dark, stored);
             ax += f.mx; ay += f.my; az += f.mz;
             ax += f.qx; ay += f.qy; az += f.qz;
             if (leaf) ++npp; else ++npc;
@@ -185,6 +195,183 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
     if (active) {
         bd.ax[i] = ax; bd.ay[i] = ay; bd.az[i] = az;
         if (bd.pot) bd.pot[i] = 0.0;
+    }
+    add_stats(stats, npp, npc);
+}
+
+// Reference physics with 8, 16 or 32 lanes per body, for small systems: the
+// lanes test the siblings of an opened cell at once and evaluate as many
+// accepted nodes at once as there are lanes; the addends go through shared
+// memory to the lanes that own the sums and are added there one by one in
+// depth-first order, so every bit is that of the walk above.
+//
+// Small systems are bound by the latency of one body's walk, a chain of some
+// hundred tests and interactions of about a microsecond each, whatever the
+// number of bodies.  Walk of 256 bodies 157 -> 46 us, 1,000 264 -> 60 us, 4,096
+// 377 -> 100 us, 16,384 460 -> 249 us, 32,768 485 -> 404 us (Plummer spheres;
+// infalling ones 87 -> 26, 132 -> 31, 178 -> 53, 228 -> 124, 249 -> 203 us).
+// More lanes are better while all warps are resident (five blocks per SM): 2,048
+// bodies 72 us with 32 lanes, 86 with 16 and 108 with 8; 4,096 129, 100 and 121
+// us; 8,192 210, 179 and 141 us.  Above 40,960 bodies the walk above has warps
+// enough and takes fewer instructions (65,536: 614 us against 796 us).
+//
+// A sub-warp's walk: the group being tested, or what is left of one behind its
+// first opened cell -- (first sibling, masks of accepted, opened, single-body
+// and bucket siblings) -- with the levels above on a stack.  Accepted siblings
+// before the next opened one join a ring of listed nodes.
+constexpr int kWideRing = 64;
+constexpr int64_t kWideWarps = 148 * 20;                           // resident at once
+constexpr int64_t kWideMax = 40960;
+template <int LANES>
+struct WideShared {
+    double term[6][33];                                            // mass and quadrupole addends per lane
+    int2 stack[32 / LANES][kMaxLevel + 2];
+    unsigned ring[32 / LANES][kWideRing];
+};
+
+template <int LANES>
+__global__ void __launch_bounds__(kRefThreads)
+walk_reference_wide_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree t, Params P,
+                           unsigned long long* stats, int* err) {
+    if (*err & kErrAbort) return;
+    __shared__ WideShared<LANES> shared[kRefThreads / 32];
+    WideShared<LANES>& S = shared[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, sub = lane / LANES, sl = lane % LANES;
+    const int64_t nodes = t.counts[1];
+    const int64_t i = (blockIdx.x * static_cast<int64_t>(kRefThreads / 32) + (threadIdx.x >> 5)) * (32 / LANES) + sub;
+    const bool active = i < n && i >= P.own_lo && i < P.own_hi;
+    const int64_t ii = active ? i : 0;
+    unsigned npp = 0, npc = 0;
+    const double xi = bd.x[ii], yi = bd.y[ii], zi = bd.z[ii], mi = bd.m[ii];
+    const bool dark = bd.type[ii] == 1;
+    const bool stored = dark && mi == *t.dark_mass;
+    const double theta = P.theta, theta2 = theta * theta;
+    double sum = 0.0;                                              // lanes 0..2 of a body: x, y, z
+    int first = sysid ? sysid[ii] : 0, count = active ? 1 : 0;     // siblings to test
+    unsigned rest = 0;                                             // or masks of tested ones, 8 bits each:
+    int sp = 0, head = 0, cnt = 0, bucket = -1;                    // accepted, opened, single bodies, buckets
+    for (;;) {
+        for (;;) {
+            const bool open_work = (count > 0 || rest != 0 || sp > 0) && bucket < 0;
+            if (!__any_sync(0xffffffffu, open_work && cnt < LANES)) break;
+            const bool go = open_work && cnt <= kWideRing - 8;
+            const bool fresh = go && count > 0;
+            if (go && !fresh && rest == 0) {
+                --sp;
+                const int2 item = S.stack[sub][sp];
+                first = item.x;
+                rest = static_cast<unsigned>(item.y);
+            }
+            __syncwarp();
+            bool accept = false, leaf = false, open = false, many = false;
+            int2 lk = make_int2(0, 0);
+            const int64_t k = static_cast<int64_t>(first) + sl;
+            if (fresh && sl < count) {
+                if (k < 0 || k >= nodes) {
+                    raise_error(err, kErrIndex);
+                } else {
+                    const double4 c = t.com[k];
+                    const double2 nh = t.soft[2 * k];              // half-width and link
+                    lk = make_int2(__double2loint(nh.y), __double2hiint(nh.y));
+                    leaf = lk.y <= 0;
+                    // children lie behind their parent in the tree, so a walk ends
+                    if (leaf ? (lk.x < 0 || static_cast<int64_t>(lk.x) - lk.y > n) : (lk.x <= k || lk.y > 8)) {
+                        if (c.w != 0.0) raise_error(err, kErrIndex);
+                    } else if (c.w != 0.0) {
+                        many = leaf && lk.y != -1;
+                        open = many || (!leaf && ref_opens(c, nh.x, xi, yi, zi, theta, theta2, P.theta_squarable));
+                        accept = !open && !(leaf && lk.x == i);    // not its own leaf (octree.h:135)
+                    }
+                }
+            }
+            const int shift = LANES * sub;
+            const unsigned am = __ballot_sync(0xffffffffu, accept) >> shift & 0xffu;
+            const unsigned om = __ballot_sync(0xffffffffu, open) >> shift & 0xffu;
+            const unsigned lm = __ballot_sync(0xffffffffu, accept && leaf) >> shift & 0xffu;
+            const unsigned bm = __ballot_sync(0xffffffffu, many) >> shift & 0xffu;
+            if (fresh) { rest = am | om << 8 | lm << 16 | bm << 24; count = 0; }
+            const unsigned acc = rest & 0xffu, opened = rest >> 8 & 0xffu;
+            const int j = opened ? __ffs(static_cast<int>(opened)) - 1 : 8;
+            const int2 lj = make_int2(__shfl_sync(0xffffffffu, lk.x, shift + (j & 7)),
+                                      __shfl_sync(0xffffffffu, lk.y, shift + (j & 7)));
+            if (go) {
+                const unsigned pre = acc & ((1u << j) - 1u);
+                if (pre >> sl & 1u)
+                    S.ring[sub][(head + cnt + __popc(pre & ((1u << sl) - 1u))) % kWideRing] =
+                        static_cast<unsigned>(k) | (rest >> (16 + sl) & 1u ? kRefLeaf : 0u);
+                cnt += __popc(pre);
+                if (j == 8) {
+                    rest = 0;
+                } else {
+                    const unsigned later = 0xffu & ~((2u << j) - 1u);
+                    const unsigned left = rest & (later | later << 8 | later << 16 | later << 24);
+                    const bool is_bucket = rest >> (24 + j) & 1u;
+                    const int nd = first + j;
+                    if (left & 0xffffu) {
+                        if (sp < kMaxLevel + 2) {
+                            if (sl == 0) S.stack[sub][sp] = make_int2(first, static_cast<int>(left));
+                            ++sp;
+                        } else if (sl == 0) {
+                            raise_error(err, kErrStack);
+                        }
+                    }
+                    rest = 0;
+                    if (is_bucket) {
+                        bucket = nd;                               // its bodies follow the listed nodes
+                    } else {
+                        int2 ch = lj;
+                        if (!fresh) {
+                            const double2 nh = t.soft[2 * static_cast<int64_t>(nd)];
+                            ch = make_int2(__double2loint(nh.y), __double2hiint(nh.y));
+                        }
+                        first = ch.x;
+                        count = ch.y;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        const int take = min(cnt, LANES);
+        if (!__any_sync(0xffffffffu, take > 0 || bucket >= 0)) break;
+        if (sl < take) {
+            const unsigned entry = S.ring[sub][(head + sl) % kWideRing];
+            const bool leaf = entry & kRefLeaf;
+            const RefTerm f = ref_entry(t, entry & ~kRefLeaf, leaf, xi, yi, zi, mi, dark, stored);
+            S.term[0][lane] = f.mx; S.term[1][lane] = f.my; S.term[2][lane] = f.mz;
+            S.term[3][lane] = f.qx; S.term[4][lane] = f.qy; S.term[5][lane] = f.qz;
+            if (leaf) ++npp; else ++npc;
+        }
+        __syncwarp();
+        if (sl < 3)
+            for (int e = 0; e < take; ++e) {
+                sum += S.term[sl][sub * LANES + e];
+                sum += S.term[3 + sl][sub * LANES + e];
+            }
+        __syncwarp();
+        head += take;
+        cnt -= take;
+        if (bucket >= 0 && cnt == 0) {
+            // deepest-level bucket: its bodies act as one-body leaves of this size
+            const double2 nh = t.soft[2 * static_cast<int64_t>(bucket)];
+            const int2 lk = make_int2(__double2loint(nh.y), __double2hiint(nh.y));
+            const double2 zero = make_double2(0.0, 0.0);
+            for (int b = lk.x; b < lk.x - lk.y; ++b) {
+                const double mj = bd.m[b];
+                if (b == i || mj == 0.0) continue;
+                const double ex = bd.x[b] - xi, ey = bd.y[b] - yi, ez = bd.z[b] - zi;
+                const double e2 = ex * ex + ey * ey + ez * ez;
+                const RefTerm f = ref_term(mj, ex, ey, ez, e2, softening_base(nh.x, mj),
+                                           dark ? softening_dark(nh.x, mj, mi) : -1.0, zero, zero, zero);
+                sum += sl == 0 ? f.mx : sl == 1 ? f.my : f.mz;
+                sum += sl == 0 ? f.qx : sl == 1 ? f.qy : f.qz;
+                if (sl == 0) ++npp;
+            }
+            bucket = -1;
+        }
+    }
+    if (active) {
+        if (sl < 3) (sl == 0 ? bd.ax : sl == 1 ? bd.ay : bd.az)[i] = sum;
+        if (sl == 3 && bd.pot) bd.pot[i] = 0.0;
     }
     add_stats(stats, npp, npc);
 }
@@ -495,6 +682,11 @@ cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int6
         const unsigned blocks = static_cast<unsigned>((warps + kPlainWarps - 1) / kPlainWarps);
         auto kern = potential ? walk_accurate_kernel<true> : walk_accurate_kernel<false>;
         kern<<<blocks, 32 * kPlainWarps, 0, st>>>(bd, sys.n > 1 ? d_offsets : nullptr, sys.n, sys.cube, n, t, P, stats, err);
+    } else if (n <= kWideMax) {
+        const int lanes = n <= kWideWarps ? 32 : n <= 2 * kWideWarps ? 16 : 8, per = kRefThreads / lanes;
+        auto kern = lanes == 32 ? walk_reference_wide_kernel<32>
+                                : lanes == 16 ? walk_reference_wide_kernel<16> : walk_reference_wide_kernel<8>;
+        kern<<<static_cast<unsigned>((n + per - 1) / per), kRefThreads, 0, st>>>(bd, sid, n, t, P, stats, err);
     } else {
         const unsigned blocks = static_cast<unsigned>((n + kRefThreads - 1) / kRefThreads);
         walk_reference_kernel<<<blocks, kRefThreads, 0, st>>>(bd, sid, n, t, P, stats, err);

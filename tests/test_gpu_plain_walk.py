@@ -158,6 +158,28 @@ def test_reference_walk_after_other_dark_masses(oracle):
     sim.close()
 
 
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 9, 33, 1000, 2960, 2961, 5920, 5921, 20001])
+def test_reference_walk_small_equals_large(n):
+    """A small system, walked by 32, 16 or 8 lanes per body, gets the bits it gets beside a system so large that one
+    thread walks for each body: with dark matter of two masses, coincident bodies (buckets) and massless ones."""
+    b, rest = reference_bodies(n, n), reference_bodies(41000, 2)
+    if n > 700:
+        for k in ("x", "y", "z"):
+            b[k][100:140] = b[k][100]
+            b[k][300:303] = b[k][300]
+        b["m"][200:600:9] = 0.0
+        b["m"][5:400:7] *= 3.0
+    one, both = Simulation("reference", "fp64"), Simulation("reference", "fp64")
+    one.upload(b)
+    both.upload({c: np.concatenate([b[c], rest[c]]) for c in b}, np.array([0, n, n + 41000]))
+    got, want = one.accel(), both.accel()
+    assert one.stats()["device_error"] == 0 and both.stats()["device_error"] == 0
+    for c in ("ax", "ay", "az"):
+        np.testing.assert_array_equal(got[c], want[c][:n])
+    one.close()
+    both.close()
+
+
 @pytest.mark.parametrize("length", [2.0 ** -400, 2.0 ** 400])
 def test_accurate_walk_far_from_unit_lengths(length):
     """Lengths scaled by a power of two round nothing: forces and potentials scale exactly, where the distances'
