@@ -257,7 +257,8 @@ int alloc_tree(next_handle* h, int64_t cap_int) {
     t.cap_group = n + h->nsys + 64;
     cudaError_t e = cudaSuccess;
     auto A = [&](auto** p, size_t c) { if (e == cudaSuccess) e = dalloc(p, c); };
-    A(&t.dlev, n + 1); A(&t.nint, n + 1);
+    A(&t.dlev, n + 16);                        // read 16 bytes at a time
+    A(&t.nint, n + 1);
     A(&t.int_start, cap_int); A(&t.int_level, cap_int); A(&t.int_bounds, 9 * cap_int);
     A(&t.int_packed, cap_int + 1); A(&t.counter, cap_int); A(&t.climb, cap_int); A(&t.cell, cap_int);
     A(&t.ready, cap_int);

@@ -202,9 +202,14 @@ __device__ int pack_groups(const int32_t* b, int level, int levels, int leaf_cap
 // flight per step and no divergence.  The counts of children and walk groups
 // are scanned here too (tiles of cells by ticket, look-back between them); the
 // last tile checks the totals.
-#ifndef NB_INT_SCAN
-#define NB_INT_SCAN 128
-#endif
+//
+// Bound by the instructions of a thread's searches (keys in shared memory
+// changed nothing at up to 22,000 bodies): reading dlev as 16-byte vectors,
+// tested four bytes at a time, and 32-bit positions instead of a byte at a time
+// and 64-bit ones took the build from 0.076 to 0.072 ms at 1,024 bodies, 0.109
+// to 0.106 ms at 16,384, 0.215 to 0.210 ms at 1,048,576, and 0.548 to 0.522 ms
+// with as many one-body leaves.
+constexpr int kEndScan = 128;
 // The child bounds of cell q, stored, and its counts of children and groups.
 __device__ __forceinline__ void find_children(const uint64_t* __restrict__ keys, int64_t n,
                                               const int32_t* __restrict__ sysid, const int64_t* __restrict__ offsets,
@@ -224,28 +229,39 @@ __device__ __forceinline__ void find_children(const uint64_t* __restrict__ keys,
 #pragma unroll
     for (int c = 1; c < 8; ++c) v[c] = prefix | (static_cast<uint64_t>(c) << csh);
     // A small cell's end is the first p > s whose key shares fewer than l
-    // digits with its predecessor (dlev[p] < l): found by reading dlev
-    // forward, 16 positions per round trip, for up to NB_INT_SCAN
-    // positions; the children's searches then run over the cell only.
-    int64_t e = -1;
-    if (NB_INT_SCAN > 0) {
-        const int64_t lim = hi < static_cast<int64_t>(s) + 1 + NB_INT_SCAN ? hi : static_cast<int64_t>(s) + 1 + NB_INT_SCAN;
-        for (int64_t p0 = static_cast<int64_t>(s) + 1; p0 < lim && e < 0; p0 += 16) {
-            int dv[16];
+    // digits with its predecessor (dlev[p] < l): found by reading dlev forward,
+    // 32 aligned bytes per round trip, for some kEndScan positions; the
+    // children's searches then run over the cell only.
+    const int hi32 = static_cast<int>(hi);
+    int e = -1;
+    {
+        const int lim = min(hi32, s + 1 + kEndScan);
+        const unsigned l4 = 0x01010101u * static_cast<unsigned>(l);
+        for (int w0 = (s + 1) & ~15; w0 < lim && e < 0; w0 += 32) {
+            uint4 v2[2];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) dv[j] = p0 + j < lim ? t.dlev[p0 + j] : 127;
+            for (int j = 0; j < 2; ++j)
+                v2[j] = w0 + 16 * j < lim ? *reinterpret_cast<const uint4*>(t.dlev + w0 + 16 * j) : make_uint4(~0u, ~0u, ~0u, ~0u);
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
-                if (e < 0 && dv[j] < l) e = p0 + j;
+            for (int j = 7; j >= 0; --j) {
+                const uint4& q4 = v2[j >> 2];
+                const unsigned word = (j & 3) == 0 ? q4.x : (j & 3) == 1 ? q4.y : (j & 3) == 2 ? q4.z : q4.w;
+                // the top bit of each byte below l: bytes and l are at most 21, and a system's start
+                // (-1) is never inside the range
+                unsigned less = ~((word | 0x80808080u) - l4) & 0x80808080u;
+                const int p = w0 + 4 * j;
+                if (p <= s) less = s + 1 - p >= 4 ? 0u : less & (~0u << 8 * (s + 1 - p));
+                if (less) e = p + ((__ffs(static_cast<int>(less)) - 1) >> 3);
+            }
         }
-        if (e < 0 && lim == hi) e = hi;
+        if (e > lim || (e < 0 && lim == hi32)) e = lim == hi32 ? hi32 : -1;
     }
-    int64_t pos[8];
+    int pos[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) pos[c] = s;
-    int64_t len = (e >= 0 ? e : hi) - s;
+    int len = (e >= 0 ? e : hi32) - s;
     while (len > 1) {
-        const int64_t half = len >> 1;
+        const int half = len >> 1;
 #pragma unroll
         for (int c = 0; c < 8; ++c) pos[c] = __ldg(keys + pos[c] + half) < v[c] ? pos[c] + half : pos[c];
         len -= half;
@@ -253,8 +269,8 @@ __device__ __forceinline__ void find_children(const uint64_t* __restrict__ keys,
     int32_t b[9];
     b[0] = s;
 #pragma unroll
-    for (int c = 1; c < 8; ++c) b[c] = static_cast<int32_t>(pos[c] + (__ldg(keys + pos[c]) < v[c] ? 1 : 0));
-    b[8] = e >= 0 ? static_cast<int32_t>(e) : static_cast<int32_t>(pos[0] + (__ldg(keys + pos[0]) < v[0] ? 1 : 0));
+    for (int c = 1; c < 8; ++c) b[c] = pos[c] + (__ldg(keys + pos[c]) < v[c] ? 1 : 0);
+    b[8] = e >= 0 ? e : pos[0] + (__ldg(keys + pos[0]) < v[0] ? 1 : 0);
     for (int c = 0; c < 8; ++c) *nchild += b[c + 1] > b[c];
     if (b[8] - b[0] > group_cap)
         *ngroups = pack_groups(b, l, levels, leaf_cap, group_cap, [](int, int) {});

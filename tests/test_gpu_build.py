@@ -54,6 +54,29 @@ def test_build_of_coincident_bodies_and_many_systems(oracle):
     sim.close()
 
 
+@pytest.mark.parametrize("leaf_cap", [1, 3, 16])
+def test_cells_of_every_length_and_alignment(oracle, leaf_cap):
+    """Clumps of 1 to 150 bodies, deep cells that start at every offset from a 16-byte boundary and end before, at and
+    behind the reach of the forward scan for a cell's end: the oracle's tree, node for node."""
+    rng = np.random.default_rng(6)
+    sizes = list(range(1, 40)) + [61, 62, 63, 64, 65, 95, 96, 97, 111, 112, 113, 126, 127, 128, 129, 130, 143, 144, 145, 150]
+    parts = [rng.uniform(-1.0, 1.0, 3) + rng.uniform(-1e-3, 1e-3, (k, 3)) for k in rng.permutation(sizes)]
+    p = np.concatenate(parts)
+    b = {k: np.ascontiguousarray(p[:, a]) for a, k in enumerate("xyz")}
+    for k in ("vx", "vy", "vz"):
+        b[k] = np.zeros(len(p))
+    b["m"] = np.full(len(p), 1.0 / len(p))
+    sim = Simulation("accurate", "fp64", leaf_cap=leaf_cap)
+    sim.upload(b)
+    t, r = sim.debug_tree(), oracle.tree(b, mode="accurate", leaf_cap=leaf_cap)
+    assert t.shape == r.shape
+    for c in (LEVEL, HALF, LEAF):
+        np.testing.assert_array_equal(t[:, c], r[:, c])
+    np.testing.assert_allclose(t[:, MASS], r[:, MASS], rtol=1e-14, atol=0)
+    assert sim.stats()["device_error"] == 0
+    sim.close()
+
+
 @pytest.mark.parametrize("n", [1, 2, 1023, 1024, 1025, 148 * 1024, 148 * 1024 + 1, 148 * 2048, 148 * 2048 + 1, 148 * 4096,
                                148 * 4096 + 1, 148 * 7680, 148 * 7680 + 1])
 def test_sort_at_the_layouts_edges(n):
