@@ -17,6 +17,8 @@
 // NEXT_DEVERR_SORT_TIMEOUT instead of spinning forever.
 //
 // Memory bound: per pass 12 B read + 12 B written per pair.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 #include "kernels.cuh"
 #include "sort_digits.cuh"
@@ -307,13 +309,6 @@ onesweep_kernel(const uint64_t* __restrict__ keys_in, const uint32_t* __restrict
 // in shared memory, by the same counts and ranking as above, without the
 // counts in global memory and their clearing.  In place or not: all pairs are
 // read before the first is written.
-//
-// Small sorts are bound by their launches, one per pass: the sort of a tree
-// build of 1,024 bodies 19 -> 10.5 us (30 key bits), of 2,048 21 -> 12.5 us, of
-// 4,096 22.5 -> 16.5 us; a sort of 63-bit keys by the entry point for device
-// buffers, host call included, 75 -> 37, 39 and 49 us.  Tiles on several SMs win
-// from there on: a build of 6,000 bodies sorts in 21 us so and in 25 us in one
-// block.
 template <int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS)
 one_block_kernel(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out, uint32_t* vals_out, int n,
@@ -390,18 +385,20 @@ one_block_kernel(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* key
     }
 }
 
-struct OneBlock {
+struct SmallSort {
     int pairs;
-    void (*launch)(int n, const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int key_bits, cudaStream_t st);
+    cudaError_t (*launch)(int n, const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int key_bits,
+                          cudaStream_t st);
     cudaError_t (*prepare)();
 };
 
 template <int THREADS, int ITEMS>
-constexpr OneBlock one_block() {
+constexpr SmallSort one_block() {
     return {THREADS * ITEMS,
             [](int n, const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int key_bits, cudaStream_t st) {
                 one_block_kernel<THREADS, ITEMS><<<1, THREADS, sizeof(SortSmemT<THREADS, ITEMS>), st>>>(ki, vi, ko, vo, n,
                                                                                                        key_bits);
+                return cudaGetLastError();
             },
             []() {
                 return cudaFuncSetAttribute(one_block_kernel<THREADS, ITEMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -409,18 +406,161 @@ constexpr OneBlock one_block() {
             }};
 }
 
-constexpr OneBlock kOneBlock[] = {one_block<256, 4>(), one_block<512, 4>(), one_block<512, 8>()};
-constexpr int64_t kOneBlockPairs = 4096;
+// A sort of at most C x THREADS x ITEMS pairs by one cluster of C blocks: a
+// block holds a tile of the pairs in registers; a pass exchanges the tiles'
+// digit counts through the cluster's shared memory, so every block knows the
+// next position of each of its pairs, and sends them to the shared memory of
+// the blocks that hold those positions.  Bound by those scattered stores and
+// the two cluster barriers of a pass: a pair goes as one 16-byte store (as two,
+// 16,384 pairs 26.9 us against 24.8 us).
+template <int THREADS, int ITEMS>
+struct ClusterSmemT {
+    uint32_t warp_hist[THREADS / 32][kRadix];
+    uint32_t count[kRadix];           // the tile's, read by the other blocks
+    uint32_t warp_total[kRadix / 32];
+    ulonglong2 pairs[THREADS * ITEMS];   // key and value, written by the other blocks
+    uint32_t peers[ITEMS][THREADS];
+};
 
-cudaError_t sort_one_block(const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int64_t n, int key_bits,
-                           cudaStream_t st) {
-    for (const OneBlock& b : kOneBlock)
-        if (n <= b.pairs) {
-            b.launch(static_cast<int>(n), ki, vi, ko, vo, key_bits, st);
-            break;
+template <int C, int THREADS, int ITEMS>
+__global__ void __launch_bounds__(THREADS)
+cluster_sort_kernel(const uint64_t* keys_in, const uint32_t* vals_in, uint64_t* keys_out, uint32_t* vals_out, int n,
+                    int key_bits) {
+    namespace cg = cooperative_groups;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    using Smem = ClusterSmemT<THREADS, ITEMS>;
+    Smem& S = *reinterpret_cast<Smem*>(smem_raw);
+    constexpr int kWarps = THREADS / 32, kTile = THREADS * ITEMS;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = static_cast<int>(cluster.block_rank());
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int d = threadIdx.x;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint64_t key[ITEMS];
+    uint32_t val[ITEMS];
+    load_tile<THREADS, ITEMS>(keys_in, vals_in, n, rank, w, lane, key, val);   // the padding stays behind every pair
+    for (int p = 0; 8 * p < key_bits; ++p) {
+        const int shift = 8 * p;
+        const uint32_t dmask = pass_mask(key_bits, p);
+        for (int i = threadIdx.x; i < kWarps * kRadix; i += THREADS) (&S.warp_hist[0][0])[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int dk = static_cast<int>((key[k] >> shift) & dmask);
+            const uint32_t peers = digit_peers(dk);
+            S.peers[k][threadIdx.x] = peers;
+            if ((peers & lt) == 0) atomicAdd(&S.warp_hist[w][dk], static_cast<uint32_t>(__popc(peers)));
         }
-    count_launches(1);
-    return cudaGetLastError();
+        __syncthreads();
+        uint32_t c[kWarps], mine = 0;
+        if (d < kRadix) {
+#pragma unroll
+            for (int ww = 0; ww < kWarps; ++ww) c[ww] = S.warp_hist[ww][d];
+#pragma unroll
+            for (int ww = 0; ww < kWarps; ++ww) mine += c[ww];
+            S.count[d] = mine;
+        }
+        cluster.sync();
+        // per digit: the pairs of the tiles before this one, and of all tiles
+        uint32_t before = 0, all = 0;
+        if (d < kRadix) {
+            uint32_t v[C];
+#pragma unroll
+            for (int b = 0; b < C; ++b) v[b] = *cluster.map_shared_rank(&S.count[d], b);
+#pragma unroll
+            for (int b = 0; b < C; ++b) {
+                before += b < rank ? v[b] : 0u;
+                all += v[b];
+            }
+        }
+        uint32_t inc = all;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (d < kRadix && lane == 31) S.warp_total[w] = inc;
+        __syncthreads();
+        if (d < kRadix) {
+            uint32_t start = inc - all + before;
+            for (int ww = 0; ww < w; ++ww) start += S.warp_total[ww];
+#pragma unroll
+            for (int ww = 0; ww < kWarps; ++ww) { S.warp_hist[ww][d] = start; start += c[ww]; }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int dk = static_cast<int>((key[k] >> shift) & dmask);
+            const uint32_t peers = S.peers[k][threadIdx.x];
+            const uint32_t base = S.warp_hist[w][dk];
+            const uint32_t pos = base + __popc(peers & lt);          // below C x kTile
+            __syncwarp();
+            if ((peers & lt) == 0) S.warp_hist[w][dk] = base + __popc(peers);
+            cluster.map_shared_rank(&S, pos / kTile)->pairs[pos % kTile] = make_ulonglong2(key[k], val[k]);
+            __syncwarp();
+        }
+        cluster.sync();               // every pair has arrived, and every count has been read
+#pragma unroll
+        for (int k = 0; k < ITEMS; ++k) {
+            const int i = (w * ITEMS + k) * 32 + lane;
+            const ulonglong2 kv = S.pairs[i];
+            key[k] = kv.x;
+            val[k] = static_cast<uint32_t>(kv.y);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+        const int i = rank * kTile + (w * ITEMS + k) * 32 + lane;
+        if (i < n) { keys_out[i] = key[k]; vals_out[i] = val[k]; }
+    }
+}
+
+template <int C, int THREADS, int ITEMS>
+constexpr SmallSort cluster_sort() {
+    return {C * THREADS * ITEMS,
+            [](int n, const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int key_bits, cudaStream_t st) {
+                cudaLaunchAttribute attr{};
+                attr.id = cudaLaunchAttributeClusterDimension;
+                attr.val.clusterDim.x = C;
+                attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+                cudaLaunchConfig_t cfg{};
+                cfg.gridDim = dim3(C);
+                cfg.blockDim = dim3(THREADS);
+                cfg.dynamicSmemBytes = sizeof(ClusterSmemT<THREADS, ITEMS>);
+                cfg.stream = st;
+                cfg.attrs = &attr;
+                cfg.numAttrs = 1;
+                return cudaLaunchKernelEx(&cfg, cluster_sort_kernel<C, THREADS, ITEMS>, ki, vi, ko, vo, n, key_bits);
+            },
+            []() {
+                return cudaFuncSetAttribute(cluster_sort_kernel<C, THREADS, ITEMS>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            static_cast<int>(sizeof(ClusterSmemT<THREADS, ITEMS>)));
+            }};
+}
+
+// Small sorts, by size: one block up to 2,048 pairs, a cluster of four or eight
+// blocks (which every GPU of this kind can launch) up to 16,384.  They need no
+// counts in global memory, no clearing of them and one launch, where the passes
+// above are a launch of two to six microseconds each.  Sort of a tree build,
+// 30 to 39 key bits / 63 bits: 1,024 bodies 19 -> 10 / 14 us, 2,048 21 -> 12.5 / 20
+// us, 4,096 22.5 -> 14.6 / 29 (in one block) -> 22.6 us, 8,192 21 -> 16 / 52 -> 26.5 us,
+// 16,384 27 -> 24.5 / 52 -> 35 us; by the entry point for device buffers, 63 bits,
+// host call included, 75-79 -> 34, 36, 46, 45 and 58 us.  From there on tiles on more
+// SMs win: 32,768 bodies 31 us against 35 us by a cluster of eight.  Sixteen
+// blocks per cluster measured 24.8 us at 16,384 and 19 us at 8,192.
+constexpr SmallSort kSmallSorts[] = {one_block<256, 4>(), one_block<512, 4>(), cluster_sort<4, 256, 4>(),
+                                     cluster_sort<8, 256, 4>(), cluster_sort<8, 512, 4>()};
+constexpr int64_t kSmallPairs = 16384;
+
+cudaError_t sort_small(const uint64_t* ki, const uint32_t* vi, uint64_t* ko, uint32_t* vo, int64_t n, int key_bits,
+                       cudaStream_t st) {
+    for (const SmallSort& s : kSmallSorts)
+        if (n <= s.pairs) {
+            count_launches(1);
+            return s.launch(static_cast<int>(n), ki, vi, ko, vo, key_bits, st);
+        }
+    return cudaErrorInvalidValue;
 }
 
 // Tile layouts.  Up to 148 x 512 x 15 = 1,136,640 pairs the smallest layout is
@@ -429,8 +569,8 @@ cudaError_t sort_one_block(const uint64_t* ki, const uint32_t* vi, uint64_t* ko,
 // following a chain of look-backs.  Above that, tiles of 256 x 15, three blocks
 // per SM, whose phases overlap, with the look-back.  Whole sorts of 63-bit keys
 // by the entry point for device buffers, host call included, against 256 x 8
-// up to 262,144 pairs and 256 x 15 above: 16,384 pairs 97 -> 72 us, 262,144 117 ->
-// 106 us, 1,048,576 164 -> 143 us.  A pass is bound there by the ballots and the
+// up to 262,144 pairs and 256 x 15 above: 262,144 pairs 117 -> 106 us, 1,048,576
+// 164 -> 143 us.  A pass is bound there by the ballots and the
 // ranking of an SM's own tile.
 struct Layout {
     int pairs;                 // per tile
@@ -503,12 +643,12 @@ cudaError_t sort_prepare() {
     cudaError_t e = kManyTiles.prepare();
     for (const Layout& l : kOneTile)
         if (e == cudaSuccess) e = l.prepare();
-    for (const OneBlock& b : kOneBlock)
+    for (const SmallSort& b : kSmallSorts)
         if (e == cudaSuccess) e = b.prepare();
     return e;
 }
 
-bool sort_counts_digits(int64_t n) { return n > kOneBlockPairs; }
+bool sort_counts_digits(int64_t n) { return n > kSmallPairs; }
 
 // Clears the scratch of a sort of n pairs; the digit counts (the scratch's
 // first 8 x 256 words) can be added to from then on.
@@ -563,7 +703,7 @@ cudaError_t radix_sort_pairs(uint64_t* keys, uint32_t* vals, uint64_t* alt_keys,
                              cudaStream_t st) {
     *in_alt = false;
     if (n <= 1) return cudaSuccess;
-    if (!sort_counts_digits(n)) return sort_one_block(keys, vals, keys, vals, n, key_bits, st);
+    if (!sort_counts_digits(n)) return sort_small(keys, vals, keys, vals, n, key_bits, st);
     cudaError_t e = cudaSuccess;
     if (!counted) {
         e = sort_begin(n, key_bits, scratch, st);
@@ -586,7 +726,7 @@ cudaError_t radix_sort_pairs_to(const uint64_t* keys_in, const uint32_t* vals_in
         if (e == cudaSuccess) e = cudaMemcpyAsync(vals_out, vals_in, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
         return e;
     }
-    if (!sort_counts_digits(n)) return sort_one_block(keys_in, vals_in, keys_out, vals_out, n, key_bits, st);
+    if (!sort_counts_digits(n)) return sort_small(keys_in, vals_in, keys_out, vals_out, n, key_bits, st);
     cudaError_t e = sort_begin(n, key_bits, scratch, st);
     if (e == cudaSuccess) e = sort_count(keys_in, n, key_bits, scratch, st);
     if (e != cudaSuccess) return e;

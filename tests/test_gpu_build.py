@@ -94,10 +94,11 @@ def test_sort_at_the_layouts_edges(n):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 255, 256, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096, 4097, 8192,
+                               8193, 16383, 16384, 16385])
 @pytest.mark.parametrize("bits", [1, 8, 13, 24, 63, 64])
-def test_sort_in_one_block(n, bits):
-    """Small sorts at the edges of their blocks and with partial last digits, among them keys of all ones (as the padding
+def test_sort_in_one_launch(n, bits):
+    """Small sorts at the edges of their blocks and clusters and with partial last digits, among them keys of all ones (as the padding
     behind the pairs): stable order by the low bits, bit for bit, by both entry points."""
     rng = np.random.default_rng(n + bits)
     keys = rng.integers(0, 2 ** 64, n, dtype=np.uint64, endpoint=False)
