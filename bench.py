@@ -7,8 +7,8 @@ system (tree build + force walk + kick/drift), bodies resident on the device.
 
 The JSON line's `value` is the FP32-mixed step (FP32 interactions with
 compensated accumulation, FP64 kick/drift, moments and diagnostics).  Beside
-it: the plain FP64 GPU step (one thread per body, the reference's step
-structure: two tree builds per step), the force error of both against FP64
+it: the plain FP64 GPU step (every body opens the tree by its own distance; the
+reference's step structure: two tree builds per step), the force error of both against FP64
 direct summation on 4096 seeded bodies, the walk's FP32-pipe roofline, the
 reference's own OpenMP Step() timed on the host cores, and an end-to-end
 figure through the C ABI with host buffers.
@@ -298,7 +298,7 @@ def ensemble_error(bodies, offsets, a, cfg, device, k_systems=8):
 
 
 def plain_fp64_leg(bodies, offsets, cfg, device, steps, idx):
-    """The plain FP64 GPU step (one thread per body, two tree builds per step)."""
+    """The plain FP64 GPU step (every body opens the tree itself, two tree builds per step)."""
     from next_b200.native import Simulation
     if offsets is None:
         p = Simulation("accurate", "fp64", theta=cfg["theta"], eps=cfg["eps"], leaf_cap=1, reuse_forces=False,
@@ -318,7 +318,7 @@ def plain_fp64_leg(bodies, offsets, cfg, device, steps, idx):
         p.close()
         n = bodies["x"].shape[0]
         return {"value": n * steps / (st["ms_step"] * 1e-3), "steps": steps, "ms_per_step": st["ms_step"] / steps,
-                "force_error": err, "structure": "one thread per body, leaf_cap 1, two tree builds per step"}
+                "force_error": err, "structure": "a warp per seven bodies that open the tree each by its own distance, leaf_cap 1, two tree builds per step"}
     # ensemble: loop the single-system plain FP64 step over a sample of systems
     rng = np.random.default_rng(99)
     pick = rng.choice(len(offsets) - 1, 16, replace=False)

@@ -57,8 +57,9 @@ extern "C" {
 #define NEXT_PHYSICS_REFERENCE 0
 #define NEXT_PHYSICS_ACCURATE 1
 
-/* NEXT_PRECISION_FP64: plain FP64 walk, one thread per body, depth-first in
- *   the reference's child order; two tree builds per step as in step.h.
+/* NEXT_PRECISION_FP64: plain FP64 walk, every body opening the tree by its own
+ *   distance (reference physics: depth-first in the reference's child order);
+ *   two tree builds per step as in step.h.
  * NEXT_PRECISION_MIXED: FP32 interactions in a warp-per-group walk with
  *   shared-memory interaction lists and compensated accumulation; FP64 for
  *   positions, velocities, kick/drift, tree moments and diagnostics.
