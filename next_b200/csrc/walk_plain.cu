@@ -208,20 +208,23 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
 // Small systems are bound by the latency of one body's walk, a chain of some
 // hundred tests and interactions of about a microsecond each, whatever the
 // number of bodies.  Walk of 256 bodies 157 -> 46 us, 1,000 264 -> 60 us, 4,096
-// 377 -> 100 us, 16,384 460 -> 249 us, 32,768 485 -> 404 us (Plummer spheres;
-// infalling ones 87 -> 26, 132 -> 31, 178 -> 53, 228 -> 124, 249 -> 203 us).
-// More lanes are better while all warps are resident (five blocks per SM): 2,048
-// bodies 72 us with 32 lanes, 86 with 16 and 108 with 8; 4,096 129, 100 and 121
-// us; 8,192 210, 179 and 141 us.  Above 40,960 bodies the walk above has warps
-// enough and takes fewer instructions (65,536: 614 us against 796 us).
+// 377 -> 97 us, 16,384 460 -> 206 us, 32,768 485 -> 372 us (Plummer spheres;
+// infalling ones 87 -> 26, 132 -> 31, 178 -> 51, 226 -> 102, 254 -> 191 us).
+// More lanes are better while all warps are resident: 2,048 bodies 72 us with 32
+// lanes, 86 with 16 and 108 with 8; 4,096 129, 100 and 121 us; 8,192 210, 179 and
+// 141 us.  Eight lanes at 5, 6 and 7 blocks per SM (96, 80 and 72 registers):
+// 8,192 bodies 135, 152 and 159 us, 14,000 218, 166 and 186, 16,384 236, 230 and
+// 206, 40,960 491, 449 and 499 us.  Above 49,152 bodies (550 us against 562 us)
+// the walk above has warps enough and takes fewer instructions, which bind
+// there (57,344: 575 us against 619 us); 32-bit indices and the sums without a
+// loop took 5% off these walks.
 //
 // A sub-warp's walk: the group being tested, or what is left of one behind its
 // first opened cell -- (first sibling, masks of accepted, opened, single-body
 // and bucket siblings) -- with the levels above on a stack.  Accepted siblings
 // before the next opened one join a ring of listed nodes.
 constexpr int kWideRing = 64;
-constexpr int64_t kWideWarps = 148 * 20;                           // resident at once
-constexpr int64_t kWideMax = 40960;
+constexpr int64_t kWideMax = 49152;
 template <int LANES>
 struct WideShared {
     double term[6][33];                                            // mass and quadrupole addends per lane
@@ -229,18 +232,19 @@ struct WideShared {
     unsigned ring[32 / LANES][kWideRing];
 };
 
-template <int LANES>
-__global__ void __launch_bounds__(kRefThreads)
+template <int LANES, int MINB>
+__global__ void __launch_bounds__(kRefThreads, MINB)
 walk_reference_wide_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree t, Params P,
                            unsigned long long* stats, int* err) {
     if (*err & kErrAbort) return;
     __shared__ WideShared<LANES> shared[kRefThreads / 32];
     WideShared<LANES>& S = shared[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, sub = lane / LANES, sl = lane % LANES;
-    const int64_t nodes = t.counts[1];
+    const unsigned nodes = static_cast<unsigned>(t.counts[1]), nbodies = static_cast<unsigned>(n);
     const int64_t i = (blockIdx.x * static_cast<int64_t>(kRefThreads / 32) + (threadIdx.x >> 5)) * (32 / LANES) + sub;
     const bool active = i < n && i >= P.own_lo && i < P.own_hi;
     const int64_t ii = active ? i : 0;
+    const int self = static_cast<int>(i);
     unsigned npp = 0, npc = 0;
     const double xi = bd.x[ii], yi = bd.y[ii], zi = bd.z[ii], mi = bd.m[ii];
     const bool dark = bd.type[ii] == 1;
@@ -265,22 +269,23 @@ walk_reference_wide_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t
             __syncwarp();
             bool accept = false, leaf = false, open = false, many = false;
             int2 lk = make_int2(0, 0);
-            const int64_t k = static_cast<int64_t>(first) + sl;
+            const int k = first + sl;
             if (fresh && sl < count) {
-                if (k < 0 || k >= nodes) {
+                if (static_cast<unsigned>(k) >= nodes) {
                     raise_error(err, kErrIndex);
                 } else {
                     const double4 c = t.com[k];
-                    const double2 nh = t.soft[2 * k];              // half-width and link
+                    const double2 nh = t.soft[2 * static_cast<int64_t>(k)];    // half-width and link
                     lk = make_int2(__double2loint(nh.y), __double2hiint(nh.y));
                     leaf = lk.y <= 0;
                     // children lie behind their parent in the tree, so a walk ends
-                    if (leaf ? (lk.x < 0 || static_cast<int64_t>(lk.x) - lk.y > n) : (lk.x <= k || lk.y > 8)) {
+                    if (leaf ? (lk.x < 0 || static_cast<unsigned>(lk.x) - static_cast<unsigned>(lk.y) > nbodies)
+                             : (lk.x <= k || lk.y > 8)) {
                         if (c.w != 0.0) raise_error(err, kErrIndex);
                     } else if (c.w != 0.0) {
                         many = leaf && lk.y != -1;
                         open = many || (!leaf && ref_opens(c, nh.x, xi, yi, zi, theta, theta2, P.theta_squarable));
-                        accept = !open && !(leaf && lk.x == i);    // not its own leaf (octree.h:135)
+                        accept = !open && !(leaf && lk.x == self);    // not its own leaf (octree.h:135)
                     }
                 }
             }
@@ -342,11 +347,17 @@ walk_reference_wide_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t
             if (leaf) ++npp; else ++npc;
         }
         __syncwarp();
-        if (sl < 3)
-            for (int e = 0; e < take; ++e) {
-                sum += S.term[sl][sub * LANES + e];
-                sum += S.term[3 + sl][sub * LANES + e];
+        if (sl < 3) {
+            const double* m = &S.term[sl][sub * LANES];
+            const double* q = &S.term[3 + sl][sub * LANES];
+#pragma unroll
+            for (int e = 0; e < LANES; ++e) {
+                if (e < take) {
+                    sum += m[e];
+                    sum += q[e];
+                }
             }
+        }
         __syncwarp();
         head += take;
         cnt -= take;
@@ -683,9 +694,14 @@ cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int6
         auto kern = potential ? walk_accurate_kernel<true> : walk_accurate_kernel<false>;
         kern<<<blocks, 32 * kPlainWarps, 0, st>>>(bd, sys.n > 1 ? d_offsets : nullptr, sys.n, sys.cube, n, t, P, stats, err);
     } else if (n <= kWideMax) {
-        const int lanes = n <= kWideWarps ? 32 : n <= 2 * kWideWarps ? 16 : 8, per = kRefThreads / lanes;
-        auto kern = lanes == 32 ? walk_reference_wide_kernel<32>
-                                : lanes == 16 ? walk_reference_wide_kernel<16> : walk_reference_wide_kernel<8>;
+        // as many lanes, then as many registers, as leave every warp resident at once
+        const int64_t block = 148 * (kRefThreads / 32);           // warps of one block per SM
+        const int lanes = n <= 5 * block ? 32 : n <= 10 * block ? 16 : 8, per = kRefThreads / lanes;
+        auto kern = lanes == 32      ? walk_reference_wide_kernel<32, 5>
+                    : lanes == 16    ? walk_reference_wide_kernel<16, 5>
+                    : n <= 20 * block ? walk_reference_wide_kernel<8, 5>
+                    : n > 24 * block && n <= 28 * block ? walk_reference_wide_kernel<8, 7>
+                                                        : walk_reference_wide_kernel<8, 6>;
         kern<<<static_cast<unsigned>((n + per - 1) / per), kRefThreads, 0, st>>>(bd, sid, n, t, P, stats, err);
     } else {
         const unsigned blocks = static_cast<unsigned>((n + kRefThreads - 1) / kRefThreads);

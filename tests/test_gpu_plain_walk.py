@@ -158,11 +158,11 @@ def test_reference_walk_after_other_dark_masses(oracle):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 7, 9, 33, 1000, 2960, 2961, 5920, 5921, 20001])
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 9, 33, 1000, 2960, 2961, 5920, 5921, 11841, 16000, 20001])
 def test_reference_walk_small_equals_large(n):
     """A small system, walked by 32, 16 or 8 lanes per body, gets the bits it gets beside a system so large that one
     thread walks for each body: with dark matter of two masses, coincident bodies (buckets) and massless ones."""
-    b, rest = reference_bodies(n, n), reference_bodies(41000, 2)
+    b, rest = reference_bodies(n, n), reference_bodies(50000, 2)
     if n > 700:
         for k in ("x", "y", "z"):
             b[k][100:140] = b[k][100]
@@ -171,7 +171,7 @@ def test_reference_walk_small_equals_large(n):
         b["m"][5:400:7] *= 3.0
     one, both = Simulation("reference", "fp64"), Simulation("reference", "fp64")
     one.upload(b)
-    both.upload({c: np.concatenate([b[c], rest[c]]) for c in b}, np.array([0, n, n + 41000]))
+    both.upload({c: np.concatenate([b[c], rest[c]]) for c in b}, np.array([0, n, n + 50000]))
     got, want = one.accel(), both.accel()
     assert one.stats()["device_error"] == 0 and both.stats()["device_error"] == 0
     for c in ("ax", "ay", "az"):
