@@ -1,6 +1,7 @@
-// Stable LSD radix sort of (uint64 key, uint32 value) pairs: one count of all
-// digits over the keys (made with the keys in a tree build), then one "onesweep" pass per 8-bit
-// digit.  A onesweep pass works on tiles of pairs (see Layout):
+// Stable LSD radix sort of (uint64 key, uint32 value) pairs, 8-bit digits.  Up
+// to 16,384 pairs one block or one cluster does all passes (kSmallSorts).  Above,
+// one count of all digits over the keys (made with the keys in a tree build),
+// then one "onesweep" pass per digit.  A onesweep pass works on tiles of pairs (see Layout):
 //   1. load the tile, count its digits per warp (ballot peer masks, kept in
 //      shared memory for the ranking; one shared add per digit group) and
 //      publish the per-digit tile counts in a status array (flag + count
