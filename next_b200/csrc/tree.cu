@@ -282,7 +282,9 @@ __global__ void __launch_bounds__(kChildThreads)
 internal_kernel(const uint64_t* __restrict__ keys, int64_t n, const int32_t* __restrict__ sysid,
                 const int64_t* __restrict__ offsets, int nsys, int base, int levels, int leaf_cap, int group_cap,
                 int64_t status_at, Tree t, int* err) {
-    if (*err & kErrAbort) {
+    // the whole block leaves or none of it: other blocks of this launch may be raising bits, and a block that
+    // only some of its threads left would take its tiles from a ticket that nobody writes
+    if (__syncthreads_or(*err & kErrAbort)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             t.counts[1] = t.counts[2] = nsys;
             t.counts[3] = static_cast<int64_t>(t.work[kWorkDeepest]);

@@ -669,7 +669,6 @@ template <class A>
 __global__ void __launch_bounds__(128, A::kMinBlocks)
 walk_group_kernel(Bodies bd, int64_t nbodies, Tree t, typename A::Scalar G, typename A::Scalar eps2, int stack_cap,
                   unsigned long long* stats, int* err, int sm_count, int64_t own_lo, int64_t own_hi) {
-    if (*err & kErrAbort) return;
     unsigned int* queue = reinterpret_cast<unsigned int*>(t.work + kTreeWorkQueue);   // zeroed by the build
     using WarpLists = WarpListsT<A::kStageBytes>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -683,7 +682,8 @@ walk_group_kernel(Bodies bd, int64_t nbodies, Tree t, typename A::Scalar G, type
     if (threadIdx.x == 0) {
         unsigned int sm;
         asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-        block_of_sm = atomicAdd(queue + kTreeWorkSms + sm % kTreeWorkSmCount, 1u);
+        // one look at the error word for the block: other blocks of this launch may be raising bits
+        block_of_sm = *err & kErrAbort ? ~0u : atomicAdd(queue + kTreeWorkSms + sm % kTreeWorkSmCount, 1u);
     }
     __syncthreads();
     if (static_cast<int64_t>(block_of_sm) * nwarps + w >= warps_per_sm(ngroups, sm_count)) return;

@@ -114,7 +114,7 @@ constexpr unsigned kRefLeaf = 0x80000000u;                         // list entry
 __global__ void __launch_bounds__(kRefThreads, 6)
 walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree t, Params P,
                       unsigned long long* stats, int* err) {
-    if (*err & kErrAbort) return;
+    if (__any_sync(0xffffffffu, *err & kErrAbort)) return;       // whole warps: other blocks may be raising bits
     __shared__ unsigned list[kRefList][kRefThreads];
     const int64_t nodes = t.counts[1];
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -236,7 +236,7 @@ template <int LANES, int MINB>
 __global__ void __launch_bounds__(kRefThreads, MINB)
 walk_reference_wide_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, Tree t, Params P,
                            unsigned long long* stats, int* err) {
-    if (*err & kErrAbort) return;
+    if (__any_sync(0xffffffffu, *err & kErrAbort)) return;       // whole warps: other blocks may be raising bits
     __shared__ WideShared<LANES> shared[kRefThreads / 32];
     WideShared<LANES>& S = shared[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, sub = lane / LANES, sl = lane % LANES;
@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(32 * kPlainWarps, 4)
 walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, const double4* __restrict__ cubes,
                      int64_t n, Tree t, Params P,
                      unsigned long long* stats, int* err) {
-    if (*err & kErrAbort) return;
+    if (__any_sync(0xffffffffu, *err & kErrAbort)) return;       // whole warps: other blocks may be raising bits
     __shared__ PlainShared shared[kPlainWarps];
     PlainShared& S = shared[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
