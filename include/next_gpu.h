@@ -202,6 +202,10 @@ int next_debug_keys(next_handle* h, uint64_t* keys, double* cube4);
 int next_debug_softening(int device, int64_t k, const double* size, const double* mass, const double* dist,
                          double* out);
 
+/* Test support: the inverse square root of the FP64 walks on k values, their
+ * exponents kept within the walks' limits (2^-960 .. 2^960). */
+int next_debug_inverse_root(int device, int64_t k, const double* x, double* out);
+
 /* Test support: sets the tree's capacity to cap_internal internal cells and
  * from then on grows it only when a build overflows it (not ahead of need),
  * so that tests can make a graph-replayed step overflow. */

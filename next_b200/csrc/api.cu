@@ -1691,6 +1691,19 @@ int next_debug_softening(int device, int64_t k, const double* size, const double
     return e == cudaSuccess ? NEXT_OK : NEXT_ERR_CUDA;
 }
 
+int next_debug_inverse_root(int device, int64_t k, const double* x, double* out) {
+    if (k < 0 || (k > 0 && (!x || !out))) return NEXT_ERR_INVALID_ARGUMENT;
+    if (k == 0) return NEXT_OK;
+    if (cudaSetDevice(device) != cudaSuccess) return NEXT_ERR_CUDA;
+    double* d = nullptr;
+    if (cudaMalloc(&d, sizeof(double) * 2 * k) != cudaSuccess) return NEXT_ERR_OUT_OF_MEMORY;
+    cudaError_t e = cudaMemcpy(d, x, sizeof(double) * k, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_inverse_root_eval(d, k, d + k, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + k, sizeof(double) * k, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? NEXT_OK : NEXT_ERR_CUDA;
+}
+
 int next_debug_fix_tree_capacity(next_handle* h, int64_t cap_internal) {
     int rc = check_ready(h);
     if (rc) return rc;

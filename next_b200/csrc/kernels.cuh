@@ -49,6 +49,7 @@ cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int6
 int direct_slices(int64_t n, int64_t k);
 // in: k sizes, k masses, k distances; out: k softening lengths (reference law)
 cudaError_t launch_softening_eval(const double* in, int64_t k, double* out, cudaStream_t st);
+cudaError_t launch_inverse_root_eval(const double* in, int64_t k, double* out, cudaStream_t st);
 cudaError_t launch_direct(const Bodies& bd, int64_t n, const int64_t* targets, int64_t k, double eps, double G,
                           double* partial, int slices, double* out, cudaStream_t st);
 

@@ -674,11 +674,24 @@ __global__ void softening_kernel(const double* __restrict__ in, int64_t k, doubl
     if (t < k) out[t] = softening_at(softening_base(in[t], in[k + t]), in[2 * k + t]);
 }
 
+// The walks' inverse square root on k values (test support).
+__global__ void inverse_root_kernel(const double* __restrict__ in, int64_t k, double* __restrict__ out) {
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t < k) out[t] = rsqrt_fast(away_from_ends(in[t]));
+}
+
 }  // namespace
 
 cudaError_t launch_softening_eval(const double* in, int64_t k, double* out, cudaStream_t st) {
     if (k <= 0) return cudaSuccess;
     softening_kernel<<<static_cast<unsigned>((k + 127) / 128), 128, 0, st>>>(in, k, out);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_inverse_root_eval(const double* in, int64_t k, double* out, cudaStream_t st) {
+    if (k <= 0) return cudaSuccess;
+    inverse_root_kernel<<<static_cast<unsigned>((k + 127) / 128), 128, 0, st>>>(in, k, out);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -71,6 +71,7 @@ SIGNATURES = {
     "next_debug_tree": (C.c_int, [_h, _d, C.c_int64, _i64]),
     "next_debug_fix_tree_capacity": (C.c_int, [_h, C.c_int64]),
     "next_debug_softening": (C.c_int, [C.c_int, C.c_int64, _d, _d, _d, _d]),
+    "next_debug_inverse_root": (C.c_int, [C.c_int, C.c_int64, _d, _d]),
     "next_sort_pairs": (C.c_int, [_h, C.c_int64, _u64, _u32, _u64, _u32, C.c_int]),
     "next_fp32_peak": (C.c_int, [C.c_int, _d, _d]),
     "next_flush_l2": (C.c_int, [_h]),
@@ -135,6 +136,17 @@ def debug_softening(size, mass, dist, device: int = 0):
     rc = lib.next_debug_softening(device, size.shape[0], _p(size, _d), _p(mass, _d), _p(dist, _d), _p(out, _d))
     if rc:
         raise NextError(f"next_debug_softening failed ({rc})")
+    return out
+
+
+def debug_inverse_root(x, device: int = 0):
+    """The FP64 walks' inverse square root on an array of values."""
+    lib = load()
+    x = _f64(x)
+    out = np.empty(x.shape[0])
+    rc = lib.next_debug_inverse_root(device, x.shape[0], _p(x, _d), _p(out, _d))
+    if rc:
+        raise NextError(f"next_debug_inverse_root failed ({rc})")
     return out
 
 
