@@ -31,3 +31,20 @@ def test_few_groups_equal_many(precision, n, group):
         for c in COLS:
             np.testing.assert_array_equal(got[c], want[c][:n])
         one.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64group"])
+@pytest.mark.parametrize("n", [33, 1000, 5000, 30000])
+def test_few_full_groups_equal_many(precision, n):
+    """The same with the default leaf and group sizes, beside so many bodies that every resident warp takes part."""
+    b, rest = ic.plummer(n, seed=n), ic.uniform_sphere(200000, seed=3)
+    both, one = Simulation("accurate", precision, eps=0.01), Simulation("accurate", precision, eps=0.01)
+    both.upload({c: np.concatenate([b[c], rest[c]]) for c in b}, np.array([0, n, n + 200000]))
+    one.upload(b)
+    want, got = both.accel(), one.accel()
+    assert both.stats()["n_groups"] > 20 * 148 > one.stats()["n_groups"]
+    assert one.stats()["device_error"] == 0
+    for c in COLS:
+        np.testing.assert_array_equal(got[c], want[c][:n])
+    both.close()
+    one.close()
