@@ -575,14 +575,25 @@ __device__ __forceinline__ void leaf_moments(const Bodies& bd, const uint64_t* _
         const double x0 = cnt > 0 ? bd.x[first] : 0.0, y0 = cnt > 0 ? bd.y[first] : 0.0,
                      z0 = cnt > 0 ? bd.z[first] : 0.0;
         double m = 0, sx = 0, sy = 0, sz = 0, sxx = 0, syy = 0, szz = 0, sxy = 0, sxz = 0, syz = 0;
-        for (int j = first; j < first + cnt; ++j) {
-            const double mj = bd.m[j];
-            const double dx = bd.x[j] - x0, dy = bd.y[j] - y0, dz = bd.z[j] - z0;
+        const auto add = [&](double mj, double xj, double yj, double zj) {
+            const double dx = xj - x0, dy = yj - y0, dz = zj - z0;
             const double mx = mj * dx, my = mj * dy, mz = mj * dz;
             m += mj; sx += mx; sy += my; sz += mz;
             sxx += mx * dx; syy += my * dy; szz += mz * dz;
             sxy += mx * dy; sxz += mx * dz; syz += my * dz;
+        };
+        int j = first;
+        // A bucket of the deepest level may hold any number of bodies: eight at a time, all loads before the first
+        // sum, else the thread waits for one sector of four bodies after another, as long as the bucket's alignment
+        // has it (build with a bucket of 3,900 bodies 681 us, of 3,950 434 us; now 385 and 435 us).
+        for (; j + 8 <= first + cnt && cnt > kMaxLeafCap; j += 8) {
+            double v[8][4];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) { v[k][0] = bd.m[j + k]; v[k][1] = bd.x[j + k]; v[k][2] = bd.y[j + k]; v[k][3] = bd.z[j + k]; }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) add(v[k][0], v[k][1], v[k][2], v[k][3]);
         }
+        for (; j < first + cnt; ++j) add(bd.m[j], bd.x[j], bd.y[j], bd.z[j]);
         double cx, cy, cz;
         if (m > 0) {
             const double ox = sx / m, oy = sy / m, oz = sz / m;

@@ -170,3 +170,27 @@ def test_keys_by_cell_number_equal_the_descent(oracle, kind):
     np.testing.assert_array_equal(cube, oracle.root_cube(b))
     np.testing.assert_array_equal(keys, oracle.keys(b))
     sim.close()
+
+
+def test_moments_of_buckets_of_every_remainder(oracle):
+    """Leaves of the deepest level with more bodies than any leaf size, at every alignment and remainder of the loop
+    over them: masses and centres of the oracle's tree (both sides round some thousand terms; one body left out of a
+    bucket would move its centre by 1e-10)."""
+    rng = np.random.default_rng(8)
+    sizes = rng.permutation([*range(60, 84), 127, 128, 129, 1001, 1006, 1, 2, 3, 5])
+    p = np.concatenate([rng.uniform(-1.0, 1.0, 3) + rng.uniform(-1e-7, 1e-7, (k, 3)) for k in sizes])
+    b = {k: np.ascontiguousarray(p[:, a]) for a, k in enumerate("xyz")}
+    for k in ("vx", "vy", "vz"):
+        b[k] = np.zeros(len(p))
+    b["m"] = rng.uniform(0.5, 1.5, len(p)) / len(p)
+    sim = Simulation("accurate", "fp64", leaf_cap=4)
+    sim.upload(b)
+    t, r = sim.debug_tree(), oracle.tree(b, mode="accurate", leaf_cap=4)
+    assert t.shape == r.shape
+    leaves = r[:, LEAF] == 1
+    np.testing.assert_array_equal(t[leaves, COUNT], r[leaves, COUNT])
+    assert np.max(t[leaves, COUNT]) > 900 and np.sum(t[leaves, COUNT] > 64) > 15
+    np.testing.assert_allclose(t[:, MASS], r[:, MASS], rtol=1e-12, atol=0)
+    np.testing.assert_allclose(t[:, MASS + 1:MASS + 4], r[:, MASS + 1:MASS + 4], rtol=0, atol=1e-12)
+    assert sim.stats()["device_error"] == 0
+    sim.close()
