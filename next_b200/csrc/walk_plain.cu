@@ -91,12 +91,43 @@ __device__ __forceinline__ RefTerm ref_entry(const Tree& t, int64_t nd, bool lea
     return ref_term(c.w, dx, dy, dz, r2, soft.x, sd, qa, qb, qc);
 }
 
-// Reference physics.  The warp alternates between two phases: first every
-// lane runs its own depth-first walk with the opening tests only, until it has
-// a list of kRefList accepted nodes (or its walk is over); then all lanes
-// evaluate their lists in order.  The tests diverge but are cheap; the
-// evaluation (two square roots, two divisions, the quadrupole) runs with
-// nearly all lanes.
+// What the softening of a bucket's bodies takes from their masses alone, computed when the mass changes (mostly
+// once: the cube root and the power are most of a bucket's work otherwise).
+struct BucketSoftening {
+    double mass = -1.0, base = 0.0, dark = -1.0;
+    __device__ __forceinline__ void of(double mj, double size, double mi, bool is_dark) {
+        if (mj == mass) return;
+        mass = mj;
+        base = softening_base(size, mj);
+        dark = is_dark ? softening_dark(size, mj, mi) : -1.0;
+    }
+};
+
+// The bodies of a deepest-level bucket act as one-body leaves of its size; added one by one.
+__device__ __forceinline__ void ref_bucket(const Bodies& bd, double size, const int2& lk, int64_t self, double xi, double yi,
+                                           double zi, double mi, bool dark, double& ax, double& ay, double& az,
+                                           unsigned& npp) {
+    const double2 zero = make_double2(0.0, 0.0);
+    BucketSoftening soft;
+    for (int j = lk.x; j < lk.x - lk.y; ++j) {
+        const double mj = bd.m[j];
+        if (j == self || mj == 0.0) continue;
+        const double ex = bd.x[j] - xi, ey = bd.y[j] - yi, ez = bd.z[j] - zi;
+        const double e2 = ex * ex + ey * ey + ez * ez;
+        soft.of(mj, size, mi, dark);
+        const RefTerm f = ref_term(mj, ex, ey, ez, e2, soft.base, soft.dark, zero, zero, zero);
+        ax += f.mx; ay += f.my; az += f.mz;
+        ax += f.qx; ay += f.qy; az += f.qz;
+        ++npp;
+    }
+}
+
+// Reference physics.  The warp alternates between two phases: first every lane runs its own depth-first walk with the
+// opening tests only, until it has a list of kRefList accepted nodes, stands
+// before a bucket or its walk is over; then all lanes evaluate their lists in
+// order, and the buckets, which neighbours mostly reach together.  The tests
+// diverge but are cheap; the evaluation (two square roots, two divisions, the
+// quadrupole) runs with nearly all lanes.
 //
 // Bound by FP64 latency: bhAccel's operations in bhAccel's order leave a chain
 // of four roots and divisions per interaction and no fused multiply-adds.
@@ -106,7 +137,9 @@ __device__ __forceinline__ RefTerm ref_entry(const Tree& t, int64_t nd, bool lea
 // bodies' power anew in every interaction.  Lists of 8 and 6 blocks per SM (80
 // registers) were the fastest of lists of 4-32 at 4-8 blocks; loading a sibling's
 // record while its predecessor is tested, or evaluating two entries at once,
-// cost more in registers than it hid (3.9-4.4 ms).
+// cost more in registers than it hid (3.9-4.4 ms).  Buckets: 300,000 bodies with
+// radii log-uniform over 2^-20 .. 1, 57 -> 24 ms against evaluating a bucket in the
+// middle of the tests, with a cube root per body of it (the plain loop: 47 ms).
 constexpr int kRefThreads = 128;
 constexpr int kRefList = 8;
 constexpr unsigned kRefLeaf = 0x80000000u;                         // list entry: the node is a single body
@@ -120,13 +153,13 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const bool active = i < n && i >= P.own_lo && i < P.own_hi;
     const int64_t ii = active ? i : 0;
-    unsigned npp = 0, npc = 0;
     const double xi = bd.x[ii], yi = bd.y[ii], zi = bd.z[ii], mi = bd.m[ii];
     const bool dark = bd.type[ii] == 1;
     // the mass whose dark-matter softening the upward pass stored per node
     const bool stored = dark && mi == *t.dark_mass;
-    const double theta = P.theta, theta2 = theta * theta;
     double ax = 0.0, ay = 0.0, az = 0.0;
+    unsigned npp = 0, npc = 0;
+    const double theta = P.theta, theta2 = theta * theta;
     int2 stack[kMaxLevel + 2];
     int sp = 0;
     int cur = sysid ? sysid[ii] : 0, end = active ? cur + 1 : cur;
@@ -162,23 +195,9 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
                 }
             } else if (lk.y == -1) {
                 if (lk.x != i) list[cnt++][threadIdx.x] = static_cast<unsigned>(k) | kRefLeaf;   // not its own leaf (octree.h:135)
-            } else if (cnt > 0) {
-                --cur;                                             // a bucket follows the listed nodes: evaluate them first
-                break;
             } else {
-                // deepest-level bucket: its bodies act as one-body leaves of this size
-                const double2 zero = make_double2(0.0, 0.0);
-                for (int j = lk.x; j < lk.x - lk.y; ++j) {
-                    const double mj = bd.m[j];
-                    if (j == i || mj == 0.0) continue;
-                    const double ex = bd.x[j] - xi, ey = bd.y[j] - yi, ez = bd.z[j] - zi;
-                    const double e2 = ex * ex + ey * ey + ez * ez;
-                    const RefTerm f = ref_term(mj, ex, ey, ez, e2, softening_base(size, mj),
-                                               dark ? softening_dark(size, mj, mi) : -1.0, zero, zero, zero);
-                    ax += f.mx; ay += f.my; az += f.mz;
-                    ax += f.qx; ay += f.qy; az += f.qz;
-                    ++npp;
-                }
+                --cur;                                             // a bucket: behind the listed nodes, with the other lanes' ones
+                break;
             }
         }
         __syncwarp();
@@ -189,6 +208,12 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
             ax += f.mx; ay += f.my; az += f.mz;
             ax += f.qx; ay += f.qy; az += f.qz;
             if (leaf) ++npp; else ++npc;
+        }
+        __syncwarp();
+        if (cnt < kRefList && cur < end) {                         // stopped before a bucket
+            const double2 head = t.soft[2 * static_cast<int64_t>(cur++)];
+            ref_bucket(bd, head.x, make_int2(__double2loint(head.y), __double2hiint(head.y)), i, xi, yi, zi, mi, dark, ax, ay, az,
+                       npp);
         }
         __syncwarp();
     }
@@ -207,17 +232,22 @@ walk_reference_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t n, T
 //
 // Small systems are bound by the latency of one body's walk, a chain of some
 // hundred tests and interactions of about a microsecond each, whatever the
-// number of bodies.  Walk of 256 bodies 157 -> 46 us, 1,000 264 -> 60 us, 4,096
-// 377 -> 97 us, 16,384 460 -> 206 us, 32,768 485 -> 372 us (Plummer spheres;
-// infalling ones 87 -> 26, 132 -> 31, 178 -> 51, 226 -> 102, 254 -> 191 us).
+// number of bodies.  Walk of 256 bodies 157 -> 45 us, 1,000 264 -> 54 us, 4,096
+// 377 -> 93 us, 16,384 460 -> 187 us, 32,768 485 -> 364 us (Plummer spheres).
 // More lanes are better while all warps are resident: 2,048 bodies 72 us with 32
 // lanes, 86 with 16 and 108 with 8; 4,096 129, 100 and 121 us; 8,192 210, 179 and
 // 141 us.  Eight lanes at 5, 6 and 7 blocks per SM (96, 80 and 72 registers):
 // 8,192 bodies 135, 152 and 159 us, 14,000 218, 166 and 186, 16,384 236, 230 and
-// 206, 40,960 491, 449 and 499 us.  Above 49,152 bodies (550 us against 562 us)
-// the walk above has warps enough and takes fewer instructions, which bind
-// there (57,344: 575 us against 619 us); 32-bit indices and the sums without a
-// loop took 5% off these walks.
+// 206, 40,960 491, 449 and 499 us.  Above 49,152 bodies (550 us against 562 us;
+// 57,344: 575 us against 619 us) the walk above has warps enough and takes fewer
+// instructions, which bind there.  Those comparisons were made with the buckets
+// evaluated by every lane for itself; a bucket's bodies spread over the lanes
+// need fewer registers, and all of these walks take 5-8% less (49,000 bodies
+// 541 -> 506 us); with 5,000 of 20,000 bodies at one place 4.3 -> 0.73 ms.
+//
+// The numbers of lanes and blocks are a table for the 148 SMs of this GPU and
+// all bodies of the launch; on another number of SMs, or where a rank walks only
+// its share of the bodies, another entry may be the fastest.
 //
 // A sub-warp's walk: the group being tested, or what is left of one behind its
 // first opened cell -- (first sibling, masks of accepted, opened, single-body
@@ -361,23 +391,52 @@ walk_reference_wide_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t
         __syncwarp();
         head += take;
         cnt -= take;
-        if (bucket >= 0 && cnt == 0) {
-            // deepest-level bucket: its bodies act as one-body leaves of this size
-            const double2 nh = t.soft[2 * static_cast<int64_t>(bucket)];
-            const int2 lk = make_int2(__double2loint(nh.y), __double2hiint(nh.y));
-            const double2 zero = make_double2(0.0, 0.0);
-            for (int b = lk.x; b < lk.x - lk.y; ++b) {
-                const double mj = bd.m[b];
-                if (b == i || mj == 0.0) continue;
-                const double ex = bd.x[b] - xi, ey = bd.y[b] - yi, ez = bd.z[b] - zi;
-                const double e2 = ex * ex + ey * ey + ez * ez;
-                const RefTerm f = ref_term(mj, ex, ey, ez, e2, softening_base(nh.x, mj),
-                                           dark ? softening_dark(nh.x, mj, mi) : -1.0, zero, zero, zero);
-                sum += sl == 0 ? f.mx : sl == 1 ? f.my : f.mz;
-                sum += sl == 0 ? f.qx : sl == 1 ? f.qy : f.qz;
-                if (sl == 0) ++npp;
+        // Deepest-level buckets, behind their sub-warps' listed nodes: the bodies act as one-body leaves of that
+        // size, as many at once as there are lanes.
+        const bool at_bucket = bucket >= 0 && cnt == 0;
+        if (__any_sync(0xffffffffu, at_bucket)) {
+            double size = 0.0;
+            int from = 0, bodies = 0;
+            if (at_bucket) {
+                const double2 nh = t.soft[2 * static_cast<int64_t>(bucket)];
+                size = nh.x;
+                from = __double2loint(nh.y);
+                bodies = -__double2hiint(nh.y);
+                bucket = -1;
             }
-            bucket = -1;
+            const double2 zero = make_double2(0.0, 0.0);
+            BucketSoftening soft;
+            for (int o = 0; __any_sync(0xffffffffu, o < bodies); o += LANES) {
+                const int b = from + o + sl;
+                bool use = false;
+                if (o + sl < bodies) {
+                    const double mj = bd.m[b];
+                    use = b != self && mj != 0.0;
+                    if (use) {
+                        const double ex = bd.x[b] - xi, ey = bd.y[b] - yi, ez = bd.z[b] - zi;
+                        const double e2 = ex * ex + ey * ey + ez * ez;
+                        soft.of(mj, size, mi, dark);
+                        const RefTerm f = ref_term(mj, ex, ey, ez, e2, soft.base, soft.dark, zero, zero, zero);
+                        S.term[0][lane] = f.mx; S.term[1][lane] = f.my; S.term[2][lane] = f.mz;
+                        S.term[3][lane] = f.qx; S.term[4][lane] = f.qy; S.term[5][lane] = f.qz;
+                        ++npp;
+                    }
+                }
+                const unsigned used = __ballot_sync(0xffffffffu, use) >> (LANES * sub);
+                __syncwarp();
+                if (sl < 3) {
+                    const double* m = &S.term[sl][sub * LANES];
+                    const double* q = &S.term[3 + sl][sub * LANES];
+#pragma unroll
+                    for (int e = 0; e < LANES; ++e) {
+                        if (used >> e & 1u) {
+                            sum += m[e];
+                            sum += q[e];
+                        }
+                    }
+                }
+                __syncwarp();
+            }
         }
     }
     if (active) {

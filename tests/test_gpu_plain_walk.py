@@ -196,3 +196,27 @@ def test_accurate_walk_far_from_unit_lengths(length):
     for k in ("ax", "ay", "az"):
         np.testing.assert_array_equal(out[1][k] * length * length, out[0][k])
     np.testing.assert_array_equal(out[1]["pot"] * length, out[0]["pot"])
+
+
+@pytest.mark.parametrize("n,theta", [(300, 0.6), (2000, 0.4), (5000, 0.25), (5000, 0.5), (9000, 0.39), (20001, 0.3), (20001, 0.5)])
+def test_reference_walk_buckets_of_every_size(n, theta):
+    """Coincident bodies in buckets below, at and above the numbers of lanes, with two masses, massless ones and dark
+    matter among them: the walks of several lanes per body, of lists and of small opening angles give the same bits."""
+    b, rest = reference_bodies(n, n + 1), reference_bodies(50000, 2)
+    at = 0
+    for size in (2, 3, 7, 8, 9, 15, 16, 17, 31, 32, 33, 65):
+        for k in ("x", "y", "z"):
+            b[k][at:at + size] = b[k][at]
+        at += size
+    b["m"][0:at:3] *= 2.0
+    b["m"][1:at:7] = 0.0
+    one, both = Simulation("reference", "fp64", theta=theta), Simulation("reference", "fp64", theta=theta)
+    one.upload(b)
+    both.upload({c: np.concatenate([b[c], rest[c]]) for c in b}, np.array([0, n, n + 50000]))
+    one.reset_timers()
+    got, want = one.accel(), both.accel()
+    assert one.stats()["device_error"] == 0 and both.stats()["device_error"] == 0
+    for c in ("ax", "ay", "az"):
+        np.testing.assert_array_equal(got[c], want[c][:n])
+    one.close()
+    both.close()
