@@ -220,3 +220,19 @@ def test_reference_walk_buckets_of_every_size(n, theta):
         np.testing.assert_array_equal(got[c], want[c][:n])
     one.close()
     both.close()
+
+
+def test_reference_walk_buckets_against_the_oracle(oracle):
+    """The same buckets in a walk of one thread per body, at an opening angle on either side of the lists' limit."""
+    b = reference_bodies(50001, 7)
+    for at, size in ((0, 70), (100, 33), (200, 2)):
+        for k in ("x", "y", "z"):
+            b[k][at:at + size] = b[k][at]
+    b["m"][0:70:3] *= 2.0
+    for theta in (0.39, 0.4):
+        sim = Simulation("reference", "fp64", theta=theta)
+        sim.upload(b)
+        a, r = sim.accel(), oracle.accel(b, mode="ref", theta=theta)
+        assert sim.stats()["device_error"] == 0
+        close(a, r, ("ax", "ay", "az"))
+        sim.close()
