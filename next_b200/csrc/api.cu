@@ -835,6 +835,13 @@ static int upload_staged(next_handle* h, int64_t n_systems, const int64_t* offse
         h->n = n;
         Systems& S = h->sys;
         S.n = h->nsys;
+        S.smallest = n;
+        S.largest = 0;
+        for (int64_t s = 0; s < n_systems; ++s) {
+            const int64_t k = offsets[s + 1] - offsets[s];
+            S.largest = std::max(S.largest, k);
+            if (k > 0) S.smallest = std::min(S.smallest, k);
+        }
         int bits = 0;
         while (h->nsys > 1 && (int64_t(1) << bits) < n_systems) ++bits;
         h->sys_bits = bits;

@@ -30,6 +30,7 @@ struct Bodies {
 // Per-system geometry: root cube and body range.
 struct Systems {
     int n;               // number of systems
+    int64_t smallest, largest;   // bodies of the smallest (that has any) and of the largest one
     int base;            // key >> base = system number (63 for one system)
     int levels;          // octant levels per key (base / 3)
     const int64_t* offsets;   // n + 1

@@ -545,6 +545,7 @@ walk_reference_wide_kernel(Bodies bd, const int32_t* __restrict__ sysid, int64_t
 // 128 registers, 4 blocks per SM (5: 9.3 ms and more).
 constexpr int kPlainW = 7;
 constexpr int kPlainWarps = 4;
+constexpr int64_t kSmallSystem = 80;                     // systems of fewer bodies take the walk below
 // Popping k nodes adds at most 7 k entries, and one node at a time never more
 // than 7 per level: rounds are cut short so that 7 * kMaxLevel + 8 entries stay
 // free for a walk that goes on one node at a time.
@@ -585,7 +586,7 @@ walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, c
             else top = mid;
         }
         first = offsets[sys] + (w - (offsets[sys] / kPlainW + sys)) * kPlainW;
-        last = offsets[sys + 1];
+        last = offsets[sys + 1] - offsets[sys] < kSmallSystem ? first : offsets[sys + 1];   // small: the walk below
     }
     // a warp with any body of this device's share computes all of its bodies (again so that a body's
     // sums do not depend on the share) and stores the share's
@@ -756,6 +757,215 @@ walk_accurate_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, c
     add_stats(stats, npp, npc);
 }
 
+// The same for systems of fewer than kSmallSystem bodies, with eight lanes for W
+// bodies: such a system's walk has few nodes at a time, and four of them share
+// a warp (loops are the warp's, stacks and lists each group's own).
+//
+// A whole warp leaves most lanes idle there, and batches of many tiny systems
+// were slower than by a thread per body: walk of 1,048,576 systems of 4 bodies
+// 9.2 ms, here 2.8 ms (a thread per body 0.45 ms), 262,144 of 16 6.1 -> 2.2 (1.5) ms,
+// 65,536 of 32 2.7 -> 1.45 (1.31) ms, of 64 5.8 -> 4.4 (4.7) ms, 40,000 of 100 6.1 -> 6.0
+// (6.6) ms, 30,000 of 128 6.1 -> 7.0 (7.2) ms.  A small system on its own is bound by
+// its rounds instead: 20 bodies 18 -> 21 (38) us, 50 20 -> 39 (88) us, which is why
+// the line lies below the one of batches.  It is by a system's own size, so that
+// a body's sums stay the same alone and in a batch.
+constexpr int kSmallLanes = 8;
+constexpr int kSmallStack = kPlainReserve + 7 * kSmallLanes;
+constexpr int kSmallChunk = 4;                           // bodies of an opened leaf appended per lane and turn
+constexpr int kSmallList = kSmallLanes + kSmallLanes * kSmallChunk;
+struct SmallShared {
+    int2 stack[kSmallStack];
+    int2 list[kSmallList];
+    double pos[kPlainW][4];
+};
+
+template <bool POT>
+__global__ void __launch_bounds__(32 * kPlainWarps, 4)
+walk_accurate_small_kernel(Bodies bd, const int64_t* __restrict__ offsets, int nsys, const double4* __restrict__ cubes,
+                           int64_t n, Tree t, Params P, unsigned long long* stats, int* err) {
+    if (__any_sync(0xffffffffu, *err & kErrAbort)) return;       // whole warps: other blocks may be raising bits
+    __shared__ SmallShared shared[32 * kPlainWarps / kSmallLanes];
+    SmallShared& S = shared[threadIdx.x / kSmallLanes];
+    const int lane = threadIdx.x & 31, sl = lane % kSmallLanes, shift = lane - sl;
+    const uint32_t lt = (1u << sl) - 1u;
+    // the group's part of a ballot
+    const auto mine_of = [&](bool v) { return __ballot_sync(0xffffffffu, v) >> shift & ((1u << kSmallLanes) - 1u); };
+    const int64_t w = (blockIdx.x * static_cast<int64_t>(32 * kPlainWarps) + threadIdx.x) / kSmallLanes;
+    unsigned npp = 0, npc = 0;
+    int sys = 0;
+    int64_t first = w * kPlainW, last = n;
+    if (offsets) {
+        int top = nsys;
+        while (top - sys > 1) {
+            const int mid = (sys + top) >> 1;
+            if (offsets[mid] / kPlainW + mid <= w) sys = mid;
+            else top = mid;
+        }
+        first = offsets[sys] + (w - (offsets[sys] / kPlainW + sys)) * kPlainW;
+        last = offsets[sys + 1] - offsets[sys] < kSmallSystem ? offsets[sys + 1] : first;   // large: the walk above
+    }
+    unsigned bodies = 0, own = 0;
+#pragma unroll
+    for (int b = 0; b < kPlainW; ++b) {
+        if (first + b >= last) continue;
+        bodies |= 1u << b;
+        if (first + b >= P.own_lo && first + b < P.own_hi) own |= 1u << b;
+    }
+    const unsigned nodes = static_cast<unsigned>(t.counts[1]), nbodies = static_cast<unsigned>(n);
+    const int ex = static_cast<int>((__double_as_longlong(cubes[sys].w) >> 52) & 0x7ff) - 1023;
+    const bool scaled = ex > 150 || ex < -150;
+    const double S1 = scaled ? scalbn(1.0, -ex) : 1.0;
+    const double eps2 = (P.eps * S1) * (P.eps * S1);
+    double ax[kPlainW], ay[kPlainW], az[kPlainW], pot[kPlainW];
+    int sp = own ? 1 : 0, pn = 0;
+#pragma unroll
+    for (int b = 0; b < kPlainW; ++b) {
+        const int64_t i = own && first + b < last ? first + b : 0;
+        if (sl == b) { S.pos[b][0] = bd.x[i] * S1; S.pos[b][1] = bd.y[i] * S1; S.pos[b][2] = bd.z[i] * S1; }
+        ax[b] = ay[b] = az[b] = pot[b] = 0.0;
+    }
+    if (sl == 0) S.stack[0] = make_int2(sys, static_cast<int>(bodies));
+    __syncwarp();
+    while (__any_sync(0xffffffffu, sp > 0 || pn > 0)) {
+        const int room = (kSmallStack - kPlainReserve - sp) / 7;
+        const int nb = min(min(sp, kSmallLanes), max(room, 1));
+        sp -= nb;
+        const int2 entry = sl < nb ? S.stack[sp + sl] : make_int2(-1, 0);
+        const int node = entry.x;
+        unsigned mask = static_cast<unsigned>(entry.y);
+        __syncwarp();
+        int2 lk = make_int2(0, 0);
+        double4 c = make_double4(0.0, 0.0, 0.0, 0.0);
+        double2 qa = make_double2(0.0, 0.0), qb = qa, qc = qa, qd = qa;
+        if (mask) {
+            bool ok = static_cast<unsigned>(node) < nodes;
+            if (ok) {
+                lk = __ldg(t.link + node);
+                const double2* c2 = reinterpret_cast<const double2*>(t.com + node);
+                const double2 ca = __ldg(c2), cb = __ldg(c2 + 1);
+                const double2* q2 = reinterpret_cast<const double2*>(t.quad64 + 8 * static_cast<int64_t>(node));
+                qd = __ldg(q2 + 3);
+                if (P.quad) { qa = __ldg(q2); qb = __ldg(q2 + 1); qc = __ldg(q2 + 2); }
+                c = make_double4(ca.x, ca.y, cb.x, cb.y);
+                const unsigned e = static_cast<unsigned>(lk.x) + static_cast<unsigned>(lk.y > 0 ? lk.y : -lk.y);
+                ok = lk.x >= 0 && lk.y <= 8 && e <= (lk.y > 0 ? nodes : nbodies);
+            }
+            if (!ok) raise_error(err, kErrIndex);
+            if (!ok || c.w == 0.0) mask = 0;
+        }
+        if (scaled) {
+            c.x *= S1; c.y *= S1; c.z *= S1;
+            qd.y *= S1;
+            qa.x = qa.x * S1 * S1; qa.y = qa.y * S1 * S1; qb.x = qb.x * S1 * S1;
+            qb.y = qb.y * S1 * S1; qc.x = qc.x * S1 * S1; qc.y = qc.y * S1 * S1;
+        }
+        const double rc2 = qd.y * qd.y;
+        unsigned opened = 0;
+#pragma unroll
+        for (int b = 0; b < kPlainW; ++b) {
+            const bool mine = mask >> b & 1u;
+            const double dx = c.x - at(S.pos[b][0]), dy = c.y - at(S.pos[b][1]), dz = c.z - at(S.pos[b][2]);
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            const bool open = mine && r2 < rc2, use = mine && !open;
+            opened |= static_cast<unsigned>(open) << b;
+            const double r2s = away_from_ends(r2 + eps2);
+            const double rinv = use ? rsqrt_fast(r2s) : 0.0;
+            const double rinv2 = rinv * rinv;
+            const double qx = fma(qc.x, dz, fma(qb.y, dy, qa.x * dx));
+            const double qy = fma(qc.y, dz, fma(qa.y, dy, qb.y * dx));
+            const double qz = fma(qb.x, dz, fma(qc.y, dy, qc.x * dx));
+            const double q = fma(dz, qz, fma(dy, qy, dx * qx));
+            const double rinv5 = rinv * (rinv2 * rinv2);
+            const double k = fma(2.5 * q, rinv2, c.w * r2s);
+            ax[b] = fma(rinv5, fma(k, dx, -qx), ax[b]);
+            ay[b] = fma(rinv5, fma(k, dy, -qy), ay[b]);
+            az[b] = fma(rinv5, fma(k, dz, -qz), az[b]);
+            if (POT) pot[b] -= fma(0.5 * q, rinv5, c.w * rinv);
+        }
+        npc += __popc(mask & ~opened & own);
+        // children of opened cells -> stack
+        const int push = opened && lk.y > 0 ? lk.y : 0;
+        int off = 0, total = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t m = mine_of((push >> k) & 1);
+            off += __popc(m & lt) << k;
+            total += __popc(m) << k;
+        }
+        const bool broken = sp + total > kSmallStack;    // only a broken tree gets here
+        if (broken) {
+            if (sl == 0) raise_error(err, kErrIndex);
+            sp = total = 0;
+        } else if (total > 0) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k < push) S.stack[sp + off + k] = make_int2(lk.x + k, static_cast<int>(opened));
+        }
+        sp += total;
+        // bodies of opened leaves -> list, evaluated eight at a time, the rest when the walk ends
+        int remaining = opened && lk.y < 0 && !broken ? -lk.y : 0;
+        int src = lk.x;
+        while (__any_sync(0xffffffffu, remaining > 0 || (sp == 0 && pn > 0))) {
+            const int take = min(remaining, kSmallChunk);
+            int o2 = 0, tot = 0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const uint32_t m = mine_of((take >> k) & 1);
+                o2 += __popc(m & lt) << k;
+                tot += __popc(m) << k;
+            }
+            for (int k = 0; k < take; ++k) S.list[pn + o2 + k] = make_int2(src + k, static_cast<int>(opened));
+            pn += tot;
+            src += take;
+            remaining -= take;
+            const bool more = mine_of(remaining > 0) != 0;
+            __syncwarp();
+            for (;;) {
+                const bool go = pn >= kSmallLanes || (pn > 0 && sp == 0 && !more);
+                if (!__any_sync(0xffffffffu, go)) break;
+                const int k = go ? max(pn - kSmallLanes, 0) : pn;        // from the end: nothing moves
+                const int2 pe = k + sl < pn ? S.list[k + sl] : make_int2(-1, 0);
+                const int j = pe.x;
+                const unsigned jm = static_cast<unsigned>(pe.y);
+                pn = k;
+                double xj = 0.0, yj = 0.0, zj = 0.0, mj = 0.0;
+                if (jm) { xj = bd.x[j]; yj = bd.y[j]; zj = bd.z[j]; mj = bd.m[j]; }
+                if (scaled) { xj *= S1; yj *= S1; zj *= S1; }
+#pragma unroll
+                for (int b = 0; b < kPlainW; ++b) {
+                    if (!(jm >> b & 1u) || j == first + b) continue;
+                    const double dx = xj - at(S.pos[b][0]), dy = yj - at(S.pos[b][1]), dz = zj - at(S.pos[b][2]);
+                    const double rinv = rsqrt(dx * dx + dy * dy + dz * dz + eps2);
+                    const double mr = mj * rinv, mr3 = mr * rinv * rinv;
+                    ax[b] = fma(mr3, dx, ax[b]);
+                    ay[b] = fma(mr3, dy, ay[b]);
+                    az[b] = fma(mr3, dz, az[b]);
+                    if (POT) pot[b] -= mr;
+                    npp += own >> b & 1u;
+                }
+                __syncwarp();
+            }
+        }
+        __syncwarp();
+    }
+#pragma unroll
+    for (int b = 0; b < kPlainW; ++b) {
+        for (int o = kSmallLanes / 2; o > 0; o >>= 1) {
+            ax[b] += __shfl_xor_sync(0xffffffffu, ax[b], o);
+            ay[b] += __shfl_xor_sync(0xffffffffu, ay[b], o);
+            az[b] += __shfl_xor_sync(0xffffffffu, az[b], o);
+            if (POT) pot[b] += __shfl_xor_sync(0xffffffffu, pot[b], o);
+        }
+        const int64_t i = first + b;
+        if (sl == 0 && (own >> b & 1u)) {
+            const double g = P.G * S1;
+            bd.ax[i] = g * ax[b] * S1; bd.ay[i] = g * ay[b] * S1; bd.az[i] = g * az[b] * S1;
+            if (POT) bd.pot[i] = g * pot[b];
+        }
+    }
+    add_stats(stats, npp, npc);
+}
+
 // FP64 direct summation: block (x = 128 targets, y = source slice).
 constexpr int kDirectThreads = 128;
 
@@ -838,10 +1048,20 @@ cudaError_t launch_walk_plain(const Bodies& bd, const int32_t* sysid, const int6
     if (n <= 0) return cudaSuccess;
     const int32_t* sid = sys.n > 1 ? sysid : nullptr;
     if (P.physics == NEXT_PHYSICS_ACCURATE) {
-        const int64_t warps = (n + kPlainW - 1) / kPlainW + (sys.n > 1 ? sys.n : 0);
-        const unsigned blocks = static_cast<unsigned>((warps + kPlainWarps - 1) / kPlainWarps);
-        auto kern = potential ? walk_accurate_kernel<true> : walk_accurate_kernel<false>;
-        kern<<<blocks, 32 * kPlainWarps, 0, st>>>(bd, sys.n > 1 ? d_offsets : nullptr, sys.n, sys.cube, n, t, P, stats, err);
+        const int64_t* offsets = sys.n > 1 ? d_offsets : nullptr;
+        const int64_t chunks = (n + kPlainW - 1) / kPlainW + (sys.n > 1 ? sys.n : 0);    // of up to W bodies
+        if (sys.smallest < kSmallSystem) {
+            constexpr int per = 32 * kPlainWarps / kSmallLanes;
+            auto kern = potential ? walk_accurate_small_kernel<true> : walk_accurate_small_kernel<false>;
+            kern<<<static_cast<unsigned>((chunks + per - 1) / per), 32 * kPlainWarps, 0, st>>>(bd, offsets, sys.n, sys.cube, n, t,
+                                                                                            P, stats, err);
+        }
+        if (sys.largest >= kSmallSystem) {
+            auto kern = potential ? walk_accurate_kernel<true> : walk_accurate_kernel<false>;
+            kern<<<static_cast<unsigned>((chunks + kPlainWarps - 1) / kPlainWarps), 32 * kPlainWarps, 0, st>>>(
+                bd, offsets, sys.n, sys.cube, n, t, P, stats, err);
+        }
+        if (sys.smallest < kSmallSystem && sys.largest >= kSmallSystem) count_launches(1);
     } else if (n <= kWideMax) {
         // as many lanes, then as many registers, as leave every warp resident at once
         const int64_t block = 148 * (kRefThreads / 32);           // warps of one block per SM

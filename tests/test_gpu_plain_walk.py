@@ -236,3 +236,57 @@ def test_reference_walk_buckets_against_the_oracle(oracle):
         assert sim.stats()["device_error"] == 0
         close(a, r, ("ax", "ay", "az"))
         sim.close()
+
+
+@pytest.mark.parametrize("n,leaf_cap,theta,eps,quad,shape", [
+    (6, 1, 0.5, 0.01, 1, "sphere"), (8, 1, 0.5, 0.0, 1, "sphere"), (50, 1, 1.0, 0.01, 0, "sphere"),
+    (79, 1, 0.5, 0.01, 1, "sphere"), (80, 1, 0.5, 0.01, 1, "sphere"), (81, 5, 0.5, 0.01, 1, "sphere"),
+    (79, 64, 0.5, 0.01, 1, "sphere"), (79, 1, 0.02, 0.01, 1, "sphere"), (77, 3, 0.02, 0.01, 1, "chain"),
+    (60, 1, 0.5, 0.01, 1, "chain"), (79, 1, 0.5, 0.02, 1, "bucket"), (30, 2, 0.7, 0.02, 1, "bucket"),
+])
+def test_accurate_walk_of_small_systems(oracle, n, leaf_cap, theta, eps, quad, shape):
+    """Eight lanes for seven bodies: around the size where whole warps take over, full stacks, cells down to the deepest
+    level, leaves of many bodies, massless ones."""
+    b = ic.plummer(n, seed=n)
+    if shape == "chain":
+        r = 2.0 ** -np.linspace(0, 19, n)
+        for k, s in zip("xyz", (1.0, -0.7, 0.4)):
+            b[k] = s * r
+    if shape == "bucket":
+        for k in "xyz":
+            b[k][: n // 2] = b[k][0]
+        b["m"][::5] = 0.0
+    sim = Simulation("accurate", "fp64", theta=theta, eps=eps, leaf_cap=leaf_cap, quadrupole=quad)
+    sim.upload(b)
+    sim.reset_timers()
+    a = sim.accel(potential=True)
+    r = oracle.accel(b, mode="accurate", theta=theta, eps=eps, leaf_cap=leaf_cap, quad=bool(quad), potential=True)
+    st = sim.stats()
+    assert (st["pp_interactions"], st["pc_interactions"], st["device_error"]) == (r["pp"], r["pc"], 0)
+    close(a, r, ("ax", "ay", "az"))
+    close(a, r, ("pot",))
+    sim.close()
+
+
+def test_accurate_walk_batch_of_small_systems():
+    """Systems of 0 to 90 bodies, walked by groups of lanes and by whole warps, and one large one: every system's
+    forces and potentials are bit-equal to its own."""
+    rng = np.random.default_rng(4)
+    sizes = [*rng.integers(0, 91, 400), 700, 79, 80, 1, 0]
+    parts = [ic.plummer(int(k), seed=i) for i, k in enumerate(sizes) if k]
+    b = {c: np.concatenate([p[c] for p in parts]) for c in parts[0]}
+    offsets = np.concatenate([[0], np.cumsum(sizes)])
+    sim = Simulation("accurate", "fp64")
+    sim.upload(b, offsets)
+    a = sim.accel(potential=True)
+    assert sim.stats()["device_error"] == 0
+    for i in [*range(0, 400, 23), 400, 401, 402, 403]:
+        if sizes[i] == 0:
+            continue
+        one = Simulation("accurate", "fp64")
+        one.upload(ic.plummer(int(sizes[i]), seed=i))
+        r = one.accel(potential=True)
+        for c in ("ax", "ay", "az", "pot"):
+            np.testing.assert_array_equal(a[c][offsets[i]:offsets[i + 1]], r[c])
+        one.close()
+    sim.close()
