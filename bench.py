@@ -135,10 +135,16 @@ def force_error(a, d, idx):
     return {"median": float(np.median(e)), "p90": float(np.percentile(e, 90)), "p99": float(np.percentile(e, 99))}
 
 
-def time_cpu_reference(bodies, dt, budget_s, threads=None):
+def compiled_reference():
+    """The reference compiled for the host cores, or None and the reason where it has not been built."""
+    from oracle import oracle
+    if not os.path.exists(oracle.REF_SO):
+        return None, "oracle/_ref/libnextref.so has not been built (its sources are not here)"
+    return oracle.Reference(), None
+
+
+def time_cpu_reference(R, bodies, dt, budget_s, threads=None):
     """The reference's own Step() (oracle/_ref, OpenMP on the host cores) on the same bodies."""
-    from oracle.oracle import Reference
-    R = Reference()
     threads = threads or os.cpu_count() or 1
     R.set_threads(threads)
     n = bodies["x"].shape[0]
@@ -159,11 +165,13 @@ def run_reference_arm(args):
     rank, world, _ = env_rank()
     if rank != 0:
         return 0
+    R, why = compiled_reference()
+    if R is None:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
+        return 0
     from next_b200 import ic
     bodies = ic.uniform_sphere(WORKLOAD["n"], seed=WORKLOAD["seed"])
     steps = max(1, min(args.steps, 2))
-    from oracle.oracle import Reference
-    R = Reference()
     threads = os.cpu_count() or 1
     R.set_threads(threads)
     b = dict(bodies)
@@ -564,9 +572,9 @@ def run_ours(args):
                                    max(3, args.steps // 4), idx, d_direct, sim.get_params())
     # the reference's as-shipped forces on the same sampled bodies, same state
     cpu_accel = None
-    if rank == 0 and state0 is not None and not args.skip_cpu and n <= 2_000_000:
-        from oracle.oracle import Reference
-        cpu_accel = Reference().accel_sample(state0, idx)
+    reference, no_reference = compiled_reference() if rank == 0 and not args.skip_cpu else (None, None)
+    if reference is not None and state0 is not None and n <= 2_000_000:
+        cpu_accel = reference.accel_sample(state0, idx)
     refphys = None
     if rank == 0 and state0 is not None and world == 1 and not args.skip_fp64:
         refphys = ref_physics_leg(state0, W, local, max(1, args.fp64_steps), idx, d_direct, cpu_accel)
@@ -601,8 +609,10 @@ def run_ours(args):
     # ---- CPU baseline: the reference's own Step() on the host cores
     cpu = None
     if rank == 0 and not args.skip_cpu:
-        if offsets is None and n <= 2_000_000:
-            cpu = time_cpu_reference(bodies, W["dt"], args.cpu_budget)
+        if reference is None:
+            cpu = {"unavailable": no_reference}
+        elif offsets is None and n <= 2_000_000:
+            cpu = time_cpu_reference(reference, bodies, W["dt"], args.cpu_budget)
             if cpu_accel is not None:
                 cpu["force_error"] = force_error(cpu_accel, d_direct, np.arange(idx.shape[0]))
                 cpu["force_error"]["versus"] = (f"FP64 direct summation with Plummer eps {W['eps']} on the same "
