@@ -52,8 +52,8 @@ def sort_passes(key_levels, n_systems):
 
 
 def sort_bytes_per_body(passes):
-    # each pass reads and writes a (u64 key, u32 index) pair; the histogram pass reads the keys once
-    return passes * 24 + 8
+    # each pass reads and writes a (u64 key, u32 index) pair; the digits are counted where the keys are made
+    return passes * 24
 
 
 def env_rank():
@@ -657,8 +657,8 @@ def run_ours(args):
         "pp_fraction": st["pp_interactions"] / max(1, st["pp_interactions"] + st["pc_interactions"]),
         "pp_interactions_per_s": st["pp_interactions"] / (st["ms_walk"] * 1e-3),
         "pc_interactions_per_s": st["pc_interactions"] / (st["ms_walk"] * 1e-3),
-        # the key sort's algorithmic traffic: passes x (12 B read + 12 B written) + the
-        # 8-byte histogram read, per body, over the bench's own sort stage time;
+        # the key sort's algorithmic traffic: passes x (12 B read + 12 B written) per
+        # body, over the bench's own sort stage time;
         # passes = ceil(key bits / 8) of this run's keys (trimmed to the tree depth)
         "sort_hbm": {"passes": passes, "key_levels": st["key_levels"], "bytes_per_body": sort_bpb,
                      "gbs": sort_gbs, "frac": sort_gbs / peaks["hbm_gbs"] if peaks.get("hbm_gbs") else None,

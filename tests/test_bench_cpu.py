@@ -22,3 +22,9 @@ def test_own_arm_without_the_compiled_reference(monkeypatch):
     monkeypatch.setattr(oracle, "REF_SO", os.path.join(os.sep, "nonexistent", "libnextref.so"))
     reference, why = bench.compiled_reference()
     assert reference is None and "libnextref.so" in why
+
+
+def test_sort_traffic_is_the_passes():
+    """The sort stage reads and writes a 12-byte pair per pass; its digits come counted from the kernel of the keys."""
+    assert bench.sort_bytes_per_body(bench.sort_passes(10, 1)) == 4 * 24
+    assert bench.sort_bytes_per_body(bench.sort_passes(21, 1)) == 8 * 24
