@@ -240,7 +240,7 @@ int next_sort_pairs(next_handle* h, int64_t n, const uint64_t* keys_in, const ui
  * no output may overlap an input or the other output (checked byte range by
  * byte range: NEXT_ERR_INVALID_ARGUMENT).  It allocates nothing: all scratch
  * comes from one static device array sized for NEXT_SORT_NOALLOC_MAX_PAIRS
- * pairs (14,844,192 bytes = 14.16 MiB, reserved on every GPU that loads the
+ * pairs (14,836,000 bytes = 14.15 MiB, reserved on every GPU that loads the
  * library until the process exits); larger n is rejected with
  * NEXT_ERR_INVALID_ARGUMENT.  The first call in each CUDA context (normally
  * once per device) looks up that array's address and sets the sort kernel's

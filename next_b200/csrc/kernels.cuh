@@ -21,8 +21,9 @@ cudaError_t launch_keys(const Bodies& b, const int32_t* sysid, int64_t n, const 
 #define NB_SORT_ITEMS 15
 #endif
 constexpr int64_t kSortTile = 256 * NB_SORT_ITEMS;   // pairs per onesweep tile (threads x items)
+constexpr int64_t kSortFixedWords = 8 * 256 + 8;   // digit counts of all passes, their tile tickets
 constexpr int64_t sort_scratch_words_for(int64_t n) {
-    return 2 * 8 * 256 + 8 + 8 * ((n + kSortTile - 1) / kSortTile) * 256;
+    return kSortFixedWords + 8 * ((n + kSortTile - 1) / kSortTile) * 256;
 }
 size_t sort_scratch_words(int64_t n);
 cudaError_t sort_prepare();

@@ -616,7 +616,7 @@ constexpr Layout layout() {
 constexpr Layout kOneTile[] = {layout<256, 4, 1, true>(), layout<256, 8, 1, true>(), layout<512, 8, 1, true>(),
                                layout<512, 15, 1, true>()};
 constexpr Layout kManyTiles = layout<256, NB_SORT_ITEMS, 3, false>();
-constexpr int64_t kOneTileBlocks = 148;
+constexpr int64_t kOneTileBlocks = 148;    // this GPU's SMs; a fixed table, right (if not the fastest) on any number
 
 const Layout& layout_for(int64_t n) {
     for (const Layout& l : kOneTile)
@@ -629,13 +629,14 @@ int64_t tiles_for(int64_t n) { return (n + layout_for(n).pairs - 1) / layout_for
 }  // namespace
 
 static_assert(kSortTile == kManyTiles.pairs, "tile size shared with the scratch-size formula");
+static_assert(kSortFixedWords % 4 == 0, "statuses are read as 16-byte vectors");
 
-// Scratch words for sorts of up to n pairs: digit counts (8 x 256; twice that
-// is reserved), tile tickets (8), status (8 x tiles x 256) for the layout with
-// the most tiles any such sort can use.
+// Scratch words for sorts of up to n pairs: digit counts (8 x 256), tile tickets
+// (8), status (8 x tiles x 256) for the layout with the most tiles any such sort
+// can use.
 size_t sort_scratch_words(int64_t n) {
     const int64_t one = (n + kOneTile[0].pairs - 1) / kOneTile[0].pairs;
-    const size_t few = static_cast<size_t>(2 * 8 * kRadix + 8 + 8 * kRadix * (one < kOneTileBlocks ? one : kOneTileBlocks));
+    const size_t few = static_cast<size_t>(kSortFixedWords + 8 * kRadix * (one < kOneTileBlocks ? one : kOneTileBlocks));
     const size_t many = static_cast<size_t>(sort_scratch_words_for(n));
     return few > many ? few : many;
 }
@@ -655,7 +656,7 @@ bool sort_counts_digits(int64_t n) { return n > kSmallPairs; }
 // first 8 x 256 words) can be added to from then on.
 cudaError_t sort_begin(int64_t n, int key_bits, uint32_t* scratch, cudaStream_t st) {
     if (!sort_counts_digits(n)) return cudaSuccess;
-    const size_t words = static_cast<size_t>(2 * 8 * kRadix + 8 + ((key_bits + 7) / 8) * tiles_for(n) * kRadix);
+    const size_t words = static_cast<size_t>(kSortFixedWords + ((key_bits + 7) / 8) * tiles_for(n) * kRadix);
     return cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * words, st);
 }
 
@@ -678,8 +679,8 @@ cudaError_t sort_passes(const uint64_t* keys_in, const uint32_t* vals_in, uint64
     const int passes = (key_bits + 7) / 8;
     const Layout& l = layout_for(n);
     const int64_t tiles = tiles_for(n);
-    unsigned int* tickets = scratch + 16 * kRadix;
-    uint32_t* status = scratch + 16 * kRadix + 8;
+    unsigned int* tickets = scratch + 8 * kRadix;
+    uint32_t* status = scratch + kSortFixedWords;              // read 16 bytes at a time
     const uint64_t* src_k = keys_in;
     const uint32_t* src_v = vals_in;
     for (int p = 0; p < passes; ++p) {

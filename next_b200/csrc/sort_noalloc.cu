@@ -12,7 +12,7 @@
 // fixed-size array below.
 //
 // The array is a file-scope __device__ variable, so every GPU that loads this
-// part of the library reserves it (14,844,192 bytes, 14.16 MiB) until the
+// part of the library reserves it (14,836,000 bytes, 14.15 MiB) until the
 // process exits.  Host code must not use the array's name as a device
 // address: the first call in each CUDA context (normally once per device, in
 // its primary context) looks the address up with cudaGetSymbolAddress, with
@@ -41,7 +41,7 @@ constexpr size_t kWordsBytes = sizeof(uint32_t) * sort_scratch_words_for(kMaxPai
 constexpr size_t kScratchBytes = kAltKeysBytes + kAltValsBytes + kErrBytes + kWordsBytes;
 
 static_assert(kAltKeysBytes % 256 == 0 && kAltValsBytes % 256 == 0, "sub-buffers stay 256-byte aligned");
-static_assert(kScratchBytes == 14844192, "the size the header states");
+static_assert(kScratchBytes == 14836000, "the size the header states");
 
 static __device__ __align__(256) unsigned char g_sort_scratch[kScratchBytes];
 
