@@ -408,7 +408,8 @@ def ref_physics_leg(bodies, cfg, device, steps, idx, d_direct, cpu_accel):
             "ms_per_step": st["ms_step"] / steps, "force_error": err,
             "max_rel_diff_vs_reference_cpu": parity,
             "physics": "reference (as the CPU arm: adaptive softening, half-width theta 0.5, its quadrupole)",
-            "structure": "one thread per body, one body per leaf, two tree builds per step (step.h:113,164)"}
+            "structure": ("a thread per body" if n > 49_152 else "8 to 32 lanes per body") +
+                         ", one body per leaf, two tree builds per step (step.h:113,164)"}
 
 
 def large_sort_leg(cfg, device, n=8_388_608, steps=3):

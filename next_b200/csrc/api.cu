@@ -170,7 +170,7 @@ struct next_handle {
     int sys_bits = 0;                 // bits of the system number above the octant digits
     int key_bits = 63;                // sorted key bits
     bool depth_decided = false;
-    bool cube_fresh = false;          // the last kick-drift wrote the root cube (one system)
+    bool cube_fresh = false;          // the last kick-drift wrote the root cubes
     int64_t builds = 0;               // tree builds enqueued
     int64_t depth_seen = 0;           // the build whose depth report was last acted on
     bool pot_valid = false;
@@ -462,7 +462,7 @@ int read_device_error(next_handle* h, int* bits) {
     NB_TRY(cudaStreamSynchronize(h->st), "sync");
     *bits = h->host->status.err;
     // the first build after an upload measured the tree depth: later builds
-    // keep three levels of margin below it.  A tree that outgrows them gets
+    // keep a margin of levels below it (trimmed_levels).  A tree that outgrows them gets
     // leaves of more than leaf_cap bodies at the last level (still exact,
     // slower): seen here, the keys get three more levels.
     const int64_t deepest = h->host->status.counts[3];

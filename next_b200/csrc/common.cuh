@@ -46,9 +46,11 @@ struct Systems {
 // last key level (a leaf over capacity: the keys need more levels)
 constexpr unsigned kDepthOverfull = 64;
 
-constexpr int kTreeWorkQueue = 4;      // word of Tree::work the group walk counts its groups in,
-constexpr int kTreeWorkSms = 2, kTreeWorkSmCount = 512;  // from its 2nd 32-bit half on, its blocks per SM
-constexpr int kTreeWorkWalk = 1 + kTreeWorkSmCount / 2;  // words of the walk
+// The group walk's 64-bit words of Tree::work: it counts its groups in the
+// first, and its blocks per SM, 32 bits each, in those behind it.
+constexpr int kTreeWorkQueue = 4;
+constexpr int kTreeWorkSms = 2, kTreeWorkSmCount = 512;  // 32-bit words from the queue's
+constexpr int kTreeWorkWalk = 1 + kTreeWorkSmCount / 2;
 
 struct Tree {
     // capacities

@@ -7,9 +7,9 @@
 // afford cudaMalloc/cudaFree, which may synchronise the whole device in the
 // middle of a pipelined time step.  For them this entry point sorts pairs
 // between caller-owned device buffers and takes every byte of scratch --
-// the ping-pong half of the LSD passes, the digit histograms, the tile
-// tickets, the look-back status words and the error word -- from the
-// fixed-size array below.
+// the ping-pong half of the LSD passes, the digit counts, the tile tickets,
+// the tiles' status words and the error word -- from the fixed-size array
+// below (up to 16,384 pairs only the error word: those are sorted on chip).
 //
 // The array is a file-scope __device__ variable, so every GPU that loads this
 // part of the library reserves it (14,836,000 bytes, 14.15 MiB) until the
@@ -85,7 +85,7 @@ unsigned long long current_context_id() {
 }
 
 // Set-up, once per context, with that context current: the array's device
-// address and the onesweep kernel's shared-memory attribute.
+// address and the sort kernels' shared-memory attributes.
 int context_scratch(unsigned char** out) {
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     unsigned long long id = current_context_id();

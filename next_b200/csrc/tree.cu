@@ -749,9 +749,9 @@ upward_leaves_kernel(Bodies bd, int64_t nbodies, const uint64_t* __restrict__ ke
 //
 // Bound by the longest chain of levels, each an arrival, a round trip for the
 // children and the combination: all the children's records are in flight at
-// once (one warp per block leaves it 255 registers; chunks of two or four
-// children needed two to four round trips a level), and the cell's centre,
-// half-width and parent come from the child-search pass instead of a descent
+// once (247 registers, 126 in the reference's physics, in blocks of one warp;
+// chunks of two or four children needed two to four round trips a level), and
+// the cell's centre, half-width and parent come from the child-search pass instead of a descent
 // from the key.  16,384 bodies: build 0.158 -> 0.134 ms; 65,536 bodies with one
 // body per leaf 0.260 -> 0.223 ms; 1,048,576 such 0.67 -> 0.60 ms; 16.7 M bodies
 // 2.86 -> 2.81 ms.

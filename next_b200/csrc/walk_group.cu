@@ -658,7 +658,9 @@ struct Fp64Arith {
 // 8 (2,616) 147 -> 135 us; collapse of 32,768 in groups of 32 (1,205) 212 ->
 // 136 us; of 65,536 (2,874, past the line) 250 us both; 1,048,576 unchanged.
 // Rounding down instead ran 101 us against 91 us at 2,800 groups of 8, rounding
-// up 150 us against 136 us at 2,616.
+// up 150 us against 136 us at 2,616.  The share assumes the whole GPU: where
+// other work holds most SMs, the free ones still use only their share of warps,
+// and a rank that walks part of the groups shares out all of them.
 __device__ __forceinline__ int64_t warps_per_sm(int64_t ngroups, int sm_count) {
     const int64_t whole = (ngroups + sm_count - 1) / sm_count;
     if (whole <= 4) return whole;

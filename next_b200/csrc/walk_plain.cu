@@ -1,11 +1,12 @@
 // Plain FP64 force walks: every body opens the tree by its own distance.
 //
 // Reference physics: one thread per target body (several lanes in small
-// systems), depth-first over the tree in octant order 0..7 -- the order bhAccel recurses (src/gravity/octree.h:176-178)
-// -- with a per-level (next sibling, end) stack instead of recursion, and
-// bhAccel's arithmetic (octree.h:134-173, softening.h:21-35) operation for
-// operation.  Accurate physics (Plummer softening, full-width opening test,
-// corrected quadrupole): one warp per few bodies, one node per lane.
+// systems), depth-first over the tree in octant order 0..7 -- the order bhAccel
+// recurses (src/gravity/octree.h:176-178) -- with a per-level (next sibling,
+// end) stack instead of recursion, and bhAccel's arithmetic (octree.h:134-173,
+// softening.h:21-35) operation for operation.  Accurate physics (Plummer
+// softening, full-width opening test, corrected quadrupole): a warp, or eight
+// lanes in small systems, per few bodies, one node per lane.
 //
 // Also: the FP64 direct-summation kernel used to state force errors.
 //
